@@ -8,7 +8,7 @@
 // and the request's 64-bit key, times 2^-32.  No sort is done: the rank that a
 // target mass falls on is found by bisection on the bit pattern of p (32 block
 // sums in a fixed order), then ties of that value are counted in id order.
-// Every sum is taken in an order fixed by the vocabulary size alone.
+// Every sum is taken in an order fixed by the vocabulary size alone, or is a sum of whole numbers.
 #include <math_constants.h>
 
 #include "common.cuh"
@@ -210,17 +210,31 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs,
 }
 
 // --------------------------------------------------------------------------
-// The same sampling with a row spread over the eight blocks of a cluster: a thread keeps its
-// tokens' probabilities in registers (ids gthread * per .. + per - 1, contiguous, so that ties
-// are met in id order), every pass of the bisection is a compare-and-add over those registers,
-// a block sum and one exchange of the eight blocks' partials through distributed shared
-// memory, summed in rank order.  One block a row walked the row's 152 k probabilities from
-// memory 31 times a selection (≈ 1 ms a call, 1.8 ms with top-p, whatever the number of rows).
-// Sums are taken in an order fixed by the vocabulary size alone; all blocks of a cluster see the
-// same totals and take the same decisions.
+// The same sampling with a row spread over the 1, 2, 4 or 8 blocks of a cluster: a block keeps
+// e = exp(l / T - max) of its contiguous part of the row in shared memory and finds the rank that
+// a mass falls on digit by digit of e's bit pattern, highest first: 12 + 10 + 10 bits, a
+// histogram of 1,024 bins a digit (e <= 1, so the first digit stays below 1,017).
+//
+// All masses are whole numbers.  The tokens of a bin share their exponent, so a bin's mass is the
+// sum of their 24-bit mantissas, kept as two 32-bit sums (of the low and of the high 12 bits)
+// that shared-memory atomics add in any order with the same result: no sum here depends on how
+// the row is spread.  Over the first digit masses are counted in units of 2^-46 (163,840 tokens of
+// e = 1 fit 64 bits; a bin's own sum is cut to a unit, 1e-14 of the largest token), below it in
+// the mantissa units of the chosen bin, exactly.  Every block adds up the eight histograms by
+// itself (one exchange a digit), so all take the same decisions.
+//
+// What bounds it: the exchanges (one for the maximum, one a digit: five digits with a nucleus,
+// since the first digit's histogram serves both selections, else three), about 4 us each at eight
+// blocks.  Bisecting on the bit pattern instead took 16 passes over registers and 17 exchanges a
+// selection.  151,936 tokens with top-p, 1 / 8 / 64 rows: 33 / 35 / 76 us (bisecting: 103 / 106 /
+// 525); 64 rows of 32,768: 29 us (509).
 // --------------------------------------------------------------------------
-constexpr int SAMPLE_CLUSTER = 8;
-constexpr int SAMPLE_PER = 20;        // probabilities a thread keeps: vocabularies up to 8 x 1024 x 20 = 163,840
+constexpr int SAMPLE_CLUSTER = 8;                   // most blocks a row is spread over
+constexpr int SAMPLE_MOST = 8 * 1024 * 20;          // largest vocabulary of this kernel
+constexpr int SAMPLE_PART = 49152;                  // most tokens of a block: 192 KB of shared memory
+constexpr int SAMPLE_BINS = 1024;                   // a thread adds up one bin
+constexpr int SAMPLE_UNIT = 46;                     // masses over the whole row: units of 2^-46
+static_assert(SAMPLE_BINS == SAMPLE_THREADS, "a thread a bin");
 
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
@@ -235,273 +249,292 @@ __device__ __forceinline__ uint32_t peer_addr(const void* mine, int rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
   return r;
 }
-__device__ __forceinline__ float ld_peer_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ int ld_peer_s32(uint32_t addr) {
-  int v;
-  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+__device__ __forceinline__ uint2 ld_peer_u2(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
   return v;
 }
 
-// What the blocks of a cluster exchange: two sets of slots used in turn, so that a block may
-// write its next partial while a slow peer still reads the last one.
-struct ClusterShare {
-  float f[2][4];
-  int i[2][2];
-  float all_f[SAMPLE_CLUSTER][4];
-  int all_i[SAMPLE_CLUSTER][2];
-  float warp_f[3][32];
+struct SampleShare {
+  uint2 hist[2][SAMPLE_BINS];       // sums of the low and high 12 bits of the mantissas; digits use the two in turn
+  uint2 best;                       // this block's largest logit and its id
+  float warp_v[32];
   int warp_i[32];
+  unsigned long long warp_mass[32];
+  unsigned long long total;         // of the row, in units of 2^-46
+  unsigned long long above;         // mass in front of the chosen bin
+  unsigned long long through;       // mass up to and including the chosen token (units of 2^-46)
+  unsigned long long peer_sum[SAMPLE_CLUSTER];   // the chosen value's mass in each block
+  int bin;
+  int bad;                          // the row holds something that is no number
 };
 
-// Every block gives (a, b); every thread gets the eight blocks' pairs in rank order in sh.all_f.
-// `turn` (every thread's own copy, the same in all) says which set of slots this exchange uses.
-__device__ void cluster_gather_f(ClusterShare& sh, int& turn, float a, float b = 0.f, float c = 0.f) {
-  const int t = turn;
-  turn ^= 1;
-  if (threadIdx.x == 0) { sh.f[t][0] = a; sh.f[t][1] = b; sh.f[t][2] = c; }
-  cluster_sync_all();
-  if (threadIdx.x < SAMPLE_CLUSTER * 4) {
-    const int rank = threadIdx.x >> 2, which = threadIdx.x & 3;
-    sh.all_f[rank][which] = ld_peer_f32(peer_addr(&sh.f[t][which], rank));
-  }
-  __syncthreads();
-}
-__device__ void cluster_gather_i(ClusterShare& sh, int& turn, int a, int b) {
-  const int t = turn;
-  turn ^= 1;
-  if (threadIdx.x == 0) { sh.i[t][0] = a; sh.i[t][1] = b; }
-  cluster_sync_all();
-  if (threadIdx.x < SAMPLE_CLUSTER * 2) {
-    const int rank = threadIdx.x >> 1, which = threadIdx.x & 1;
-    sh.all_i[rank][which] = ld_peer_s32(peer_addr(&sh.i[t][which], rank));
-  }
-  __syncthreads();
-}
-
-// sum over the cluster: a thread's value, lanes by xor tree, warps ascending, blocks in rank order
-__device__ float cluster_sum(ClusterShare& sh, int& turn, float v) {
-  const float block = ls_block_sum(v, sh.warp_f[0]);
-  cluster_gather_f(sh, turn, block);
-  float total = 0.f;
-#pragma unroll
-  for (int r = 0; r < SAMPLE_CLUSTER; ++r) total += sh.all_f[r][0];
-  __syncthreads();          // all have read before the next gather writes
-  return total;
-}
-
-// three sums over the cluster at once (each in the order of cluster_sum): one exchange for all
-__device__ void cluster_sum3(ClusterShare& sh, int& turn, float& a, float& b, float& c) {
+// The block's inclusive scan of `mass` in thread order (bins from the highest down: thread t has bin
+// SAMPLE_BINS - 1 - t); `excl` is what lies in front of this thread.
+__device__ unsigned long long sample_scan(SampleShare& sh, unsigned long long mass, unsigned long long& excl) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  a = ls_warp_sum(a);
-  b = ls_warp_sum(b);
-  c = ls_warp_sum(c);
-  __syncthreads();
-  if (lane == 0) { sh.warp_f[0][warp] = a; sh.warp_f[1][warp] = b; sh.warp_f[2][warp] = c; }
-  __syncthreads();
-  float ta = 0.f, tb = 0.f, tc = 0.f;
-  for (int w = 0; w < 32; ++w) { ta += sh.warp_f[0][w]; tb += sh.warp_f[1][w]; tc += sh.warp_f[2][w]; }
-  cluster_gather_f(sh, turn, ta, tb, tc);
-  a = b = c = 0.f;
-#pragma unroll
-  for (int r = 0; r < SAMPLE_CLUSTER; ++r) { a += sh.all_f[r][0]; b += sh.all_f[r][1]; c += sh.all_f[r][2]; }
-  __syncthreads();
-}
-
-// mass of this cluster's row with p >= the value whose bits are `bits`
-__device__ float mass_at_least_regs(ClusterShare& sh, int& turn, const float* p, int per, uint32_t bits) {
-  float s = 0.f;
-#pragma unroll
-  for (int j = 0; j < SAMPLE_PER; ++j)
-    if (j < per && __float_as_uint(p[j]) >= bits) s += p[j];
-  return cluster_sum(sh, turn, s);
-}
-
-// select_rank over the registers of a cluster: the token on which `target` falls in the
-// (-p, id) order, written to *token_out by the one thread that holds it; returns the mass up to
-// and including that token.
-__device__ float select_rank_regs(ClusterShare& sh, int& turn, const float* p, int per, int begin, float target,
-                                  int* token_out) {
-  target = fmaxf(target, 1e-37f);
-  // the largest bit pattern lo with mass(lo) >= target, the interval cut in four a pass (three
-  // thresholds' masses from one sweep over the registers and one exchange)
-  uint32_t lo = 0u, hi = 0x7f800000u;
-  for (int it = 0; it < 32 && lo < hi; ++it) {
-    const uint32_t span = hi - lo;
-    const uint32_t q1 = span >> 2, q2 = span >> 1, q3 = span - (span >> 2);
-    const uint32_t t1 = lo + (q1 ? q1 : 1u), t2 = lo + (q2 ? q2 : 1u), t3 = lo + (q3 ? q3 : 1u);
-    float m1 = 0.f, m2 = 0.f, m3 = 0.f;
-#pragma unroll
-    for (int j = 0; j < SAMPLE_PER; ++j) {
-      if (j < per) {
-        const uint32_t b = __float_as_uint(p[j]);
-        if (b >= t1) m1 += p[j];
-        if (b >= t2) m2 += p[j];
-        if (b >= t3) m3 += p[j];
-      }
-    }
-    cluster_sum3(sh, turn, m1, m2, m3);
-    if (m3 >= target) lo = t3;
-    else if (m2 >= target) { lo = t2; hi = t3 - 1u; }
-    else if (m1 >= target) { lo = t1; hi = t2 - 1u; }
-    else hi = t1 - 1u;
-  }
-  // snap lo to the smallest probability that occurs at or above it
-  float vmin = CUDART_INF_F;
-#pragma unroll
-  for (int j = 0; j < SAMPLE_PER; ++j)
-    if (j < per && __float_as_uint(p[j]) >= lo) vmin = fminf(vmin, p[j]);
-  vmin = -ls_warp_max(-vmin);
-  {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh.warp_f[0][warp] = vmin;
-    __syncthreads();
-    vmin = sh.warp_f[0][0];
-    for (int w = 1; w < 32; ++w) vmin = fminf(vmin, sh.warp_f[0][w]);
-    __syncthreads();
-  }
-  cluster_gather_f(sh, turn, vmin);
-#pragma unroll
-  for (int r = 0; r < SAMPLE_CLUSTER; ++r) vmin = fminf(vmin, sh.all_f[r][0]);
-  __syncthreads();
-  const uint32_t vbits = __float_as_uint(vmin);
-  const float above = mass_at_least_regs(sh, turn, p, per, vbits + 1u);
-  int j = 0;
-  if (vmin > 0.f && vmin < CUDART_INF_F) {
-    j = (int)ceilf((target - above) / vmin) - 1;
-    if (j < 0) j = 0;
-  }
-  // ties of value vmin in ascending id: a thread's ids are contiguous and ascend with the thread
-  int count = 0;
-#pragma unroll
-  for (int q = 0; q < SAMPLE_PER; ++q) count += (q < per && __float_as_uint(p[q]) == vbits);
-  // exclusive prefix over the block: lanes by a scan, warps ascending
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int incl = count;
+  unsigned long long incl = mass;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int up = __shfl_up_sync(0xffffffffu, incl, o);
+    const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += up;
   }
-  if (lane == 31) sh.warp_i[warp] = incl;
+  if (lane == 31) sh.warp_mass[warp] = incl;
   __syncthreads();
-  int before = incl - count, block_total = 0;
-  for (int w = 0; w < 32; ++w) {
-    if (w < warp) before += sh.warp_i[w];
-    block_total += sh.warp_i[w];
-  }
-  __syncthreads();
-  cluster_gather_i(sh, turn, block_total, 0);
-  const int rank = (int)cluster_rank();
-  int total = 0;
+  unsigned long long before = lane < warp ? sh.warp_mass[lane] : 0ull;
 #pragma unroll
-  for (int r = 0; r < SAMPLE_CLUSTER; ++r) {
-    if (r < rank) before += sh.all_i[r][0];
-    total += sh.all_i[r][0];
-  }
-  __syncthreads();
-  if (j >= total) j = total - 1;
-  if (j < 0) j = 0;
-  if (total <= 0 && rank == 0 && threadIdx.x == 0) *token_out = 0;      // nothing to choose from (a row of NaN)
-  if (j >= before && j < before + count) {
-    int k = before;
-#pragma unroll
-    for (int q = 0; q < SAMPLE_PER; ++q) {
-      if (q < per && __float_as_uint(p[q]) == vbits) {
-        if (k == j) *token_out = begin + q;
-        ++k;
-      }
-    }
-  }
-  return above + (float)(j + 1) * vmin;
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  incl += before;
+  excl = incl - mass;
+  return incl;
 }
 
-__global__ void __cluster_dims__(SAMPLE_CLUSTER, 1, 1) __launch_bounds__(SAMPLE_THREADS)
+// one token's mantissa into its bin
+__device__ __forceinline__ void sample_count(uint2* hist, uint32_t bin, uint32_t bits) {
+  const uint32_t m = (bits & 0x7fffffu) | (bits >= 0x800000u ? 0x800000u : 0u);
+  atomicAdd(&hist[bin].x, m & 0xfffu);
+  atomicAdd(&hist[bin].y, m >> 12);
+}
+
+// The token that `target` (>= 1, at most the row's mass; units of 2^-46) falls on in the (-e, id)
+// order, `l1_excl` and `l1_incl` being the scan of the first digit's bins.  Writes sh.through and,
+// in the block that holds the token, *token_out where it is not null.  `turn`: the histogram free
+// for the next digit (zeroed); every thread's own copy, the same in all.
+template <int CL>
+__device__ void sample_select(SampleShare& sh, const float* e, int live, int begin, int& turn, unsigned long long l1_excl,
+                              unsigned long long l1_incl, unsigned long long target, int* token_out) {
+  const int tid = threadIdx.x, b = SAMPLE_BINS - 1 - tid;
+  if (l1_excl < target && target <= l1_incl) {
+    sh.bin = b;
+    sh.above = l1_excl;
+  }
+  __syncthreads();
+  uint32_t prefix = (uint32_t)sh.bin;
+  const unsigned long long l1_above = sh.above;
+  // from here on in mantissa units of the bin: 2^(exponent - 150)
+  const int exponent = (int)(prefix >> 3) > 0 ? (int)(prefix >> 3) : 1;
+  const int shift = exponent - (150 - SAMPLE_UNIT);
+  unsigned long long want = target - l1_above;
+  want = shift >= 0 ? (want + ((1ull << shift) - 1)) >> shift : want << -shift;
+  unsigned long long within = 0;                      // mantissa units in front, inside the first digit's bin
+#pragma unroll 1
+  for (int digit = 1; digit < 3; ++digit) {
+    uint2* hist = sh.hist[turn];
+    const int down = digit == 1 ? 10 : 0;
+    for (int i = tid; i < live; i += SAMPLE_THREADS) {
+      const uint32_t bits = __float_as_uint(e[i]);
+      if (bits >> (down + 10) == prefix && bits != 0u) sample_count(hist, (bits >> down) & 1023u, bits);
+    }
+    cluster_sync_all();
+    const int here = turn;
+    turn ^= 1;
+    sh.hist[turn][tid] = make_uint2(0u, 0u);          // nobody reads the digit before any more
+    unsigned long long sum[CL], mass = 0;
+#pragma unroll
+    for (int r = 0; r < CL; ++r) {
+      const uint2 v = ld_peer_u2(peer_addr(&sh.hist[here][b], r));
+      sum[r] = v.x + ((unsigned long long)v.y << 12);
+      mass += sum[r];
+    }
+    unsigned long long excl;
+    const unsigned long long incl = sample_scan(sh, mass, excl);
+    if (excl < want && want <= incl) {
+      sh.bin = b;
+      sh.above = excl;
+      if (digit == 2) {
+#pragma unroll
+        for (int r = 0; r < CL; ++r) sh.peer_sum[r] = sum[r];
+      }
+    }
+    __syncthreads();
+    prefix = (prefix << 10) | (uint32_t)sh.bin;
+    want -= sh.above;
+    within += sh.above;
+    __syncthreads();
+  }
+  // prefix is now the bit pattern of the chosen value; its tokens in ascending id, one mantissa each
+  const unsigned long long m = (prefix & 0x7fffffu) | (prefix >= 0x800000u ? 0x800000u : 0u);
+  const unsigned long long rank_j = (want + m - 1) / m - 1;         // want lies in 1 .. ties x m
+  if (tid == 0) {
+    const unsigned long long in = within + (rank_j + 1) * m;
+    sh.through = l1_above + (shift >= 0 ? in << shift : in >> -shift);
+  }
+  if (token_out != nullptr) {
+    unsigned long long before = 0;
+    const int rank = (int)cluster_rank();
+    for (int r = 0; r < rank; ++r) before += sh.peer_sum[r];
+    const unsigned long long own = sh.peer_sum[rank] / m;
+    before /= m;
+    if (rank_j >= before && rank_j < before + own) {               // the same in all threads of a block
+      const int per = (live + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
+      const int lo = min(tid * per, live), hi = min(lo + per, live);
+      unsigned long long count = 0, excl;
+      for (int i = lo; i < hi; ++i) count += __float_as_uint(e[i]) == prefix;
+      sample_scan(sh, count, excl);
+      unsigned long long k = before + excl;
+      for (int i = lo; i < hi; ++i)
+        if (__float_as_uint(e[i]) == prefix && k++ == rank_j) *token_out = begin + i;
+    }
+  }
+  __syncthreads();
+}
+
+template <int CL>
+__global__ void __launch_bounds__(SAMPLE_THREADS, 1)
 sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
                       const float* __restrict__ top_p, const uint32_t* __restrict__ keys,
                       const uint32_t* __restrict__ positions, int* __restrict__ out, int vocab) {
   ls_dependency_sync();
-  __shared__ ClusterShare sh;
-  const int r = blockIdx.x / SAMPLE_CLUSTER;
+  __shared__ SampleShare sh;
+  extern __shared__ float sample_e[];                // this block's part of the row
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r = blockIdx.x / CL;
   const int rank = (int)cluster_rank();
-  const float* row = logits + (int64_t)r * vocab;
-  const int per = (vocab + SAMPLE_CLUSTER * SAMPLE_THREADS - 1) / (SAMPLE_CLUSTER * SAMPLE_THREADS);
-  const int begin = (rank * SAMPLE_THREADS + (int)threadIdx.x) * per;
-  int turn = 0;
-  // this thread's logits; the row's argmax (ties to the lowest id; NaN never wins)
-  float p[SAMPLE_PER];
+  const int part = (vocab + CL - 1) / CL;
+  const int begin = rank * part;
+  const int live = min(part, vocab - begin);         // may be negative: no tokens
+  const float* row = logits + (int64_t)r * vocab + begin;
+  // the row's argmax (ties to the lowest id; NaN never wins)
   ArgMax best{-CUDART_INF_F, 0x7fffffff};
-#pragma unroll
-  for (int j = 0; j < SAMPLE_PER; ++j) {
-    p[j] = -CUDART_INF_F;
-    if (j < per && begin + j < vocab) {
-      p[j] = row[begin + j];
-      if (p[j] > best.v || (p[j] == best.v && begin + j < best.i)) best = ArgMax{p[j], begin + j};
-    }
+#pragma unroll 8
+  for (int i = tid; i < live; i += SAMPLE_THREADS) {
+    const float v = row[i];
+    sample_e[i] = v;
+    if (v > best.v || (v == best.v && begin + i < best.i)) best = ArgMax{v, begin + i};
   }
+  sh.hist[0][tid] = sh.hist[1][tid] = make_uint2(0u, 0u);
+  if (tid == 0) sh.bad = 0;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     ArgMax other{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
     best = better(best, other);
   }
-  {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) { sh.warp_f[0][warp] = best.v; sh.warp_i[warp] = best.i; }
-    __syncthreads();
-    best = ArgMax{sh.warp_f[0][0], sh.warp_i[0]};
-    for (int w = 1; w < 32; ++w) best = better(best, ArgMax{sh.warp_f[0][w], sh.warp_i[w]});
-    __syncthreads();
-  }
-  cluster_gather_f(sh, turn, best.v);
-  cluster_gather_i(sh, turn, best.i, 0);
-  ArgMax top{sh.all_f[0][0], sh.all_i[0][0]};
-#pragma unroll
-  for (int q = 1; q < SAMPLE_CLUSTER; ++q) top = better(top, ArgMax{sh.all_f[q][0], sh.all_i[q][0]});
+  if (lane == 0) { sh.warp_v[warp] = best.v; sh.warp_i[warp] = best.i; }
   __syncthreads();
-  if (top.i == 0x7fffffff) top.i = 0;
+  best = ArgMax{sh.warp_v[lane], sh.warp_i[lane]};
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    ArgMax other{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
+    best = better(best, other);
+  }
+  if (tid == 0) sh.best = make_uint2(__float_as_uint(best.v), (uint32_t)best.i);
+  cluster_sync_all();
+  {
+    const uint2 peer = ld_peer_u2(peer_addr(&sh.best, lane & (CL - 1)));
+    best = ArgMax{__uint_as_float(peer.x), (int)peer.y};
+#pragma unroll
+    for (int o = CL / 2; o > 0; o >>= 1) {
+      ArgMax other{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
+      best = better(best, other);
+    }
+  }
+  if (best.i == 0x7fffffff) best.i = 0;
   const float temp = temperature[r];
   if (!(temp > 0.f)) {                       // the same branch in every block of the cluster
-    if (rank == 0 && threadIdx.x == 0) out[r] = top.i;
+    if (rank == 0 && tid == 0) out[r] = best.i;
     cluster_sync_all();                      // no block leaves while a peer may still read its shared memory
     return;
   }
-  // p = exp(l / T - max) / sum, as the one-block kernel takes it
-  const float vmax = __fdiv_rn(top.v, temp);
-  float s = 0.f;
-#pragma unroll
-  for (int j = 0; j < SAMPLE_PER; ++j) {
-    if (j < per && begin + j < vocab) {
-      p[j] = expf(__fdiv_rn(p[j], temp) - vmax);
-      s += p[j];
-    } else {
-      p[j] = 0.f;
-    }
+  const float vmax = __fdiv_rn(best.v, temp);
+  // e, and the first digit's histogram; what is no number goes to the last bin
+  for (int i = tid; i < live; i += SAMPLE_THREADS) {
+    const float v = expf(__fdiv_rn(sample_e[i], temp) - vmax);
+    sample_e[i] = v;
+    const uint32_t bits = __float_as_uint(v);
+    if (bits > 0x3f800000u) atomicAdd(&sh.hist[0][SAMPLE_BINS - 1].x, 1u);
+    else if (bits != 0u) sample_count(sh.hist[0], bits >> 20, bits);
   }
-  const float z = cluster_sum(sh, turn, s);
+  cluster_sync_all();
+  int turn = 1;
+  unsigned long long l1_excl, l1_incl;
+  {
+    const int b = SAMPLE_BINS - 1 - tid;
+    unsigned long long mass = 0;
 #pragma unroll
-  for (int j = 0; j < SAMPLE_PER; ++j) p[j] = __fdiv_rn(p[j], z);
-  // tokens past the vocabulary hold 0: they never count as ties of a positive value, and a
-  // selection never lands on them since `vmin` is taken over values at or above a mass that exists
-  const int live = begin < vocab ? (vocab - begin < per ? vocab - begin : per) : 0;
-
+    for (int q = 0; q < CL; ++q) {
+      const uint2 v = ld_peer_u2(peer_addr(&sh.hist[0][b], q));
+      mass += v.x + ((unsigned long long)v.y << 12);
+    }
+    if (b == SAMPLE_BINS - 1) {
+      sh.bad = mass != 0;
+      mass = 0;
+    }
+    const int shift = max(b >> 3, 1) - (150 - SAMPLE_UNIT);
+    mass = shift >= 0 ? mass << shift : -shift < 64 ? mass >> -shift : 0ull;
+    l1_incl = sample_scan(sh, mass, l1_excl);
+    if (tid == SAMPLE_THREADS - 1) sh.total = l1_incl;
+  }
+  __syncthreads();
+  if (sh.bad || sh.total == 0ull) {          // a row with something that is no number: token 0
+    if (rank == 0 && tid == 0) out[r] = 0;
+    cluster_sync_all();
+    return;
+  }
   const float u = (float)((double)philox_word0(positions[2 * r], positions[2 * r + 1], keys[2 * r],
                                                keys[2 * r + 1]) * 2.3283064365386963e-10);
   const float tp = top_p[r];
-  int token = -1;
-  float head;
+  unsigned long long head = sh.total;
+  // a share of a mass, at least one unit (a draw of exactly 0 falls on the first rank) and at most the mass
+  auto share_of = [](float share, unsigned long long mass) {
+    const double d = ceil((double)share * (double)mass);
+    return d < 1.0 ? 1ull : d >= (double)mass ? mass : (unsigned long long)d;
+  };
   if (tp < 1.0f) {
-    int unused = -1;
-    head = select_rank_regs(sh, turn, p, live, begin, tp, &unused);
-  } else {
-    head = mass_at_least_regs(sh, turn, p, live, 0u);
+    sample_select<CL>(sh, sample_e, live, begin, turn, l1_excl, l1_incl, share_of(tp, head), nullptr);
+    head = sh.through;
   }
-  select_rank_regs(sh, turn, p, live, begin, u * head, &token);
-  if (token >= 0) out[r] = token;            // exactly one thread of the cluster holds it
+  sample_select<CL>(sh, sample_e, live, begin, turn, l1_excl, l1_incl, share_of(u, head), &out[r]);
   cluster_sync_all();                        // no block leaves while a peer may still read its shared memory
+}
+
+template <int CL>
+cudaLaunchConfig_t sample_config(int rows, size_t smem, cudaStream_t stream, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(rows * CL));
+  cfg.blockDim = dim3(SAMPLE_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CL;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ls_dependent_launch ? 2 : 1;
+  return cfg;
+}
+
+// Rows that run at one time when each is spread over CL blocks (a block takes an SM's registers).
+template <int CL>
+int sample_rows_at_once() {
+  static int rows = 0;
+  if (rows == 0) {
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = sample_config<CL>(1, 0, nullptr, attr);
+    if (cudaOccupancyMaxActiveClusters(&rows, sample_cluster_kernel<CL>, &cfg) != cudaSuccess || rows <= 0) {
+      cudaGetLastError();
+      rows = 96 / CL;
+    }
+  }
+  return rows;
+}
+
+template <int CL>
+int launch_sample_cluster(const float* logits, const float* temperature, const float* top_p, const uint32_t* keys,
+                          const uint32_t* positions, int* out, int rows, int vocab, cudaStream_t stream) {
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(sample_cluster_kernel<CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SAMPLE_PART * (int)sizeof(float)) != cudaSuccess)
+      return LS_E_SMEM;
+    configured = true;
+  }
+  cudaLaunchAttribute attr[2];
+  const cudaLaunchConfig_t cfg = sample_config<CL>(rows, (size_t)((vocab + CL - 1) / CL) * sizeof(float), stream, attr);
+  LS_COUNT(LS_K_SAMPLE);
+  cudaLaunchKernelEx(&cfg, sample_cluster_kernel<CL>, logits, temperature, top_p, keys, positions, out, vocab);
+  return ls_launch_status();
 }
 
 // argmax in two stages, so that a few rows of a wide vocabulary fill the device:
@@ -566,9 +599,9 @@ LS_API int ls_argmax(const float* logits, int* out, void* scratch, int rows, int
 }
 
 // How many floats of scratch ls_sample needs for its probabilities: none where a row fits the
-// registers of a cluster (vocabularies up to 163,840), else rows x vocab.
+// shared memory of a cluster (vocabularies up to 163,840), else rows x vocab.
 LS_API long long ls_sample_scratch_floats(int rows, int vocab) {
-  return vocab <= SAMPLE_CLUSTER * SAMPLE_THREADS * SAMPLE_PER ? 0LL : (long long)rows * vocab;
+  return vocab <= SAMPLE_MOST ? 0LL : (long long)rows * vocab;
 }
 
 // probs: scratch of ls_sample_scratch_floats(rows, vocab) floats (may be null when that is 0).
@@ -577,11 +610,17 @@ LS_API int ls_sample(const float* logits, float* probs, const float* temperature
                      const float* top_p, const uint32_t* keys, const uint32_t* positions, int* out,
                      int rows, int vocab, cudaStream_t stream) {
   if (rows <= 0) return 0;
-  if (vocab <= SAMPLE_CLUSTER * SAMPLE_THREADS * SAMPLE_PER) {
-    // a row over the eight blocks of a cluster, its probabilities in registers
-    LS_COUNT(LS_K_SAMPLE), ls_launch(sample_cluster_kernel, rows * SAMPLE_CLUSTER, SAMPLE_THREADS, 0, stream, logits, temperature,
-                                     top_p, keys, positions, out, vocab);
-    return ls_launch_status();
+  if (vocab <= SAMPLE_MOST) {
+    // as many blocks a row as still run all rows at once (a row's token does not depend on how it is
+    // spread: 16 rows of 151,936 over 8 blocks each take two rounds, 66 us, over 4 one, 38); where no
+    // spread does, the fewest blocks that hold a row
+#define LS_SAMPLE_AS(CL) \
+  return launch_sample_cluster<CL>(logits, temperature, top_p, keys, positions, out, rows, vocab, stream)
+    if (vocab > 4 * SAMPLE_PART || rows <= sample_rows_at_once<8>()) LS_SAMPLE_AS(8);
+    if (vocab > 2 * SAMPLE_PART || rows <= sample_rows_at_once<4>()) LS_SAMPLE_AS(4);
+    if (vocab > SAMPLE_PART || rows <= sample_rows_at_once<2>()) LS_SAMPLE_AS(2);
+    LS_SAMPLE_AS(1);
+#undef LS_SAMPLE_AS
   }
   if (probs == nullptr) return LS_E_SIZE;
   LS_COUNT(LS_K_SAMPLE), ls_launch(sample_kernel, rows, SAMPLE_THREADS, 0, stream, logits, probs, temperature, top_p, keys,
@@ -592,6 +631,6 @@ LS_API int ls_sample(const float* logits, float* probs, const float* temperature
 LS_API const char* ls_constants_sampling() {
   static char buf[256];
   static const LsConstant c[] = {{"argmax.chunks", ARGMAX_CHUNKS}, {"sample.threads", SAMPLE_THREADS},
-                                 {"sample.cluster_blocks", SAMPLE_CLUSTER}, {"sample.kept_per_thread", SAMPLE_PER}};
+                                 {"sample.cluster_blocks", SAMPLE_CLUSTER}, {"sample.cluster_vocab", SAMPLE_MOST}};
   return ls_format_constants(buf, sizeof buf, c, (int)(sizeof c / sizeof c[0]));
 }
