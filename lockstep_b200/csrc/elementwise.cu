@@ -58,6 +58,19 @@ __device__ __forceinline__ float4 ls_load4(const TG* p) {
     return make_float4(__bfloat162float(a.x), __bfloat162float(a.y), __bfloat162float(b.x), __bfloat162float(b.y));
   }
 }
+// the same in two steps: the bits as they lie in memory, and their values
+template <typename TG>
+struct LsRaw4 {
+  float4 raw;
+  __device__ __forceinline__ void load(const TG* p) { raw = *reinterpret_cast<const float4*>(p); }
+  __device__ __forceinline__ float4 value() const { return raw; }
+};
+template <>
+struct LsRaw4<__nv_bfloat16> {
+  uint2 raw;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { raw = *reinterpret_cast<const uint2*>(p); }
+  __device__ __forceinline__ float4 value() const { return ls_load4<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(&raw)); }
+};
 template <typename TO>
 __device__ __forceinline__ void ls_store4(TO* p, float a, float b, float c, float d) {
   if constexpr (sizeof(TO) == 4) {
@@ -76,9 +89,17 @@ __device__ __forceinline__ void ls_store4(TO* p, float a, float b, float c, floa
 // rows may be gathered through row_index (the rows whose logits are wanted).
 // --------------------------------------------------------------------------
 // One warp per row: lane l takes the float4 groups l, l + 32, ... of the row, keeps
-// them in registers between the two passes (rows up to 8192 wide; wider rows are
+// the first KEEP of them in registers between the two passes (a wider row's rest is
 // read twice), sums its squares in that order and the lanes by an xor tree.  The
 // order depends on the width alone.
+// What bounds it: with few rows the chain launch, read, sum, write; with thousands the reads
+// and writes of L2.  KEEP is the smallest of 8, 16, 24 and 32 groups that holds the row (rows of
+// 1,024 to 4,096 elements), so that a row's reads are in flight together, and EARLY asks
+// for the gains, which no kernel writes, before the wait on the kernel before; with many rows
+// the registers of more than 8 groups and their gains would cost more rows an SM than that
+// saves (2,048 rows of 2,560 with 32 groups: 13.7 us, with 16 and late gains 8.0).  Back to back,
+// 6 rows of 1,024 / 2,560 / 4,096: 1.6 / 3.3 / 4.6 us (with 16 groups and late gains 3.2 / 5.9 / 9.0);
+// 2,048 rows of 1,024: 2.4 us (4.0), 12.6 MB read and written at 5.2 TB/s.
 // y[0..4) = x * rstd * gain, in one access each for the gains and the outputs where `vec`
 template <typename TO, typename TG>
 __device__ __forceinline__ void rmsnorm_out4(TO* y, const TG* gain, const float* x, float rstd, bool vec) {
@@ -91,19 +112,30 @@ __device__ __forceinline__ void rmsnorm_out4(TO* y, const TG* gain, const float*
   }
 }
 
-template <typename TO, typename TG>
+template <typename TO, typename TG, int KEEP, bool EARLY>
 __global__ void __launch_bounds__(128)
 rmsnorm_kernel(const float* __restrict__ x, const int* __restrict__ row_index,
                const TG* __restrict__ gain_all, TO* __restrict__ y, int rows, int width, int src_rows,
                float eps, int parts, int64_t x_ld, int* err) {
-  ls_dependency_sync();
-  constexpr int KEEP = 64;                    // floats a lane keeps: 16 float4
+  ls_dependency_trigger();
   const int lane = threadIdx.x & 31;
   // a row of `parts` equal consecutive parts, each normalised by its own root mean square, is
   // `parts` rows of `width` elements to this kernel (the gain runs over the whole row)
   const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (unit >= rows * parts) return;
   const int r = unit / parts, part = unit - r * parts;
+  const TG* gain = gain_all + (int64_t)part * width;
+  // four outputs an access where the outputs and the gains allow it (this changes no sum)
+  const bool vec_out = ((uintptr_t)y & (4 * sizeof(TO) - 1)) == 0 && ((uintptr_t)gain & (4 * sizeof(TG) - 1)) == 0;
+  const int groups = width >> 2;
+  const bool early = EARLY && vec_out && (width & 3) == 0;
+  LsRaw4<TG> gn[EARLY ? KEEP : 1];
+  if (early) {
+#pragma unroll
+    for (int i = 0; i < (EARLY ? KEEP : 0); ++i)
+      if (lane + 32 * i < groups) gn[i].load(gain + 4 * (lane + 32 * i));
+  }
+  ls_dependency_wait();
   int src = row_index ? row_index[r] : r;
   if (src < 0 || src >= src_rows) {
     if (lane == 0) ls_record_fault(err, LS_DEV_ROW_RANGE, r);
@@ -112,23 +144,19 @@ rmsnorm_kernel(const float* __restrict__ x, const int* __restrict__ row_index,
   // (x_ld: the source rows' pitch, where the normed columns are the first of a wider row)
   const float* xr = x + (int64_t)src * x_ld + (int64_t)part * width;
   TO* yr = y + ((int64_t)r * parts + part) * width;
-  const TG* gain = gain_all + (int64_t)part * width;
   const bool vec = (width & 3) == 0 && ((uintptr_t)xr & 15) == 0;
-  // four outputs an access where the outputs and the gains allow it (this changes no sum)
-  const bool vec_out = ((uintptr_t)y & (4 * sizeof(TO) - 1)) == 0 && ((uintptr_t)gain & (4 * sizeof(TG) - 1)) == 0;
-  float keep[KEEP];
+  float keep[4 * KEEP];
   float ss = 0.f;
   if (vec) {
-    const int groups = width >> 2;
 #pragma unroll
-    for (int i = 0; i < KEEP / 4; ++i) {
+    for (int i = 0; i < KEEP; ++i) {
       const int g = lane + 32 * i;
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       if (g < groups) v = *reinterpret_cast<const float4*>(xr + 4 * g);
       keep[4 * i + 0] = v.x; keep[4 * i + 1] = v.y; keep[4 * i + 2] = v.z; keep[4 * i + 3] = v.w;
       ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
     }
-    for (int g = lane + 32 * (KEEP / 4); g < groups; g += 32) {
+    for (int g = lane + 32 * KEEP; g < groups; g += 32) {
       const float4 v = *reinterpret_cast<const float4*>(xr + 4 * g);
       ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
     }
@@ -138,13 +166,19 @@ rmsnorm_kernel(const float* __restrict__ x, const int* __restrict__ row_index,
   ss = ls_warp_sum(ss);
   const float rstd = 1.0f / sqrtf(ss / (float)width + eps);
   if (vec) {
-    const int groups = width >> 2;
 #pragma unroll
-    for (int i = 0; i < KEEP / 4; ++i) {
+    for (int i = 0; i < KEEP; ++i) {
       const int g = lane + 32 * i;
-      if (g < groups) rmsnorm_out4<TO, TG>(yr + 4 * g, gain + 4 * g, keep + 4 * i, rstd, vec_out);
+      if (g >= groups) continue;
+      if (early) {
+        const float4 gi = gn[EARLY ? i : 0].value();
+        ls_store4<TO>(yr + 4 * g, keep[4 * i] * rstd * gi.x, keep[4 * i + 1] * rstd * gi.y, keep[4 * i + 2] * rstd * gi.z,
+                      keep[4 * i + 3] * rstd * gi.w);
+      } else {
+        rmsnorm_out4<TO, TG>(yr + 4 * g, gain + 4 * g, keep + 4 * i, rstd, vec_out);
+      }
     }
-    for (int g = lane + 32 * (KEEP / 4); g < groups; g += 32) {
+    for (int g = lane + 32 * KEEP; g < groups; g += 32) {
       const float4 v = *reinterpret_cast<const float4*>(xr + 4 * g);
       const float four[4] = {v.x, v.y, v.z, v.w};
       rmsnorm_out4<TO, TG>(yr + 4 * g, gain + 4 * g, four, rstd, vec_out);
@@ -166,15 +200,24 @@ LS_API int ls_rmsnorm(const float* x, const int* row_index, const void* gain, in
   // few rows: one warp per block, so that the rows spread over the device
   const int warps = (int64_t)rows * parts >= 1024 ? 4 : 1;
   const int blocks = (rows * parts + warps - 1) / warps;
-#define LS_RMS(TO, TG)                                                                          \
-  LS_COUNT(LS_K_RMSNORM), ls_launch(rmsnorm_kernel<TO, TG>, blocks, warps * 32, 0, stream, x, row_index, (const TG*)gain, (TO*)y, \
-                                                            rows, width, src_rows, eps, parts, x_ld, err)
+#define LS_RMS_AS(TO, TG, KEEP, EARLY)                                                                              \
+  LS_COUNT(LS_K_RMSNORM), ls_launch(rmsnorm_kernel<TO, TG, KEEP, EARLY>, blocks, warps * 32, 0, stream, x, row_index, \
+                                    (const TG*)gain, (TO*)y, rows, width, src_rows, eps, parts, x_ld, err)
+#define LS_RMS(TO, TG)                                              \
+  do {                                                              \
+    if (width <= 1024) LS_RMS_AS(TO, TG, 8, true);                  \
+    else if (warps > 1) LS_RMS_AS(TO, TG, 16, false);               \
+    else if (width <= 2048) LS_RMS_AS(TO, TG, 16, true);            \
+    else if (width <= 3072) LS_RMS_AS(TO, TG, 24, true);            \
+    else LS_RMS_AS(TO, TG, 32, (sizeof(TG) == 2));                  \
+  } while (0)
   if (y_dtype == LS_F32 && gain_dtype == LS_F32) LS_RMS(float, float);
   else if (y_dtype == LS_F32 && gain_dtype == LS_BF16) LS_RMS(float, __nv_bfloat16);
   else if (y_dtype == LS_BF16 && gain_dtype == LS_F32) LS_RMS(__nv_bfloat16, float);
   else if (y_dtype == LS_BF16 && gain_dtype == LS_BF16) LS_RMS(__nv_bfloat16, __nv_bfloat16);
   else return LS_E_DTYPE;
 #undef LS_RMS
+#undef LS_RMS_AS
   return ls_launch_status();
 }
 

@@ -75,3 +75,30 @@ def test_rows_that_are_no_distribution_give_token_0_or_the_numbers_in_them():
     got = _draw(k, logits, one, torch.tensor([1.0, 0.9, 1.0, 0.9, 1.0]), [f"r{i}" for i in range(5)], [1] * 5)
     assert got[:4] == [0, 0, 0, 0]
     assert got[4] in (0, 7, 8)                                               # -3e38 / 0.5 is -inf in float32
+
+
+# ---------------------------------------------------------------------------
+# rmsnorm: rows kept in 8, 16, 24 or 32 groups a lane
+# ---------------------------------------------------------------------------
+
+@pytest.mark.parametrize("parts", [1, 2])
+@pytest.mark.parametrize("width", [1020, 1024, 1028, 2048, 2052, 3072, 3076, 4096, 4100, 6146])
+def test_a_normed_row_has_the_same_bits_among_few_and_many_rows(width, parts):
+    k = K()
+    g = torch.Generator().manual_seed(width + parts)
+    rows = 1030
+    x = (torch.randn(rows, width * parts, generator=g) * 3).to(dev())
+    err = k.new_error_word(dev())
+    for gain_dtype, out_dtype in ((torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32)):
+        gain = (1 + 0.1 * torch.randn(width * parts, generator=g)).to(gain_dtype).to(dev())
+        many = torch.empty(rows, width * parts, dtype=out_dtype, device=dev())
+        k.rmsnorm(x, gain, many, 1e-6, err, groups=parts)
+        few = torch.empty(3, width * parts, dtype=out_dtype, device=dev())
+        k.rmsnorm(x, gain, few, 1e-6, err, torch.tensor([1029, 0, 500], dtype=torch.int32, device=dev()), groups=parts)
+        assert torch.equal(few, many[[1029, 0, 500]])
+        part = x.double().view(rows, parts, width)
+        want = (part * torch.rsqrt((part * part).mean(-1, keepdim=True) + 1e-6)).view(rows, -1) * gain.double()
+        # a float32 sum of `width` squares in 32 lanes, then three roundings; bfloat16 results round once more
+        bound = 1e-6 if out_dtype == torch.float32 else 2.0 ** -8
+        assert ((many.double() - want).abs() <= bound * (want.abs() + 1e-3)).all()
+    k.raise_on_fault(err)
