@@ -127,6 +127,53 @@ __device__ __forceinline__ void ls_qkv_head_write_as(const LsQkvStore& a, const 
                            [&](int i, float v) { dst[i] = ls_from_float<T>(v); }, a.interleaved != 0);
 }
 
+// What finishing a head of D = 64 or 128 elements that is rotated whole reads besides the head itself, a
+// lane's part of it: constants and the step's inputs, so that a kernel may ask for them before the values of the
+// head exist.  `used`: the head is such a one and goes somewhere, q or k (a v head only moves).
+template <int D>
+struct LsHeadTables {
+  float gain[D / 32], cs[D / 64], sn[D / 64];
+  bool used;
+  __device__ __forceinline__ void fetch(const LsQkvStore& a, const LsHeadTarget& target, int lane) {
+    used = a.d == D && a.rot_dim == D && !a.interleaved && target.dst != nullptr && target.kind != 2;
+    if (!used) return;
+    const void* g = target.kind == 0 ? a.q_gain : a.k_gain;
+#pragma unroll
+    for (int j = 0; j < D / 32; ++j)
+      gain[j] = g == nullptr ? 1.f
+                : a.gain_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(g)[lane + 32 * j])
+                              : reinterpret_cast<const float*>(g)[lane + 32 * j];
+#pragma unroll
+    for (int j = 0; j < D / 64; ++j) {
+      cs[j] = a.cos_table[(int64_t)target.pos * (D / 2) + lane + 32 * j];
+      sn[j] = a.sin_table[(int64_t)target.pos * (D / 2) + lane + 32 * j];
+    }
+  }
+  // the head's values normed, rotated and written: ls_norm_rope_head's sums and products in its order
+  // (a product with a gain of 1 where there is no norm changes no bit)
+  template <typename T>
+  __device__ __forceinline__ void write(const LsQkvStore& a, const T* src, const LsHeadTarget& target, int lane) const {
+    float v[D / 32], rstd = 1.f;
+#pragma unroll
+    for (int j = 0; j < D / 32; ++j) v[j] = ls_to_float<T>(src[lane + 32 * j]);
+    if ((target.kind == 0 ? a.q_gain : a.k_gain) != nullptr) {
+      float ss = 0.f;
+#pragma unroll
+      for (int j = 0; j < D / 32; ++j) ss = fmaf(v[j], v[j], ss);
+      ss = ls_warp_sum(ss);
+      rstd = 1.0f / sqrtf(ss / (float)D + a.eps);
+    }
+    T* dst = reinterpret_cast<T*>(target.dst);
+#pragma unroll
+    for (int j = 0; j < D / 64; ++j) {
+      const float lo = __fmul_rn(__fmul_rn(v[j], rstd), gain[j]);
+      const float hi = __fmul_rn(__fmul_rn(v[j + D / 64], rstd), gain[j + D / 64]);
+      dst[lane + 32 * j] = ls_from_float<T>(__fsub_rn(__fmul_rn(lo, cs[j]), __fmul_rn(hi, sn[j])));
+      dst[lane + 32 * j + D / 2] = ls_from_float<T>(__fadd_rn(__fmul_rn(hi, cs[j]), __fmul_rn(lo, sn[j])));
+    }
+  }
+};
+
 template <typename T>
 __device__ __forceinline__ void ls_qkv_head_write(const LsQkvStore& a, const T* src, const LsHeadTarget& target,
                                                   int lane) {
