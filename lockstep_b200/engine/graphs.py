@@ -19,7 +19,7 @@ capacity with null items, which the kernels skip.  Nothing about the
 arithmetic changes: the same kernels run on the same values.
 
 Steps that mix portions of prompts (a step that fills the token budget, say) are recorded too,
-keyed by their exact number of tokens and the rounded numbers of wanted rows and split items,
+keyed by their exact number of tokens and the rounded numbers of wanted rows, split items and portions,
 when a step of the same shape comes for the third time: such steps launch some 300 kernels, and the
 host is slower at enqueueing them than the device at running them.
 
@@ -143,12 +143,14 @@ class StaticStepContext:
         self._pending = True
 
 
-MIXED_MIN_TOKENS = 256   # steps of fewer tokens are not worth a graph of their own
+MIXED_SHORT = 256        # steps of fewer tokens are a class of their own: they come in more shapes
 MIXED_GRAPHS = 8         # recorded steps of mixed portions kept (least recently used goes first)
+SHORT_GRAPHS = 16        # the same of short ones
 MIXED_SPLIT_STEP = 64    # the split work list of such a step holds this many items, or a power of two times as many
-MIXED_PORTIONS = 4       # portions of two or more tokens such a step may hold
+MIXED_PORTIONS = (4, 16)  # portions of two or more tokens such a step may hold: the smallest that does is part of its shape
+SHORT_WANTED = 8         # wanted rows of a short step, or a multiple of sixty-four
 MIXED_SIGHTINGS = 3      # a shape is recorded when it comes for this many times
-MIXED_RECORDINGS = 48    # recordings of such steps in a runner's life: a workload of ever new shapes stops recording
+MIXED_RECORDINGS = 48    # recordings of either class in a runner's life: a workload of ever new shapes stops recording
 
 
 class StaticMixedContext:
@@ -158,7 +160,7 @@ class StaticMixedContext:
     and the attention work lists are padded to capacities (with the first wanted row again, whose
     logits are dropped, and with null items, which the kernels skip)."""
 
-    def __init__(self, tokens: int, wanted_cap: int, split_cap: int, max_entries: int,
+    def __init__(self, tokens: int, wanted_cap: int, split_cap: int, portions: int, max_entries: int,
                  plan_keys: list[tuple], device, err, split_size: int):
         self.num_tokens, self.n_wanted = tokens, wanted_cap
         self.split_cap, self.max_entries = split_cap, max_entries
@@ -167,7 +169,7 @@ class StaticMixedContext:
         t = tokens
         # (a few items more than the tokens make in one portion: a launcher that chooses a kernel
         # by the number of items then sees about the real number)
-        self._tile_cap = {key: t // key[1] + MIXED_PORTIONS for key in self.plan_keys}
+        self._tile_cap = {key: t // key[1] + portions for key in self.plan_keys}
         size = 3 * t + wanted_cap
         self._off = {}
         for key in self.plan_keys:
@@ -263,7 +265,7 @@ class DecodeGraphs:
         self.mixed: OrderedDict[tuple, tuple] = OrderedDict()
         self.mixed_seen: OrderedDict[tuple, int] = OrderedDict()
         self.mixed_replays = 0
-        self.mixed_recordings = 0
+        self.mixed_recordings = {False: 0, True: 0}          # by whether the step is a short one
 
     def capacity_for(self, entries) -> int:
         n = split_items(entries, self.windows, self.runner.split_size)
@@ -340,17 +342,22 @@ class DecodeGraphs:
 
     # -- steps that mix portions of prompts and decoded tokens --------------
     def mixed_key_for(self, entries) -> tuple | None:
-        """(tokens, wanted rows, split items) of the recorded step that would serve ``entries``, the
-        last two rounded up; None for steps too small to be worth recording, with more portions
-        than its tile work lists are made for, or with more wanted rows than requests can be live."""
+        """(tokens, wanted rows, split items, portions) of the recorded step that would serve ``entries``, the last three
+        rounded up; None for steps without portions, with more portions than tile work lists are made for, or with more
+        wanted rows than requests can be live."""
         tokens = sum(len(e.tokens) for e in entries)
-        if tokens < MIXED_MIN_TOKENS or len(entries) > self.runner.cache.max_live:
+        max_live = self.runner.cache.max_live
+        if len(entries) > max_live:
             return None
         wanted = sum(len(e.want) for e in entries)
         singles = [e for e in entries if len(e.tokens) == 1]
+        portions = len(entries) - len(singles)
+        if not portions:
+            return None
         splits = split_items(singles, self.windows, self.runner.split_size) if singles else 0
-        # the tile work lists hold what the tokens can make in up to MIXED_PORTIONS portions
-        if sum(len(e.tokens) > 1 for e in entries) > MIXED_PORTIONS:
+        # the tile work lists hold what the tokens can make in up to so many portions
+        portions = next((cap for cap in MIXED_PORTIONS if portions <= cap), None)
+        if portions is None or wanted > max_live:
             return None
         # few classes, so that a continuous batch whose decoded rows come and go records a
         # handful of steps and not one per mix: wanted rows in sixty-fours (at most as many as requests may be live),
@@ -360,16 +367,15 @@ class DecodeGraphs:
             split_cap = MIXED_SPLIT_STEP
             while split_cap < splits:
                 split_cap *= 2
-        if wanted > self.runner.cache.max_live:
-            return None
-        return tokens, min(self.runner.cache.max_live, -(-max(wanted, 1) // 64) * 64), split_cap
+        wanted_cap = SHORT_WANTED if tokens < MIXED_SHORT and wanted <= SHORT_WANTED else -(-max(wanted, 1) // 64) * 64
+        return tokens, min(max_live, wanted_cap), split_cap, portions
 
     def mixed_ready(self, key) -> bool:
         return key in self.mixed
 
     def mixed_seen_again(self, key) -> bool:
         """Counts a step of this shape that ran unrecorded; True from the MIXED_SIGHTINGS-th on."""
-        if self.mixed_recordings >= MIXED_RECORDINGS:
+        if self.mixed_recordings[key[0] < MIXED_SHORT] >= MIXED_RECORDINGS:
             return False
         n = self.mixed_seen.pop(key, 0) + 1
         self.mixed_seen[key] = n
@@ -378,14 +384,17 @@ class DecodeGraphs:
         return n >= MIXED_SIGHTINGS
 
     def record_mixed(self, key, plan_keys) -> None:
-        tokens, wanted_cap, split_cap = key
+        tokens, wanted_cap, split_cap, portions = key
         r = self.runner
-        ctx = StaticMixedContext(tokens, wanted_cap, split_cap, r.cache.max_live, list(plan_keys), r.device,
+        ctx = StaticMixedContext(tokens, wanted_cap, split_cap, portions, r.cache.max_live, list(plan_keys), r.device,
                                  r.err, r.split_size)
         self.mixed[key] = self._record(ctx)
-        self.mixed_recordings += 1
-        while len(self.mixed) > MIXED_GRAPHS:
-            dropped, _ = self.mixed.popitem(last=False)
+        short = tokens < MIXED_SHORT
+        self.mixed_recordings[short] += 1
+        # the two classes do not push each other's recordings out
+        kept = [k for k in self.mixed if (k[0] < MIXED_SHORT) == short]
+        for dropped in kept[:max(0, len(kept) - (SHORT_GRAPHS if short else MIXED_GRAPHS))]:
+            del self.mixed[dropped]
             self.mixed_seen.pop(dropped, None)        # it has to come three times again
             self.dropped += 1
 
