@@ -15,7 +15,7 @@ import hashlib
 import json
 
 _SOURCES = {
-    "core": ["attention_simt", "gemm_simt", "sampling"],
+    "core": ["attention_simt", "attention_rows", "gemm_simt", "sampling"],
     "tc": ["gemm_tc", "attention_decode_mma", "attention_prefill_tc"],
     "seq": ["recurrent", "state_rules", "experts", "experts_tc"],
 }

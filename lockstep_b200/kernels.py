@@ -78,6 +78,9 @@ _SIGNATURES = {
         "ls_attention_tile": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                               c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                               c_float, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
+        "ls_attention_rows_tile_tokens": [c_int, c_int, c_int],
+        "ls_attention_rows": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                              c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
         "ls_attention_decode": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int,
                                 c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
                                 c_void_p, c_void_p, c_void_p, c_void_p],
@@ -595,6 +598,31 @@ def attention_tile(q, pages, out, part_acc, part_ml, work, n_work, block_table, 
         block_table.shape[-1], nq, nkv, d, pages.shape[3], pages.shape[0], int(window), int(keep_first), float(scale),
         float(softcap), _slopes(slopes, nq), _slopes(log_rates, nq), _slopes(sinks, nq), _dev(err, "err", torch.int32),
         _stream()), "attention_tile")
+
+
+def attention_rows_tile_tokens(tokens: int, nq: int, d: int, dtype) -> int:
+    """Tokens of a work item for the float32 attention of a step of ``tokens`` tokens: 64 or 32 where ``attention_rows``
+    serves it best, 16 for ``attention_tile`` (other types, other head sizes, few rows)."""
+    if dtype != torch.float32:
+        return 16
+    return int(library().ls_attention_rows_tile_tokens(int(tokens), int(nq), int(d)))
+
+
+def attention_rows(q, pages, out, work, n_work, tile_tokens, block_table, nq, nkv, d, window, scale, err, slopes=None,
+                   log_rates=None, sinks=None, softcap: float = 0.0, keep_first: int = 0) -> bool:
+    """``attention_tile`` of prompt portions for float32 heads of 64 or 128 elements, with the same bits, for work items of
+    up to ``tile_tokens`` (32 or 64) tokens (csrc/attention_rows.cu).  Returns False, having launched nothing, for sizes and
+    addresses it does not take: the caller then needs a plan of 16-token items for ``attention_tile``."""
+    status = library().ls_attention_rows(
+        _dev(q, "q", torch.float32), _dev(pages, "pages", torch.float32), _dev(out, "out", torch.float32),
+        _dev(work, "work", torch.int32), n_work, int(tile_tokens), _dev(block_table, "block_table", torch.int32),
+        block_table.shape[-1], nq, nkv, d, pages.shape[3], pages.shape[0], int(window), int(keep_first), float(scale),
+        float(softcap), _slopes(slopes, nq), _slopes(log_rates, nq), _slopes(sinks, nq), _dev(err, "err", torch.int32),
+        _stream())
+    if status in (-2, -3):
+        return False
+    _check(status, "attention_rows")
+    return True
 
 
 def attention_decode(q, pages, part_acc, part_ml, work, n_work, block_table, nq, nkv, d, window,

@@ -118,6 +118,15 @@ def attend(rt: Runtime, q, ctx, cache, nq: int, nkv: int, d: int, mask, scale: f
             q, cache.pages, attn, plan.tile_work, plan.n_tile, cache.block_table, nq, nkv, d,
             window, scale, rt.err, extras.slopes, extras.log_rates, extras.sinks, softcap=extras.softcap,
             keep_first=keep)
+    if exact:
+        # float32: tiles of more tokens where the step has enough rows to fill the device with them
+        tile_tokens = K.attention_rows_tile_tokens(t, nq, d, q.dtype)
+        if tile_tokens > 16:
+            plan = ctx.attention_plan(mask, tile_tokens)
+            done = not plan.n_tile or K.attention_rows(
+                q, cache.pages, attn, plan.tile_work, plan.n_tile, tile_tokens, cache.block_table, nq, nkv, d,
+                window, scale, rt.err, extras.slopes, extras.log_rates, extras.sinks, softcap=extras.softcap,
+                keep_first=keep)
     if not done:
         plan = ctx.attention_plan(mask)
         if plan.n_tile:

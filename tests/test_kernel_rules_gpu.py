@@ -102,3 +102,93 @@ def test_a_normed_row_has_the_same_bits_among_few_and_many_rows(width, parts):
         bound = 1e-6 if out_dtype == torch.float32 else 2.0 ** -8
         assert ((many.double() - want).abs() <= bound * (want.abs() + 1e-3)).all()
     k.raise_on_fault(err)
+
+# ---------------------------------------------------------------------------
+# float32 products: few tokens on lanes, many tokens in tiles of several sizes
+# ---------------------------------------------------------------------------
+
+@pytest.mark.parametrize("epilogue", ["store", "residual", "silu", "gelu", "relu2"])
+@pytest.mark.parametrize("n,k_", [(1000, 1060), (2048, 128), (2049, 260), (20000, 64)])
+def test_a_float32_row_has_the_same_bits_in_every_batch(n, k_, epilogue):
+    k = K()
+    g = torch.Generator().manual_seed(n)
+    code = {"store": k.EPILOGUE_STORE, "residual": k.EPILOGUE_RESIDUAL, "silu": k.EPILOGUE_SILU_MUL, "gelu": k.EPILOGUE_GELU,
+            "relu2": k.EPILOGUE_RELU2}[epilogue]
+    x = torch.randn(700, k_, generator=g).to(dev())
+    w = (torch.randn(2 * n if epilogue == "silu" else n, k_, generator=g) / math.sqrt(k_)).to(dev())
+    base = torch.randn(700, n, generator=g).to(dev())
+    rows = {}
+    for m in (1, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129, 300, 700):
+        c = base[:m].clone()
+        k.gemm_nt_simt(x[:m], w, c, code)
+        rows[m] = c
+    for m, c in rows.items():
+        assert torch.equal(c, rows[700][:m]), m
+    z = x.double() @ w.double().T
+    gelu = lambda a: torch.nn.functional.gelu(a, approximate="tanh")
+    want = {"store": lambda: z, "residual": lambda: base.double() + z, "gelu": lambda: gelu(z), "relu2": lambda: z.clamp(min=0) ** 2,
+            "silu": lambda: torch.nn.functional.silu(z[:, :n]) * z[:, n:]}[epilogue]()
+    # one chain of k_ float32 products of size 1 / sqrt(k_): an error of a few 2^-24 sqrt(k_) against |z| of about 1
+    assert (rows[700].double() - want).abs().max() <= 2.0 ** -21 * math.sqrt(k_) * (1 + float(want.abs().max()))
+
+
+# ---------------------------------------------------------------------------
+# float32 attention of prompt portions: tiles of 16, 32 and 64 tokens
+# ---------------------------------------------------------------------------
+
+@pytest.mark.parametrize("nq,nkv,d,portions,mask,extra", [
+    (4, 2, 128, [(0, 300), (513, 65)], 0, None), (2, 2, 64, [(0, 2), (255, 129), (0, 63)], 0, None),
+    (4, 1, 128, [(300, 200)], 100, "sinks"), (2, 1, 64, [(700, 130)], (50, 5), "slopes"),
+    (4, 2, 128, [(100, 333)], -64, "log"), (2, 2, 128, [(0, 70), (900, 64)], (64, 300), "cap"), (2, 1, 64, [(640, 64)], -256, None)])
+def test_float32_attention_has_the_same_bits_in_tiles_of_every_size(nq, nkv, d, portions, mask, extra):
+    from lockstep_b200.engine.batch import mask_parts, plan_attention
+
+    k = K()
+    page = 16
+    g = torch.Generator().manual_seed(d + len(portions))
+    tokens = sum(n for _, n in portions)
+    pages_of = [-(-(s + n) // page) for s, n in portions]
+    num_pages = sum(pages_of) + 2
+    table = torch.zeros(len(portions), max(pages_of) + 1, dtype=torch.int32)
+    ids, at, rows, off = torch.randperm(num_pages, generator=g), 0, [], 0
+    for i, (s, n) in enumerate(portions):
+        table[i, :pages_of[i]] = ids[at:at + pages_of[i]].to(torch.int32)
+        at += pages_of[i]
+        rows.append((i, off, s, n))
+        off += n
+    q = torch.randn(tokens, nq * d, generator=g).to(dev())
+    pages = torch.randn(num_pages, 2, nkv, page, d, generator=g).to(dev())
+    table = table.to(dev())
+    slopes = (torch.rand(nq, generator=g) * 0.3).to(dev()) if extra in ("slopes", "log") else None
+    rates = torch.rand(nq, generator=g).to(dev()) if extra == "log" else None
+    sinks = torch.randn(nq, generator=g).to(dev()) if extra == "sinks" else None
+    cap = 5.0 if extra == "cap" else 0.0
+    window, keep = mask_parts(mask)
+    err = k.new_error_word(dev())
+    outs = {}
+    for size in (16, 32, 64):
+        tile = plan_attention(rows, mask, k.attention_split_size(), size)[0]
+        work = torch.from_numpy(tile).to(dev())
+        out = torch.full_like(q, float("nan"))
+        if size == 16:
+            k.attention_tile(q, pages, out, None, None, work, len(tile), table, nq, nkv, d, window, d ** -0.5, err, slopes,
+                             rates, sinks, softcap=cap, keep_first=keep)
+        else:
+            assert k.attention_rows(q, pages, out, work, len(tile), size, table, nq, nkv, d, window, d ** -0.5, err, slopes,
+                                    rates, sinks, softcap=cap, keep_first=keep)
+        outs[size] = out
+    k.raise_on_fault(err)
+    assert bool(torch.isfinite(outs[16]).all())
+    assert torch.equal(outs[16], outs[32]) and torch.equal(outs[16], outs[64])
+
+
+def test_float32_attention_declines_what_it_does_not_cover():
+    k = K()
+    assert k.attention_rows_tile_tokens(4096, 16, 128, torch.bfloat16) == 16
+    assert k.attention_rows_tile_tokens(4096, 16, 96, torch.float32) == 16
+    assert k.attention_rows_tile_tokens(3, 16, 128, torch.float32) == 16
+    assert k.attention_rows_tile_tokens(4096, 16, 128, torch.float32) == 64
+    q = torch.zeros(64, 96, device=dev())
+    pages = torch.zeros(4, 2, 1, 16, 96, device=dev())
+    work, table = torch.zeros(1, 8, dtype=torch.int32, device=dev()), torch.zeros(1, 4, dtype=torch.int32, device=dev())
+    assert not k.attention_rows(q, pages, torch.empty_like(q), work, 1, 64, table, 1, 1, 96, 0, 1.0, k.new_error_word(dev()))
