@@ -1944,6 +1944,16 @@ LS_API int ls_gemm_nt_tc_rmsnorm(const float* h, const int* row_index, int src_r
   return run(nullptr, &norm, nullptr, W, C, c_dtype, T, N, K, 0, ldw, ldc, epilogue, err, stream);
 }
 
+// Whether the norm is better made inside the product of T tokens (1) or by ls_rmsnorm before it (0); the
+// bits are the same.  Inside saves a launch, and every block norms all rows of its tile again, a trip to L2 for
+// the sums and one for every 128 columns of its share, a warp two rows at a time.  Measured behind a residual
+// product (us, inside / apart): 8 rows of 1,024, 4,096 features 6.1 / 6.2, 16 rows 8.2 / 7.0, 32 rows 12.5 / 8.3; 8 rows
+// of 2,048 with a share of 512 columns 8.2 / 8.8, of 1,024 columns 11.5 / 10.7; 8 rows of 2,560 20.5 / 15.6; a norm in
+// two parts, 2 trips for the sums and a division a group: 8 rows 14.0 / 9.9, 1 row 11.9 / 8.4.
+LS_API int ls_gemm_tc_norm_inside(int T, int N, int K, int epilogue, int parts) {
+  return T <= 8 && parts == 1 && K <= 2048 && make_plan(T, N, K, epilogue).kb_per_share <= 8 ? 1 : 0;
+}
+
 // The q/k/v projection of few tokens with its heads finished in the epilogue: what
 // ls_gemm_nt_tc (or ls_gemm_nt_tc_rmsnorm when h is given instead of X) followed by
 // ls_qk_norm_rope_store writes, bit for bit, without the projection going through memory.

@@ -95,6 +95,7 @@ _SIGNATURES = {
 _SIGNATURES["tc"] = {
     "ls_gemm_tc_token_tile": [c_int, c_int, c_int, c_int],
     "ls_gemm_tc_k_shares": [c_int, c_int],
+    "ls_gemm_tc_norm_inside": [c_int, c_int, c_int, c_int, c_int],
     "ls_attention_decode_mma": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int,
                                 c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p,
                                 c_void_p, c_void_p],
@@ -741,6 +742,14 @@ def gemm_nt_tc(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, epilogue: int,
         return False
     _check(status, "gemm_nt_tc")
     return True
+
+
+def norm_inside_pays(tokens: int, features: int, w: torch.Tensor, epilogue: int = EPILOGUE_STORE, groups: int = 1) -> bool:
+    """Whether the RMSNorm in front of a product of ``tokens`` rows with ``w`` is better made inside the product
+    (``gemm_nt_tc_rmsnorm``, ``gemm_nt_tc_qkv_heads``) than by a kernel before it; the bits are the same."""
+    if not USE_TENSOR_CORES[0] or w.dtype != torch.bfloat16:
+        return False
+    return bool(library("tc").ls_gemm_tc_norm_inside(int(tokens), int(features), w.shape[1], int(epilogue), int(groups)))
 
 
 def gemm_nt_tc_rmsnorm(h: torch.Tensor, gain: torch.Tensor, eps: float, w: torch.Tensor, c: torch.Tensor,

@@ -351,7 +351,8 @@ class GQAttention(Mixer):
         fused = False
         if t <= K.FEW_TOKENS and not self.exact and not interleaved:
             # (the product that finishes its heads knows the norm over the whole row only)
-            pending = isinstance(x, NormedRows) and x.pending() and x.groups == 1
+            pending = isinstance(x, NormedRows) and x.pending() and x.groups == 1 \
+                and K.norm_inside_pays(t, self.w_qkv.shape[0], self.w_qkv)
             fused = K.gemm_nt_tc_qkv_heads(None if pending else (x.materialize() if isinstance(x, NormedRows) else x),
                                            self.w_qkv, *heads,
                                            normed=(x.h, x.gain, x.eps, x.row_index) if pending else None)

@@ -131,7 +131,8 @@ class LatentAttention(Mixer):
             K.gemm_nt(x, self.w_q_down, raw, err=rt.err)
             queries = rt.rows(t, H * (self.d + self.dr))
             # (few tokens: the second map's product norms its rows itself, with the bits of the separate kernel)
-            if not K.gemm_nt_tc_rmsnorm(raw, self.q_gain, self.eps, self.w_q_up, queries, K.EPILOGUE_STORE, rt.err):
+            if not K.norm_inside_pays(t, queries.shape[1], self.w_q_up) or \
+                    not K.gemm_nt_tc_rmsnorm(raw, self.q_gain, self.eps, self.w_q_up, queries, K.EPILOGUE_STORE, rt.err):
                 cq = rt.rows(t, self.q_rank)
                 K.rmsnorm(raw, self.q_gain, cq, self.eps, rt.err)
                 K.gemm_nt(cq, self.w_q_up, queries, err=rt.err)

@@ -39,9 +39,9 @@ class NormedRows:
         return self._out
 
     def linear(self, w: torch.Tensor, out: torch.Tensor, epilogue: int, err: torch.Tensor) -> None:
-        """out = epilogue(norm(h) @ w.T): fused where the kernel allows, else norm, then product."""
-        if self._out is None and K.gemm_nt_tc_rmsnorm(self.h, self.gain, self.eps, w, out, epilogue, err,
-                                                      self.row_index, self.groups):
+        """out = epilogue(norm(h) @ w.T): fused where that pays and the kernel allows, else norm, then product."""
+        if self._out is None and K.norm_inside_pays(*out.shape, w, epilogue, self.groups) and \
+                K.gemm_nt_tc_rmsnorm(self.h, self.gain, self.eps, w, out, epilogue, err, self.row_index, self.groups):
             return
         K.gemm_nt(self.materialize(), w, out, epilogue, err=err)
 

@@ -73,14 +73,6 @@ def _f32(t: torch.Tensor) -> torch.Tensor:
     return t.to(torch.float32).contiguous()
 
 
-def _product(x, w, out, err) -> None:
-    """out = x @ w.T, the norm of ``x`` made inside where it is still to be made and the kernel can."""
-    if isinstance(x, NormedRows):
-        x.linear(w, out, K.EPILOGUE_STORE, err)
-    else:
-        K.gemm_nt(x, w, out, err=err)
-
-
 class GatedDelta(Mixer):
     graph_safe = True
     accepts_normed_rows = True       # its one product of the mixer's input can make the norm itself
@@ -154,8 +146,9 @@ class GatedDelta(Mixer):
         rt, tokens = self.rt, residual.shape[0]
         f32 = torch.float32
         proj, gates = rt.rows(tokens, self.w_in.shape[0]), rt.rows(tokens, 2 * self.H, dtype=f32)
-        _product(x, self.w_in, proj, rt.err)
-        _product(x, self.w_gates, gates, rt.err)
+        x = x.materialize() if isinstance(x, NormedRows) else x          # two products share the normed rows
+        K.gemm_nt(x, self.w_in, proj, err=rt.err)
+        K.gemm_nt(x, self.w_gates, gates, err=rt.err)
         qkv = rt.rows(tokens, self.C, dtype=f32)
         decay, beta = rt.rows(tokens, self.H, dtype=f32), rt.rows(tokens, self.H, dtype=f32)
         K.delta_prep(proj, self.conv_w, self.dt_bias, self.a_log, cache.state, ctx.token_slot, qkv, decay, beta,
@@ -479,8 +472,9 @@ class MLstm(Mixer):
     def forward(self, x, ctx, cache, residual, overwrite=False):
         rt, tokens, at = self.rt, residual.shape[0], self.at
         proj, gates = rt.rows(tokens, self.w_in.shape[0]), rt.rows(tokens, 2 * self.H, dtype=torch.float32)
-        _product(x, self.w_in, proj, rt.err)
-        _product(x, self.w_gates, gates, rt.err)
+        x = x.materialize() if isinstance(x, NormedRows) else x          # two products share the normed rows
+        K.gemm_nt(x, self.w_in, proj, err=rt.err)
+        K.gemm_nt(x, self.w_gates, gates, err=rt.err)
         portions, cap = portion_list(ctx, cache.state, rt)
         o = rt.rows(tokens, self.H * (self.dv + 2), dtype=torch.float32)
         K.state_rule(K.RULE_MLSTM, rt.dtype, portions, cap, cache.state, proj[:, at["q"]:at["q"] + self.Kd],

@@ -192,3 +192,39 @@ def test_float32_attention_declines_what_it_does_not_cover():
     pages = torch.zeros(4, 2, 1, 16, 96, device=dev())
     work, table = torch.zeros(1, 8, dtype=torch.int32, device=dev()), torch.zeros(1, 4, dtype=torch.int32, device=dev())
     assert not k.attention_rows(q, pages, torch.empty_like(q), work, 1, 64, table, 1, 1, 96, 0, 1.0, k.new_error_word(dev()))
+
+
+# ---------------------------------------------------------------------------
+# the norm in front of a product: inside it or by a kernel of its own
+# ---------------------------------------------------------------------------
+
+@pytest.mark.parametrize("width,groups", [(1024, 1), (1024, 2), (2048, 1), (2560, 1)])
+def test_rows_normed_inside_the_product_or_before_it_have_the_same_bits(width, groups):
+    """Row 3 of 8 tokens (where the norm rides inside) and of 9 and 33 (where it does not)."""
+    from lockstep_b200.parts.norm import NormedRows
+
+    k = K()
+    g = torch.Generator().manual_seed(width)
+    h = (torch.randn(33, width, generator=g) * 2).to(dev())
+    gain = (1 + 0.1 * torch.randn(width, generator=g)).to(torch.bfloat16).to(dev())
+    w = (torch.randn(4096, width, generator=g) * 0.05).to(torch.bfloat16).to(dev())
+    err = k.new_error_word(dev())
+
+    class Norm:
+        def __init__(self):
+            self.gain, self.eps, self.groups = gain, 1e-6, groups
+
+        def forward(self, rows, row_index):
+            out = torch.empty(rows.shape, dtype=torch.bfloat16, device=dev())
+            k.rmsnorm(rows, gain, out, 1e-6, err, row_index, groups)
+            return out
+
+    outs = []
+    for t in (8, 9, 33):
+        rows = NormedRows(Norm(), h[:t].contiguous())
+        out = torch.empty(t, 4096, dtype=torch.bfloat16, device=dev())
+        rows.linear(w, out, k.EPILOGUE_STORE, err)
+        assert rows.pending() == (t == 8 and groups == 1 and width <= 2048)
+        outs.append(out[3].clone())
+    k.raise_on_fault(err)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
