@@ -27,10 +27,6 @@ class SamplingParams:
     position: int = 0        # position of the last context token
 
 
-def _as_int32(words: list[int]) -> list[int]:
-    return [w - (1 << 32) if w >= (1 << 31) else w for w in words]
-
-
 class Sampler:
     def __init__(self, device):
         self.device = torch.device(device)
@@ -52,12 +48,14 @@ class Sampler:
         out = torch.empty(rows, dtype=torch.int32, device=self.device)
         if rows == 0:
             return out
-        if all(p.temperature <= 0 for p in params):
+        temperatures = [p.temperature for p in params]
+        if all(t <= 0 for t in temperatures):
             K.argmax(logits, out)
             return out
-        for p in params:
-            if p.temperature > 0 and not 0 < p.top_p <= 1:
-                raise ValueError(f"{p.uid}: top_p must lie in (0, 1], got {p.top_p}")
+        top_ps = [p.top_p for p in params]
+        for p, t, top in zip(params, temperatures, top_ps):
+            if t > 0 and not 0 < top <= 1:
+                raise ValueError(f"{p.uid}: top_p must lie in (0, 1], got {top}")
         # keys, positions, temperatures and nucleus sizes in one pinned buffer and one copy
         if self._host is None or self._host.numel() < 6 * rows:
             self._host = torch.empty(6 * max(rows, 64), dtype=torch.int32).pin_memory()
@@ -66,14 +64,11 @@ class Sampler:
             self._copied.synchronize()        # the copy before this one has read the buffer
         host = self._host[:6 * rows]
         words = host.numpy()
-        reals = words.view("float32")
-        for i, p in enumerate(params):
-            k0, k1 = _key_words(p.seed, p.uid)
-            words[2 * i], words[2 * i + 1] = _as_int32([k0, k1])
-            words[2 * rows + 2 * i], words[2 * rows + 2 * i + 1] = _as_int32(
-                [p.position & 0xFFFFFFFF, (p.position >> 32) & 0xFFFFFFFF])
-            reals[4 * rows + i] = max(0.0, p.temperature)
-            reals[5 * rows + i] = p.top_p
+        pairs, reals = words[:4 * rows].view("uint64"), words.view("float32")      # low word first
+        pairs[:rows] = [_key(p.seed, p.uid) for p in params]
+        pairs[rows:] = [p.position & 0xFFFFFFFFFFFFFFFF for p in params]
+        reals[4 * rows:5 * rows] = [max(0.0, t) for t in temperatures]
+        reals[5 * rows:] = top_ps
         dev = host.to(self.device, non_blocking=True)
         self._copied.record()
         keys, positions = dev[:2 * rows].view(rows, 2), dev[2 * rows:4 * rows].view(rows, 2)
@@ -86,5 +81,6 @@ class Sampler:
 
 
 @functools.lru_cache(maxsize=4096)
-def _key_words(seed: int, uid: str) -> tuple[int, int]:
-    return philox.key_words(seed, uid)
+def _key(seed: int, uid: str) -> int:
+    low, high = philox.key_words(seed, uid)
+    return low | high << 32
