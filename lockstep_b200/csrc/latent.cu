@@ -61,18 +61,20 @@ template <typename T>
 __global__ void __launch_bounds__(THREADS) latent_finish_kernel(LatentArgs a, int* err) {
   __shared__ float scratch[32];
   extern __shared__ float q_plain[];       // with w_fold: the plain query part [d] of this block's head
-  ls_dependency_sync();
+  ls_dependency_trigger();
   const int t = blockIdx.x;
   const T* row = reinterpret_cast<const T*>(a.proj) + (int64_t)t * a.ld;
   const int pos = a.positions[t];
   const int half = a.dr >> 1;
   if (half > 0 && (pos < 0 || pos >= a.max_positions)) {
     if (threadIdx.x == 0) ls_record_fault(err, LS_DEV_POSITION_RANGE, t);
+    ls_dependency_wait();
     return;
   }
   const float* cs = a.cos_table + (int64_t)pos * half;
   const float* sn = a.sin_table + (int64_t)pos * half;
   const int qd = a.d + a.dr, tail = a.D - a.rank;
+  ls_dependency_wait();                    // (a token's position is one of the step's inputs)
   // queries: the rotated part of every head behind the columns the fold will fill, then zeros
   T* q_dst = reinterpret_cast<T*>(a.q_out) + (int64_t)t * a.H * a.D;
   for (int e = threadIdx.x; e < a.H * tail && blockIdx.y == 0; e += THREADS) {
