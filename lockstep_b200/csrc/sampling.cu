@@ -226,8 +226,8 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs,
 // What bounds it: the exchanges (one for the maximum, one a digit: five digits with a nucleus,
 // since the first digit's histogram serves both selections, else three), about 4 us each at eight
 // blocks.  Bisecting on the bit pattern instead took 16 passes over registers and 17 exchanges a
-// selection.  151,936 tokens with top-p, 1 / 8 / 64 rows: 33 / 35 / 76 us (bisecting: 103 / 106 /
-// 525); 64 rows of 32,768: 29 us (509).
+// selection.  151,936 tokens with top-p, 1 / 8 / 64 rows: 37 / 39 / 89 us (bisecting: 106 / 107 /
+// 526); 64 rows of 32,768: 32 us (510).
 // --------------------------------------------------------------------------
 constexpr int SAMPLE_CLUSTER = 8;                   // most blocks a row is spread over
 constexpr int SAMPLE_MOST = 8 * 1024 * 20;          // largest vocabulary of this kernel
@@ -289,11 +289,25 @@ __device__ unsigned long long sample_scan(SampleShare& sh, unsigned long long ma
   return incl;
 }
 
-// one token's mantissa into its bin
-__device__ __forceinline__ void sample_count(uint2* hist, uint32_t bin, uint32_t bits) {
-  const uint32_t m = (bits & 0x7fffffu) | (bits >= 0x800000u ? 0x800000u : 0u);
-  atomicAdd(&hist[bin].x, m & 0xfffu);
-  atomicAdd(&hist[bin].y, m >> 12);
+// One token's mantissa into its bin, for the lanes with `counts` (called by whole warps).  Where all of a
+// warp's tokens share a bin, as in a flat row, the warp's sums go there at once: 64 atomics on one address
+// would follow one another (a row of 151,936 equal logits 50 us, without this 126; a usual row pays 3 us).
+__device__ __forceinline__ void sample_count(uint2* hist, bool counts, uint32_t bin, uint32_t bits) {
+  const uint32_t lanes = __ballot_sync(0xffffffffu, counts);
+  if (lanes == 0u) return;
+  const uint32_t m = counts ? (bits & 0x7fffffu) | (bits >= 0x800000u ? 0x800000u : 0u) : 0u;
+  const int first = __ffs(lanes) - 1;
+  const uint32_t first_bin = __shfl_sync(0xffffffffu, bin, first);
+  if (__all_sync(0xffffffffu, !counts || bin == first_bin)) {
+    const uint32_t low = __reduce_add_sync(0xffffffffu, m & 0xfffu), high = __reduce_add_sync(0xffffffffu, m >> 12);
+    if ((int)(threadIdx.x & 31) == first) {
+      atomicAdd(&hist[bin].x, low);
+      atomicAdd(&hist[bin].y, high);
+    }
+  } else if (counts) {
+    atomicAdd(&hist[bin].x, m & 0xfffu);
+    atomicAdd(&hist[bin].y, m >> 12);
+  }
 }
 
 // The token that `target` (>= 1, at most the row's mass; units of 2^-46) falls on in the (-e, id)
@@ -321,9 +335,9 @@ __device__ void sample_select(SampleShare& sh, const float* e, int live, int beg
   for (int digit = 1; digit < 3; ++digit) {
     uint2* hist = sh.hist[turn];
     const int down = digit == 1 ? 10 : 0;
-    for (int i = tid; i < live; i += SAMPLE_THREADS) {
-      const uint32_t bits = __float_as_uint(e[i]);
-      if (bits >> (down + 10) == prefix && bits != 0u) sample_count(hist, (bits >> down) & 1023u, bits);
+    for (int i0 = 0; i0 < live; i0 += SAMPLE_THREADS) {
+      const uint32_t bits = i0 + tid < live ? __float_as_uint(e[i0 + tid]) : 0u;
+      sample_count(hist, bits >> (down + 10) == prefix && bits != 0u, (bits >> down) & 1023u, bits);
     }
     cluster_sync_all();
     const int here = turn;
@@ -437,12 +451,16 @@ sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict_
   }
   const float vmax = __fdiv_rn(best.v, temp);
   // e, and the first digit's histogram; what is no number goes to the last bin
-  for (int i = tid; i < live; i += SAMPLE_THREADS) {
-    const float v = expf(__fdiv_rn(sample_e[i], temp) - vmax);
-    sample_e[i] = v;
-    const uint32_t bits = __float_as_uint(v);
-    if (bits > 0x3f800000u) atomicAdd(&sh.hist[0][SAMPLE_BINS - 1].x, 1u);
-    else if (bits != 0u) sample_count(sh.hist[0], bits >> 20, bits);
+  for (int i0 = 0; i0 < live; i0 += SAMPLE_THREADS) {
+    const int i = i0 + tid;
+    uint32_t bits = 0u;
+    if (i < live) {
+      const float v = expf(__fdiv_rn(sample_e[i], temp) - vmax);
+      sample_e[i] = v;
+      bits = __float_as_uint(v);
+      if (bits > 0x3f800000u) atomicAdd(&sh.hist[0][SAMPLE_BINS - 1].x, 1u);
+    }
+    sample_count(sh.hist[0], bits != 0u && bits <= 0x3f800000u, bits >> 20, bits);
   }
   cluster_sync_all();
   int turn = 1;
