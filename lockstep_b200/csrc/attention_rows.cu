@@ -16,6 +16,11 @@
 // over groups of four neighbouring keys and then a tree, splits of LS_SPLIT keys at fixed positions
 // are folded in ascending order.  A row's bits therefore depend on its own position only, and are
 // those of a decoded token's splits and of the 16-token tiles.
+//
+// A key that a row does not see has the weight 0 and changes nothing, unless its value is an infinity
+// or NaN: 0 times that is NaN, and larger tiles would carry it to rows whose 16-token tile never reads
+// the key.  An item with a NaN among its results is therefore done again in groups of 16 tokens, each over
+// the keys of its own 16-token tile (in an item without one this costs a vote of the block).
 #include <math_constants.h>
 
 #include "attention_fold.cuh"
@@ -56,12 +61,12 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ pag
   const int* w = work + (int64_t)blockIdx.x * 8;
   const int req_row = w[0], tok0 = w[1], ntok = w[2], pos0 = w[3];
   if (ntok == 0) return;                     // padding item of a recorded launch
-  const int split_begin = w[4], split_end = w[5], leading = w[7];
+  int split_begin = w[4], split_end = w[5], leading = w[7];
   const int h = (int)blockIdx.y, kvh = h / (nq / nkv);
   const int tid = threadIdx.x, mg = tid >> 3, sub = tid & 7;
   const int* table_row = block_table + (int64_t)req_row * table_stride;
-  const int pos_last = pos0 + ntok - 1;
-  const int key_lo_tile = ls_first_key(pos0, window);
+  int pos_last = pos0 + ntok - 1;
+  int key_lo_tile = ls_first_key(pos0, window);
   const float slope = slopes != nullptr ? slopes[h] : 0.f;
   const float log_rate = log_rates != nullptr ? log_rates[h] : 0.f;
 
@@ -103,12 +108,15 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ pag
     }
   };
 
+  // pass 0: all rows of the item; pass g + 1, after a NaN: the rows of group g (rows 16 g .. 16 g + 15)
+#pragma unroll 1
+  for (int pass = 0;; ++pass) {
   Cursor cur;
   cur.turn = split_begin - leading;
   enter(cur);
   bool more = settle(cur);
   if (more) fetch(cur, 0);
-  for (int i = tid; i < Share::ROWS * (D / 4); i += 128) {
+  for (int i = tid; pass == 0 && i < Share::ROWS * (D / 4); i += 128) {
     const int r = i / (D / 4), c4 = 4 * (i - r * (D / 4));
     copy16_or_zero(&sh.q[r][c4], r < ntok ? q + ((int64_t)(tok0 + r) * nq + h) * D + c4 : nullptr);
   }
@@ -252,10 +260,11 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ pag
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 
+  bool nan = false;
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const int m = mg + 16 * i;
-    if (m >= ntok) continue;
+    if (m >= ntok || (pass > 0 && i != pass - 1)) continue;
     if (sinks != nullptr) {
       // a sink: one more term exp(sinks[head]) in the softmax's denominator, with no value
       float alpha, beta, m_new;
@@ -273,7 +282,18 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ pag
       y.z = l_run[i] > 0.f ? __fdiv_rn(acc_run[i][4 * jj + 2], l_run[i]) : 0.f;
       y.w = l_run[i] > 0.f ? __fdiv_rn(acc_run[i][4 * jj + 3], l_run[i]) : 0.f;
       *reinterpret_cast<float4*>(o + 32 * jj) = y;
+      nan |= !(y.x == y.x && y.y == y.y && y.z == y.z && y.w == y.w);
     }
+  }
+  if (pass == 0 && !__syncthreads_or(nan)) return;
+  if (16 * pass >= ntok) return;
+  // the next group's bounds, as the plan of 16-token tiles has them
+  const int first = pos0 + 16 * pass;
+  pos_last = min(first + 15, pos0 + ntok - 1);
+  key_lo_tile = ls_first_key(first, window);
+  split_begin = key_lo_tile / LS_SPLIT;
+  split_end = pos_last / LS_SPLIT + 1;
+  leading = min((keep_first + LS_SPLIT - 1) / LS_SPLIT, split_begin);
   }
 }
 

@@ -182,6 +182,41 @@ def test_float32_attention_has_the_same_bits_in_tiles_of_every_size(nq, nkv, d, 
     assert torch.equal(outs[16], outs[32]) and torch.equal(outs[16], outs[64])
 
 
+@pytest.mark.parametrize("d,start,n,mask", [(128, 0, 130, 0), (64, 0, 130, 0), (128, 290, 75, 100), (64, 640, 64, (40, 300)),
+                                            (128, 250, 60, -64)])
+def test_a_value_that_is_no_number_reaches_the_rows_it_reaches_in_tiles_of_16_tokens(d, start, n, mask):
+    """An infinity or a NaN among the values is NaN in every row of a 16-token tile that reads it, and in no other row."""
+    from lockstep_b200.engine.batch import mask_parts, plan_attention
+
+    k = K()
+    page, nq, nkv = 16, 2, 1
+    g = torch.Generator().manual_seed(d + n)
+    q = torch.randn(n, nq * d, generator=g).to(dev())
+    count = -(-(start + n) // page)
+    pages = torch.randn(count, 2, nkv, page, d, generator=g)
+    table = torch.arange(count, dtype=torch.int32).view(1, -1).to(dev())
+    for key, value in ((start + 37, math.inf), (start + n - 2, math.nan), (start - 90, -math.inf), (start - 3, math.inf)):
+        if key >= 0:
+            pages[key // page, 1, 0, key % page, 5:9] = value
+    pages = pages.to(dev())
+    window, keep = mask_parts(mask)
+    err, outs = k.new_error_word(dev()), {}
+    for size in (16, 32, 64):
+        tile = plan_attention([(0, 0, start, n)], mask, k.attention_split_size(), size)[0]
+        work, out = torch.from_numpy(tile).to(dev()), torch.empty_like(q)
+        if size == 16:
+            k.attention_tile(q, pages, out, None, None, work, len(tile), table, nq, nkv, d, window, d ** -0.5, err, keep_first=keep)
+        else:
+            assert k.attention_rows(q, pages, out, work, len(tile), size, table, nq, nkv, d, window, d ** -0.5, err, keep_first=keep)
+        outs[size] = out
+    k.raise_on_fault(err)
+    bad = outs[16].isnan()
+    assert bool(bad.any())
+    for size in (32, 64):
+        assert torch.equal(outs[size].isnan(), bad), size
+        assert torch.equal(outs[size][~bad], outs[16][~bad]), size
+
+
 def test_float32_attention_declines_what_it_does_not_cover():
     k = K()
     assert k.attention_rows_tile_tokens(4096, 16, 128, torch.bfloat16) == 16
