@@ -465,10 +465,14 @@ template <int EPI, int TM, int WR>
 int launch_large_as(const float* A, const float* W, float* C, int M, int N, int K, int64_t lda, int64_t ldw,
                     int64_t ldc, cudaStream_t stream) {
   constexpr int FN = EPI == 2 ? WR / 2 : WR;
-  dim3 grid((N + FN - 1) / FN, (M + TM - 1) / TM);
-  if (grid.y > 65535) return LS_E_SIZE;
-  LS_COUNT(LS_K_GEMM_SIMT_MANY);
-  ls_launch(gemm_nt_large_kernel<EPI, TM, WR>, grid, 2 * TM, 0, stream, A, W, C, M, N, K, lda, ldw, ldc);
+  // (a grid has 65,535 rows of blocks at most: 4,194,240 tokens in tiles of 64; the tokens after them are a launch of their own)
+  constexpr int MOST = 65535 * TM;
+  for (; M > 0; M -= MOST, A += (int64_t)MOST * lda, C += (int64_t)MOST * ldc) {
+    const int rows = M < MOST ? M : MOST;
+    LS_COUNT(LS_K_GEMM_SIMT_MANY);
+    ls_launch(gemm_nt_large_kernel<EPI, TM, WR>, dim3((N + FN - 1) / FN, (rows + TM - 1) / TM), 2 * TM, 0, stream, A, W, C, rows, N,
+              K, lda, ldw, ldc);
+  }
   return ls_launch_status();
 }
 
@@ -480,7 +484,8 @@ int launch_large(const float* A, const float* W, float* C, int M, int N, int K, 
   // a k-block bounds a block, and more and smaller tiles are faster, 64 x 64 (600 tokens of 4,096 features 167 us,
   // 64 x 128: 195), except where 128 x 64 is just one round of two blocks an SM (1,800 tokens of 1,024
   // features and K = 2,048: 234 us, 64 x 64: 246).
-  const long long sms = large_sm_count(), rows64 = (M + 63) / 64, rows128 = (M + 127) / 128;
+  const long long sms = large_sm_count(), rows64 = (M + 63LL) / 64, rows128 = (M + 127LL) / 128;
+  if (rows128 > 65535) return LS_E_SIZE;
   if constexpr (EPI != 2) {
     const long long tall = rows128 * ((N + 63) / 64);
     if (rows64 * ((N + 127) / 128) < 3 * sms) {

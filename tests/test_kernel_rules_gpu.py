@@ -132,6 +132,22 @@ def test_a_float32_row_has_the_same_bits_in_every_batch(n, k_, epilogue):
     assert (rows[700].double() - want).abs().max() <= 2.0 ** -21 * math.sqrt(k_) * (1 + float(want.abs().max()))
 
 
+@pytest.mark.parametrize("epilogue", ["store", "silu"])
+def test_a_float32_product_takes_more_rows_than_a_grid_has_tiles(epilogue):
+    """More than 65,535 tiles of 64 tokens: the bits of its two halves."""
+    k = K()
+    g = torch.Generator(device=dev()).manual_seed(7)
+    m, n, k_ = 65535 * 64 + 70, 5, 4
+    x = torch.randn(m, k_, generator=g, device=dev())
+    w = torch.randn(2 * n if epilogue == "silu" else n, k_, generator=g, device=dev())
+    code = k.EPILOGUE_SILU_MUL if epilogue == "silu" else k.EPILOGUE_STORE
+    whole, halves = torch.full((m, n), math.nan, device=dev()), torch.full((m, n), math.nan, device=dev())
+    k.gemm_nt_simt(x, w, whole, code)
+    for part in (slice(0, m // 2), slice(m // 2, m)):
+        k.gemm_nt_simt(x[part], w, halves[part], code)
+    assert bool(torch.isfinite(whole).all()) and torch.equal(whole, halves)
+
+
 # ---------------------------------------------------------------------------
 # float32 attention of prompt portions: tiles of 16, 32 and 64 tokens
 # ---------------------------------------------------------------------------
