@@ -317,14 +317,38 @@ int launch_rows(const float* q, const float* pages, float* out, const int* work,
 
 }  // namespace
 
-// Tokens a work item should hold for a step of `tokens` tokens: 64 where that fills most of the device's two blocks
-// an SM (16 heads: 1,024 tokens after 777 others 549 us, with 32 705; 404 rows of 8 heads 39 us, with 32 25), 32 down to
-// a quarter of the SMs (90 tokens of 16 heads 17.5 us, with 16 25.6), else 16, which ls_attention_tile takes (as it does every other head
-// size): its threads are then more, and fewer of a block's rows are empty.
-LS_API int ls_attention_rows_tile_tokens(int tokens, int nq, int d) {
+// What the portions of a step (`tokens` in all, n16 / n32 / n64 tiles of 16 / 32 / 64 tokens) take in tiles of each
+// size where there are many, in the same unit: a thread of the larger tiles holds all its rows whether they are
+// filled or not, a row of the 16-token tile that is empty is half as dear as one that is not.  64 portions of 16 heads
+// of 128 after 500 others, tiles of 16 / 32 / 64: of 2 tokens 219 / 442 / 518 us, of 8 279 / 442 / 517, of 14 414 / 483 / 584, of
+// 17 674 / 490 / 571, of 40 1,109 / 867 / 593, of 65 1,759 / 1,370 / 1,210.
+struct RowsCost {
+  long long c16, c32, c64;
+  RowsCost(int tokens, int n16, int n32, int n64) : c16(80LL * n16 + 5LL * tokens), c32(192LL * n32), c64(256LL * n64) {}
+};
+
+// The tile size that a step's portions are best cut into where there are many, whatever the heads.
+LS_API int ls_attention_rows_tile_class(int tokens, int n16, int n32, int n64) {
+  const RowsCost cost(tokens, n16, n32, n64);
+  return cost.c64 < cost.c32 && cost.c64 < cost.c16 ? 64 : cost.c32 < cost.c16 ? 32 : 16;
+}
+
+// Tokens a work item should hold for portions of `tokens` tokens that make n16, n32 and n64 tiles: 16, which
+// ls_attention_tile takes (as it does every other head size), 32 or 64.  More tiles than the two blocks an SM that run at
+// one time: the cheapest, but 64 only where there are rows for most of the device's blocks (16 heads: 1,024 tokens
+// after 777 others 549 us, with 32 705; 404 rows of 8 heads 39 us, with 32 25).  Fewer: a block's time counts and not their number, and
+// 32 is faster down to a quarter of the SMs' rows (90 tokens of 16 heads 17.5 us, with 16 25.6; 16 portions of 8 tokens
+// 10.1 and 13.2), or where tiles a quarter filled are on half of the SMs at most (4 portions of 8 tokens 7.6 and 10.3); fewer tokens take 16.
+LS_API int ls_attention_rows_tile_tokens(int tokens, int n16, int n32, int n64, int nq, int d) {
   if ((d != 64 && d != 128) || tokens <= 0 || nq <= 0) return 16;
-  const long long rows = (long long)tokens * nq;
-  return rows >= 64LL * 222 ? 64 : rows >= 32LL * 37 ? 32 : 16;
+  const long long rows = (long long)tokens * nq, sms = ls_sm_count(), blocks = (long long)n32 * nq;
+  if (blocks > 2 * sms) {
+    const int best = ls_attention_rows_tile_class(tokens, n16, n32, n64);
+    if (best != 64 || 2 * rows >= 64 * 3 * sms) return best;
+    const RowsCost cost(tokens, n16, n32, n64);
+    return cost.c32 < cost.c16 ? 32 : 16;
+  }
+  return 4 * rows >= 32 * sms || (2 * blocks <= sms && tokens >= 8LL * n32) ? 32 : 16;
 }
 
 // Work items as ls_attention_tile takes them in serial form, of up to `tile_tokens` (32 or 64) tokens.

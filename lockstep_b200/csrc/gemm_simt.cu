@@ -451,16 +451,6 @@ gemm_nt_large_kernel(const float* __restrict__ A, const float* __restrict__ W, f
   }
 }
 
-int large_sm_count() {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-  }
-  return sms;
-}
-
 template <int EPI, int TM, int WR>
 int launch_large_as(const float* A, const float* W, float* C, int M, int N, int K, int64_t lda, int64_t ldw,
                     int64_t ldc, cudaStream_t stream) {
@@ -484,7 +474,7 @@ int launch_large(const float* A, const float* W, float* C, int M, int N, int K, 
   // a k-block bounds a block, and more and smaller tiles are faster, 64 x 64 (600 tokens of 4,096 features 167 us,
   // 64 x 128: 195), except where 128 x 64 is just one round of two blocks an SM (1,800 tokens of 1,024
   // features and K = 2,048: 234 us, 64 x 64: 246).
-  const long long sms = large_sm_count(), rows64 = (M + 63LL) / 64, rows128 = (M + 127LL) / 128;
+  const long long sms = ls_sm_count(), rows64 = (M + 63LL) / 64, rows128 = (M + 127LL) / 128;
   if (rows128 > 65535) return LS_E_SIZE;
   if constexpr (EPI != 2) {
     const long long tall = rows128 * ((N + 63) / 64);

@@ -15,6 +15,8 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
+from ..kernels import portion_tiles
+
 TILE_TOKENS = 16   # query tokens of one block of the tile kernel (csrc/attention_simt.cu)
 
 
@@ -110,6 +112,7 @@ class StepContext:
             self.portions.append((slot, off, e.start, n))
             off += n
         self.num_tokens = off
+        self.portion_tiles = portion_tiles(n for _, _, _, n in self.portions)
         self.n_wanted = len(wanted)
         packed = np.asarray(ids + pos + tslot + wanted, dtype=np.int64)
         if packed.size and (packed.min() < -(2 ** 31) or packed.max() >= 2 ** 31):

@@ -19,7 +19,8 @@ capacity with null items, which the kernels skip.  Nothing about the
 arithmetic changes: the same kernels run on the same values.
 
 Steps that mix portions of prompts (a step that fills the token budget, say) are recorded too,
-keyed by their exact number of tokens and the rounded numbers of wanted rows, split items and portions,
+keyed by their exact number of tokens and the rounded numbers of wanted rows, split items and portions (and, in float32,
+the tile size that suits the portions' lengths),
 when a step of the same shape comes for the third time: such steps launch some 300 kernels, and the
 host is slower at enqueueing them than the device at running them.
 
@@ -36,6 +37,7 @@ from collections import OrderedDict
 import numpy as np
 import torch
 
+from ..kernels import attention_rows_tile_class, portion_tiles
 from .batch import AttentionPlan, first_key, kept_splits, mask_parts, plan_attention
 
 CAPACITY_STEP = 32      # the attention work list of a recorded step holds a multiple of this many items
@@ -57,6 +59,7 @@ class StaticStepContext:
         self.pad_slot = pad_slot
         self.device, self.err, self.split_size = device, err, split_size
         self.num_tokens = self.n_wanted = batch
+        self.portion_tiles = (0, 0, 0, 0)
         per_window = capacity * 8 + batch * 4
         self.size = 4 * batch + len(self.windows) * per_window
         self.host = torch.zeros(self.size, dtype=torch.int32).pin_memory()
@@ -161,8 +164,9 @@ class StaticMixedContext:
     logits are dropped, and with null items, which the kernels skip)."""
 
     def __init__(self, tokens: int, wanted_cap: int, split_cap: int, portions: int, max_entries: int,
-                 plan_keys: list[tuple], device, err, split_size: int):
+                 plan_keys: list[tuple], portion_tiles: tuple, device, err, split_size: int):
         self.num_tokens, self.n_wanted = tokens, wanted_cap
+        self.portion_tiles = portion_tiles          # of the step that is recorded: they choose its kernels
         self.split_cap, self.max_entries = split_cap, max_entries
         self.plan_keys = sorted(plan_keys, key=lambda key: (mask_parts(key[0]), key[1]))
         self.device, self.err, self.split_size = device, err, split_size
@@ -342,8 +346,8 @@ class DecodeGraphs:
 
     # -- steps that mix portions of prompts and decoded tokens --------------
     def mixed_key_for(self, entries) -> tuple | None:
-        """(tokens, wanted rows, split items, portions) of the recorded step that would serve ``entries``, the last three
-        rounded up; None for steps without portions, with more portions than tile work lists are made for, or with more
+        """(tokens, wanted rows, split items, portions, tile class) of the recorded step that would serve ``entries``, the
+        middle three rounded up, the last what the portions' lengths say about the float32 attention's kernel; None for steps without portions, with more portions than tile work lists are made for, or with more
         wanted rows than requests can be live."""
         tokens = sum(len(e.tokens) for e in entries)
         max_live = self.runner.cache.max_live
@@ -368,7 +372,8 @@ class DecodeGraphs:
             while split_cap < splits:
                 split_cap *= 2
         wanted_cap = SHORT_WANTED if tokens < MIXED_SHORT and wanted <= SHORT_WANTED else -(-max(wanted, 1) // 64) * 64
-        return tokens, min(max_live, wanted_cap), split_cap, portions
+        tile = attention_rows_tile_class(portion_tiles(len(e.tokens) for e in entries), self.runner.dtype)
+        return tokens, min(max_live, wanted_cap), split_cap, portions, tile
 
     def mixed_ready(self, key) -> bool:
         return key in self.mixed
@@ -383,11 +388,12 @@ class DecodeGraphs:
             self.mixed_seen.popitem(last=False)
         return n >= MIXED_SIGHTINGS
 
-    def record_mixed(self, key, plan_keys) -> None:
-        tokens, wanted_cap, split_cap, portions = key
+    def record_mixed(self, key, plan_keys, tiles: tuple) -> None:
+        """``plan_keys``, ``tiles``: the attention plans that the step of this shape before asked for, and its ``portion_tiles``."""
+        tokens, wanted_cap, split_cap, portions, _ = key
         r = self.runner
-        ctx = StaticMixedContext(tokens, wanted_cap, split_cap, portions, r.cache.max_live, list(plan_keys), r.device,
-                                 r.err, r.split_size)
+        ctx = StaticMixedContext(tokens, wanted_cap, split_cap, portions, r.cache.max_live, list(plan_keys), tiles,
+                                 r.device, r.err, r.split_size)
         self.mixed[key] = self._record(ctx)
         short = tokens < MIXED_SHORT
         self.mixed_recordings[short] += 1

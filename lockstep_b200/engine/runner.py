@@ -237,7 +237,7 @@ class ModelRunner:
                 logits = self.forward(ctx)
                 # a step of this shape has come often enough: later ones replay a recorded one
                 if mixed is not None and self.graphs.mixed_seen_again(mixed):
-                    self.graphs.record_mixed(mixed, ctx._plans.keys())
+                    self.graphs.record_mixed(mixed, ctx._plans.keys(), ctx.portion_tiles)
         for e in entries:
             self.cache.advance(e.uid, e.start + len(e.tokens))
         self.steps_run += 1

@@ -78,7 +78,8 @@ _SIGNATURES = {
         "ls_attention_tile": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                               c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                               c_float, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
-        "ls_attention_rows_tile_tokens": [c_int, c_int, c_int],
+        "ls_attention_rows_tile_tokens": [c_int, c_int, c_int, c_int, c_int, c_int],
+        "ls_attention_rows_tile_class": [c_int, c_int, c_int, c_int],
         "ls_attention_rows": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int,
                               c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
         "ls_attention_decode": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int,
@@ -601,12 +602,25 @@ def attention_tile(q, pages, out, part_acc, part_ml, work, n_work, block_table, 
         _stream()), "attention_tile")
 
 
-def attention_rows_tile_tokens(tokens: int, nq: int, d: int, dtype) -> int:
-    """Tokens of a work item for the float32 attention of a step of ``tokens`` tokens: 64 or 32 where ``attention_rows``
-    serves it best, 16 for ``attention_tile`` (other types, other head sizes, few rows)."""
+def portion_tiles(lengths) -> tuple[int, int, int, int]:
+    """(tokens, tiles of 16, of 32, of 64 tokens) that portions of these lengths make (single tokens make none)."""
+    lengths = [int(n) for n in lengths if n > 1]
+    return (sum(lengths), *(sum(-(-n // size) for n in lengths) for size in (16, 32, 64)))
+
+
+def attention_rows_tile_tokens(portions, nq: int, d: int, dtype) -> int:
+    """Tokens of a work item for the float32 attention of a step's ``portions`` (``portion_tiles``, or the length of a single
+    one): 64 or 32 where ``attention_rows`` serves them best, 16 for ``attention_tile`` (other types, other head
+    sizes, few rows, many portions of few tokens)."""
     if dtype != torch.float32:
         return 16
-    return int(library().ls_attention_rows_tile_tokens(int(tokens), int(nq), int(d)))
+    tiles = portions if isinstance(portions, tuple) else portion_tiles([portions])
+    return int(library().ls_attention_rows_tile_tokens(*tiles, int(nq), int(d)))
+
+
+def attention_rows_tile_class(portions: tuple, dtype) -> int:
+    """The tile size that many such portions (``portion_tiles``) are best cut into, whatever the heads."""
+    return int(library().ls_attention_rows_tile_class(*portions)) if dtype == torch.float32 else 16
 
 
 def attention_rows(q, pages, out, work, n_work, tile_tokens, block_table, nq, nkv, d, window, scale, err, slopes=None,

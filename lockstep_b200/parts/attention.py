@@ -119,8 +119,8 @@ def attend(rt: Runtime, q, ctx, cache, nq: int, nkv: int, d: int, mask, scale: f
             window, scale, rt.err, extras.slopes, extras.log_rates, extras.sinks, softcap=extras.softcap,
             keep_first=keep)
     if exact:
-        # float32: tiles of more tokens where the step has enough rows to fill the device with them
-        tile_tokens = K.attention_rows_tile_tokens(t, nq, d, q.dtype)
+        # float32: tiles of more tokens where the step's portions fill them, and the device
+        tile_tokens = K.attention_rows_tile_tokens(ctx.portion_tiles, nq, d, q.dtype)
         if tile_tokens > 16:
             plan = ctx.attention_plan(mask, tile_tokens)
             done = not plan.n_tile or K.attention_rows(

@@ -67,3 +67,45 @@ def test_a_token_is_planned_alike_in_any_batch():
     mine = [r for r in among[1].tolist() if r[0] == 3]
     # the same splits of the same position; only the token's offset and its scratch slots move
     assert [(r[3], r[4], r[5]) for r in mine] == [(r[3], r[4], r[5]) for r in alone[1].tolist()]
+
+
+def test_float32_attention_takes_large_tiles_only_where_the_portions_fill_them():
+    """Tiles of 32 and 64 tokens do the work of all their rows: many portions of few tokens stay in tiles of 16, and
+    single tokens, which are in no tile, do not count."""
+    import torch
+
+    from lockstep_b200 import kernels as K
+
+    def pick(lengths, nq=16, d=128, dtype=torch.float32):
+        return K.attention_rows_tile_tokens(K.portion_tiles(lengths), nq, d, dtype)
+
+    assert K.portion_tiles([1, 16, 17, 1, 64, 65]) == (162, 12, 7, 5)
+    assert [pick([n] * 64) for n in (2, 8, 14, 16, 17, 32, 33, 40, 64)] == [16, 16, 16, 16, 32, 32, 64, 64, 64]
+    assert [pick([n] * 64, 8, 64) for n in (2, 8, 14, 17, 40)] == [16, 16, 16, 32, 64]
+    assert pick([1] * 900 + [20]) != 64 and pick([1] * 900) == 16
+    # one portion: the count of its tokens decides, as for ``attention_rows_tile_tokens`` of a number
+    for n in (2, 7, 73, 74, 300, 600, 887, 888, 900, 4096):
+        assert pick([n]) == K.attention_rows_tile_tokens(n, 16, 128, torch.float32)
+    assert [pick([n]) for n in (2, 7, 74, 300, 600, 887, 888, 4096)] == [16, 16, 32, 32, 32, 32, 64, 64]
+    assert pick([4096], dtype=torch.bfloat16) == pick([4096], d=96) == 16
+
+
+def test_steps_whose_portions_want_other_tiles_are_recorded_apart():
+    """Equal numbers of tokens, wanted rows and portions: five portions that fill tiles of 64, or thirteen that do not."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from lockstep_b200.engine.batch import StepEntry
+    from lockstep_b200.engine.graphs import DecodeGraphs
+
+    def keys(dtype):
+        graphs = DecodeGraphs(SimpleNamespace(model=SimpleNamespace(blocks=[]), dtype=dtype, split_size=256,
+                                              cache=SimpleNamespace(max_live=64)))
+        return [graphs.mixed_key_for([StepEntry(str(i), [0] * n, 0, [n - 1]) for i, n in enumerate(lengths)])
+                for lengths in ([52] * 5, [20] * 13)]
+
+    even, uneven = keys(torch.float32)
+    assert even[:4] == uneven[:4] and even != uneven
+    even, uneven = keys(torch.bfloat16)
+    assert even == uneven
