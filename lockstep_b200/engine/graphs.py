@@ -265,11 +265,12 @@ class DecodeGraphs:
         self.pool = None
         self.replays = 0
         self.dropped = 0
-        # steps that mix portions: recorded when a step of the same shape comes a second time
+        # steps that mix portions: recorded when a step of the same shape comes a third time; what counts
+        # how often a shape came and how many were recorded goes by whether the step is a short one
         self.mixed: OrderedDict[tuple, tuple] = OrderedDict()
-        self.mixed_seen: OrderedDict[tuple, int] = OrderedDict()
+        self.mixed_seen: dict[bool, OrderedDict[tuple, int]] = {False: OrderedDict(), True: OrderedDict()}
         self.mixed_replays = 0
-        self.mixed_recordings = {False: 0, True: 0}          # by whether the step is a short one
+        self.mixed_recordings = {False: 0, True: 0}
 
     def capacity_for(self, entries) -> int:
         n = split_items(entries, self.windows, self.runner.split_size)
@@ -380,12 +381,14 @@ class DecodeGraphs:
 
     def mixed_seen_again(self, key) -> bool:
         """Counts a step of this shape that ran unrecorded; True from the MIXED_SIGHTINGS-th on."""
-        if self.mixed_recordings[key[0] < MIXED_SHORT] >= MIXED_RECORDINGS:
+        short = key[0] < MIXED_SHORT
+        if self.mixed_recordings[short] >= MIXED_RECORDINGS:
             return False
-        n = self.mixed_seen.pop(key, 0) + 1
-        self.mixed_seen[key] = n
-        while len(self.mixed_seen) > 64:
-            self.mixed_seen.popitem(last=False)
+        seen = self.mixed_seen[short]
+        n = seen.pop(key, 0) + 1
+        seen[key] = n
+        while len(seen) > 64:
+            seen.popitem(last=False)
         return n >= MIXED_SIGHTINGS
 
     def record_mixed(self, key, plan_keys, tiles: tuple) -> None:
@@ -401,7 +404,7 @@ class DecodeGraphs:
         kept = [k for k in self.mixed if (k[0] < MIXED_SHORT) == short]
         for dropped in kept[:max(0, len(kept) - (SHORT_GRAPHS if short else MIXED_GRAPHS))]:
             del self.mixed[dropped]
-            self.mixed_seen.pop(dropped, None)        # it has to come three times again
+            self.mixed_seen[short].pop(dropped, None)        # it has to come three times again
             self.dropped += 1
 
     def replay_mixed(self, key, entries, slots) -> torch.Tensor:
