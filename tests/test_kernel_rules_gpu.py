@@ -61,6 +61,68 @@ def test_a_sampled_token_does_not_depend_on_how_many_rows_there_are(vocab):
         assert want == first[i] or abs(float(base[i, want]) - float(base[i, first[i]])) < 1e-3
 
 
+@pytest.mark.parametrize("rows", [6, 37, 80, 149])
+@pytest.mark.parametrize("vocab", [777, 49153, 163840])
+def test_a_draw_falls_on_the_token_whose_share_of_the_mass_it_names(vocab, rows):
+    """Against the cumulative mass in float64, in the (-p, id) order: the drawn token's share holds the draw to 4e-6 of the
+    mass (an exponential's argument below 40 is rounded to 2^-24 of it, so the exponential is right to 2.5e-6, and so is every sum
+    of them) and, where there is a nucleus, the share of its last token, which that error may take in or leave out.  Six kinds of
+    rows, spread over 8 to 1 blocks."""
+    from lockstep_b200.sampling import philox
+
+    k = K()
+    g = torch.Generator().manual_seed(vocab)
+    base = torch.randn(6, vocab, generator=g) * 2.5
+    base[1] = torch.randint(0, 4, (vocab,), generator=g).float()             # four values
+    base[2] = torch.randint(0, 2, (vocab,), generator=g).float() * 1e-3      # two that are close
+    base[3, ::2] = -math.inf
+    base[4, vocab // 2] = 9.0
+    temperature = torch.tensor([0.8, 1.0, 0.7, 1.1, 1.3, 0.9])
+    top_p = torch.tensor([0.9, 0.5, 0.95, 1.0, 1.0, 0.05])
+    pick = [i % 6 for i in range(rows)]
+    uids, positions = [f"m{i}" for i in range(rows)], [5 + 3 * i for i in range(rows)]
+    got = _draw(k, base[pick], temperature[pick], top_p[pick], uids, positions, seed=23)
+    tables = []
+    for i in range(6):
+        z = (base[i] / temperature[i]).double()
+        e = (z - z.max()).exp()
+        order = torch.sort(e, descending=True, stable=True).indices
+        through = torch.cumsum(e[order], 0) / e.sum()
+        place = torch.empty_like(order)
+        place[order] = torch.arange(vocab)
+        head, slack = 1.0, 4e-6
+        if top_p[i] < 1:
+            last = min(int(torch.searchsorted(through, top_p[i].double())), vocab - 1)
+            head, slack = float(through[last]), 4e-6 + float(e[order[last]] / e.sum())
+        tables.append((through, place, head, slack))
+    for row, token in enumerate(got):
+        through, place, head, slack = tables[pick[row]]
+        at, draw = int(place[token]), philox.uniform(23, uids[row], positions[row]) * head
+        assert (float(through[at - 1]) if at else 0.0) - slack <= draw <= float(through[at]) + slack, (row, token)
+
+
+@pytest.mark.parametrize("rows", [1, 37, 80, 149])
+@pytest.mark.parametrize("vocab", [5, 777, 49153, 163840])
+def test_among_equal_logits_the_draw_names_the_token(vocab, rows):
+    """Every token has the same mass, so the sums are exact: the head is the first ceil(top_p V) ids, the token the one on which
+    u times its size falls."""
+    from fractions import Fraction
+
+    import numpy as np
+
+    from lockstep_b200.sampling import philox
+
+    k = K()
+    share = [Fraction(float(np.float32(p))) for p in (1.0, 0.9, 0.3)]
+    pick = [i % 3 for i in range(rows)]
+    uids, positions = [f"e{i}" for i in range(rows)], [7 * i for i in range(rows)]
+    got = _draw(k, torch.full((rows, vocab), 1.5), torch.full((rows,), 0.7), torch.tensor([float(share[i]) for i in pick]), uids,
+                positions, seed=3)
+    for row, token in enumerate(got):
+        u = Fraction(float(np.float32(philox.uniform(3, uids[row], positions[row]))))
+        assert token == max(math.ceil(u * math.ceil(share[pick[row]] * vocab)), 1) - 1, row
+
+
 def test_rows_that_are_no_distribution_give_token_0_or_the_numbers_in_them():
     k = K()
     vocab = 1000
@@ -130,6 +192,32 @@ def test_a_float32_row_has_the_same_bits_in_every_batch(n, k_, epilogue):
             "silu": lambda: torch.nn.functional.silu(z[:, :n]) * z[:, n:]}[epilogue]()
     # one chain of k_ float32 products of size 1 / sqrt(k_): an error of a few 2^-24 sqrt(k_) against |z| of about 1
     assert (rows[700].double() - want).abs().max() <= 2.0 ** -21 * math.sqrt(k_) * (1 + float(want.abs().max()))
+
+
+@pytest.mark.parametrize("epilogue", ["store", "residual", "gelu", "relu2"])
+@pytest.mark.parametrize("n", [1024, 1000])
+def test_a_float32_row_has_the_same_bits_in_tiles_of_128_tokens(n, epilogue):
+    """At 148 SMs 1,665 to 2,304 tokens of some 1,024 features take tiles of 128 x 64, one token fewer or more tiles of 64 x 64:
+    the bits of the few-token kernel, and the values in float64."""
+    k = K()
+    g = torch.Generator().manual_seed(n)
+    k_ = 260
+    code = {"store": k.EPILOGUE_STORE, "residual": k.EPILOGUE_RESIDUAL, "gelu": k.EPILOGUE_GELU, "relu2": k.EPILOGUE_RELU2}[epilogue]
+    x = torch.randn(2305, k_, generator=g).to(dev())
+    w = (torch.randn(n, k_, generator=g) / math.sqrt(k_)).to(dev())
+    base = torch.randn(2305, n, generator=g).to(dev())
+    few = base.clone()
+    for at in range(0, 2305, 32):
+        k.gemm_nt_simt(x[at:at + 32], w, few[at:at + 32], code)
+    for m in (1664, 1665, 1700, 1800, 2304, 2305):
+        c = base[:m].clone()
+        k.gemm_nt_simt(x[:m], w, c, code)
+        assert torch.equal(c, few[:m]), m
+    z = x.double() @ w.double().T
+    want = {"store": lambda: z, "residual": lambda: base.double() + z, "relu2": lambda: z.clamp(min=0) ** 2,
+            "gelu": lambda: torch.nn.functional.gelu(z, approximate="tanh")}[epilogue]()
+    # the bound of the test above
+    assert (few.double() - want).abs().max() <= 2.0 ** -21 * math.sqrt(k_) * (1 + float(want.abs().max()))
 
 
 @pytest.mark.parametrize("epilogue", ["store", "silu"])

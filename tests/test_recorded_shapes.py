@@ -42,3 +42,40 @@ def test_counts_of_long_steps_survive_many_short_ones(graphs):
     for n in range(300, 300 + 70):
         assert not see(graphs, key_of(graphs, [n]))
     assert not see(graphs, short) and see(graphs, short)
+
+
+def test_what_makes_the_shape_of_a_step(graphs):
+    assert key_of(graphs, [1, 1]) is None                              # decoded tokens alone
+    assert key_of(graphs, [3] * 17) is None and key_of(graphs, [20] * 17) is None        # more portions than work lists hold
+    assert key_of(graphs, [9] * 8, want=9) is None                     # more wanted rows than live requests
+    assert [key_of(graphs, [2] * n)[3] for n in (1, 4, 5, 16)] == [4, 4, 16, 16]
+    assert [key_of(graphs, [40], want=n)[1] for n in (0, 1, 8, 9)] == [8, 8, 8, 64]
+    assert [key_of(graphs, [n], want=1)[1] for n in (255, 256)] == [8, 64]
+    assert [key_of(graphs, [5, *[1] * n])[2] for n in (0, 1, 31)] == [0, 64, 64]
+    assert key_of(graphs, [5, *[1] * 31], start=1000)[2] == 128       # four splits of 256 keys each
+    assert key_of(graphs, [17]) != key_of(graphs, [18])
+
+
+def test_the_recordings_of_a_class_do_not_push_out_the_other_class(graphs):
+    long, short = ([key_of(graphs, [n]) for n in range(first, first + count)] for first, count in ((300, 5), (20, 30)))
+    for key in long:
+        graphs.record_mixed(key, [], (0, 0, 0, 0))
+    for i, key in enumerate(short):
+        graphs.record_mixed(key, [], (0, 0, 0, 0))
+        if i == 20:
+            graphs.mixed.move_to_end(short[10])       # replayed: kept longer
+    kept = short[-15:] + [short[10]]
+    assert len(kept) == G.SHORT_GRAPHS and set(graphs.mixed) == {*long, *kept} and graphs.dropped == 30 - G.SHORT_GRAPHS
+    assert not graphs.mixed_ready(short[0]) and not see(graphs, short[0])          # it has to come three times again
+    for n in range(400, 400 + G.MIXED_GRAPHS):
+        graphs.record_mixed(key_of(graphs, [n]), [], (0, 0, 0, 0))
+    assert not any(graphs.mixed_ready(key) for key in long) and all(graphs.mixed_ready(key) for key in kept)
+
+
+def test_a_class_stops_recording_and_the_other_goes_on(graphs):
+    recorded = 0
+    for n in range(2, 2 + G.MIXED_RECORDINGS + 3):
+        recorded += [see(graphs, key_of(graphs, [n])) for _ in range(3)][-1]
+    assert recorded == G.MIXED_RECORDINGS
+    assert not any(see(graphs, key_of(graphs, [200])) for _ in range(5))
+    assert [see(graphs, key_of(graphs, [2048])) for _ in range(3)] == [False, False, True]

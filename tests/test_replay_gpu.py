@@ -278,3 +278,45 @@ def test_steps_of_mixed_portions_are_recorded_when_their_shape_repeats(zoo, name
     assert rows[True].keys() == rows[False].keys()
     for key in rows[True]:
         assert torch.equal(rows[True][key], rows[False][key]), key
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("name", ["B", "D"])
+def test_short_steps_and_steps_of_many_portions_are_recorded_with_the_same_bits(zoo, name, dtype):
+    """Steps of fewer than 256 tokens (0, 1, 8 and 9 wanted rows) and of 4, 5 and 16 portions beside decoded tokens, each shape
+    five times: the fourth and the fifth replay a recording, bit for bit the rows of a runner that records nothing.  Seventeen
+    portions are more than a recording holds."""
+    from lockstep_b200.engine import ModelRunner
+
+    folder, _, _ = zoo(name, dtype)
+    config, page = H.CONFIGS[name]
+    # (tokens of the portions, wanted rows of each, decoded tokens beside them): a shape each
+    shapes = [([2], 1, 0), ([17], 0, 0), ([18], 8, 0), ([255], 9, 0), ([40], 1, 2), ([5] * 4, 1, 2), ([5] * 5, 1, 2),
+              ([3] * 16, 1, 2), ([2, 60, 17, 33, 9, 16], 1, 1), ([20] * 16, 1, 2), ([5] * 17, 1, 2)]
+    decoded = {u: H.random_tokens(30 + 5 * len(shapes), config["vocab_size"], seed=50 + i) for i, u in enumerate("yz")}
+    at = {u: 20 for u in decoded}
+    steps = [{"entries": [(u, decoded[u][:20], [19])], "end": []} for u in "yz"]
+    for _ in range(5):
+        for i, (lengths, want, singles) in enumerate(shapes):
+            entries, end = [], []
+            for j, n in enumerate(lengths):
+                uid = f"{len(steps)}.{j}"
+                entries.append((uid, H.random_tokens(n, config["vocab_size"], seed=97 * len(steps) + j), list(range(n - want, n))))
+                end.append(uid)
+            for u in "yz"[:singles]:
+                entries.insert(1, (u, decoded[u][at[u]:at[u] + 1], [0]))
+                at[u] += 1
+            steps.append({"entries": entries, "end": end})
+    steps[-1]["end"] += ["y", "z"]
+    rows = {}
+    for graphs in (True, False):
+        runner = ModelRunner(folder, dtype=dtype, num_pages=2048 // page, page_size=page, max_live=20, max_seq_len=512,
+                             use_graphs=graphs)
+        rows[graphs] = H.run_plan(runner, steps)
+        if graphs:
+            assert len(runner.graphs.mixed) == len(shapes) - 1
+            assert runner.graphs.mixed_replays == 2 * (len(shapes) - 1)
+        runner.cache.audit()
+    assert rows[True].keys() == rows[False].keys()
+    for key in rows[True]:
+        assert torch.equal(rows[True][key], rows[False][key]), key
