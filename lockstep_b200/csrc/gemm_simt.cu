@@ -295,7 +295,7 @@ int launch_skinny(const float* A, const float* W, float* C, int M, int N, int K,
     if (M <= 16) LS_SKINNY(1, 2, 8, 2, 128);
     LS_SKINNY(1, 4, 8, 2, 128);
   }
-  if (GLU || N <= 16 * 8 * 148) {
+  if (GLU || N <= 16 * 8 * ls_sm_count()) {
     if (M <= 4) LS_SKINNY(2, 1, 4, 1, 256);
     if (M <= 8) LS_SKINNY(2, 2, 4, 1, 256);
     if (M <= 16) LS_SKINNY(1, 2, 8, 4, 128);

@@ -6,8 +6,10 @@
 // top_p; the draw u * mass(head) picks the first rank whose cumulative mass
 // reaches it.  u is word 0 of Philox-4x32-10 with counter (pos_lo, pos_hi, 0, 0)
 // and the request's 64-bit key, times 2^-32.  No sort is done: the rank that a
-// target mass falls on is found by bisection on the bit pattern of p (32 block
-// sums in a fixed order), then ties of that value are counted in id order.
+// target mass falls on is found on the bit pattern of p, up to 163,840 tokens digit by
+// digit over histograms in shared memory (sample_cluster_kernel), beyond by bisection with a
+// scratch of p in memory (sample_kernel: 32 block sums in a fixed order); then ties of that
+// value are counted in id order.
 // Every sum is taken in an order fixed by the vocabulary size alone, or is a sum of whole numbers.
 #include <math_constants.h>
 
@@ -230,8 +232,11 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ probs,
 // 526); 64 rows of 32,768: 32 us (510).
 // --------------------------------------------------------------------------
 constexpr int SAMPLE_CLUSTER = 8;                   // most blocks a row is spread over
-constexpr int SAMPLE_MOST = 8 * 1024 * 20;          // largest vocabulary of this kernel
+// Largest vocabulary of this kernel.  Masses in units of 2^-46 fit 64 bits up to 262,143 tokens of e = 1, and eight blocks
+// hold 393,216; above this line sample_kernel is what has been run.
+constexpr int SAMPLE_MOST = 163840;
 constexpr int SAMPLE_PART = 49152;                  // most tokens of a block: 192 KB of shared memory
+static_assert(SAMPLE_MOST <= 4 * SAMPLE_PART, "clusters of four hold every row");
 constexpr int SAMPLE_BINS = 1024;                   // a thread adds up one bin
 constexpr int SAMPLE_UNIT = 46;                     // masses over the whole row: units of 2^-46
 static_assert(SAMPLE_BINS == SAMPLE_THREADS, "a thread a bin");
@@ -634,7 +639,7 @@ LS_API int ls_sample(const float* logits, float* probs, const float* temperature
     // spread does, the fewest blocks that hold a row
 #define LS_SAMPLE_AS(CL) \
   return launch_sample_cluster<CL>(logits, temperature, top_p, keys, positions, out, rows, vocab, stream)
-    if (vocab > 4 * SAMPLE_PART || rows <= sample_rows_at_once<8>()) LS_SAMPLE_AS(8);
+    if (rows <= sample_rows_at_once<8>()) LS_SAMPLE_AS(8);
     if (vocab > 2 * SAMPLE_PART || rows <= sample_rows_at_once<4>()) LS_SAMPLE_AS(4);
     if (vocab > SAMPLE_PART || rows <= sample_rows_at_once<2>()) LS_SAMPLE_AS(2);
     LS_SAMPLE_AS(1);

@@ -171,8 +171,8 @@ class StaticMixedContext:
         self.plan_keys = sorted(plan_keys, key=lambda key: (mask_parts(key[0]), key[1]))
         self.device, self.err, self.split_size = device, err, split_size
         t = tokens
-        # (a few items more than the tokens make in one portion: a launcher that chooses a kernel
-        # by the number of items then sees about the real number)
+        # (as many items as the tokens can make in that many portions: a launcher that chooses a kernel by the
+        # number of items sees this number, up to fifteen more than a step of few portions has)
         self._tile_cap = {key: t // key[1] + portions for key in self.plan_keys}
         size = 3 * t + wanted_cap
         self._off = {}

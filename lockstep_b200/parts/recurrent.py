@@ -75,7 +75,7 @@ def _f32(t: torch.Tensor) -> torch.Tensor:
 
 class GatedDelta(Mixer):
     graph_safe = True
-    accepts_normed_rows = True       # its one product of the mixer's input can make the norm itself
+    accepts_normed_rows = True       # (with a decay per channel: its one product of the input can make the norm itself)
 
     def __init__(self, hidden_size, num_heads, num_kv_heads, key_dim, value_dim, conv_taps, norm_eps, unit_eps,
                  runtime: Runtime, decay_rank=None, gate_rank=None, decay="channel", gate="low_rank"):
@@ -435,7 +435,6 @@ class Retention(Mixer):
 
 class MLstm(Mixer):
     graph_safe = True
-    accepts_normed_rows = True
     can_overwrite = True
 
     def __init__(self, hidden_size, num_heads, key_dim, value_dim, gate_cap, norm_eps, runtime: Runtime, names=None):
@@ -472,7 +471,6 @@ class MLstm(Mixer):
     def forward(self, x, ctx, cache, residual, overwrite=False):
         rt, tokens, at = self.rt, residual.shape[0], self.at
         proj, gates = rt.rows(tokens, self.w_in.shape[0]), rt.rows(tokens, 2 * self.H, dtype=torch.float32)
-        x = x.materialize() if isinstance(x, NormedRows) else x          # two products share the normed rows
         K.gemm_nt(x, self.w_in, proj, err=rt.err)
         K.gemm_nt(x, self.w_gates, gates, err=rt.err)
         portions, cap = portion_list(ctx, cache.state, rt)

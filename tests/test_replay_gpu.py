@@ -239,8 +239,8 @@ def test_bfloat16_rows_do_not_depend_on_the_neighbours(zoo, name):
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("name", ["B", "D", "E"])
 def test_steps_of_mixed_portions_are_recorded_when_their_shape_repeats(zoo, name, dtype):
-    """Steps of the same shape (a step that fills a token budget, say) come again and again: from
-    the second on they are recorded, later ones replay the recording.  Whole prompts of equal
+    """Steps of the same shape (a step that fills a token budget, say) come again and again: the
+    third is recorded, later ones replay the recording.  Whole prompts of equal
     length one after the other, then portions beside decoded tokens of three other requests: the
     rows agree with the plain implementation and, bit for bit, with a runner that records nothing."""
     from lockstep_b200.engine import ModelRunner
