@@ -47,26 +47,42 @@ struct RowsShare {
   float p[ROWS][PP];
 };
 
-template <int D, int R>
-__global__ void __launch_bounds__(128, 2)
-attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ pages, float* __restrict__ out,
-                      const int* __restrict__ work, const int* __restrict__ block_table, int table_stride, int nq, int nkv,
-                      int page_size, int num_pages, int window, int keep_first, float scale, float softcap,
-                      const float* __restrict__ slopes, const float* __restrict__ log_rates,
-                      const float* __restrict__ sinks, int* err) {
-  ls_dependency_sync();
+struct RowsArgs {
+  const float *__restrict__ q, *__restrict__ pages;
+  float* __restrict__ out;
+  const int *__restrict__ work, *__restrict__ block_table;
+  int table_stride, nq, nkv, page_size, num_pages, window, keep_first;
+  float scale, softcap;
+  const float *__restrict__ slopes, *__restrict__ log_rates, *__restrict__ sinks;
+  int* err;
+};
+
+// The rows of this block's item, or (ONE_GROUP) only those of a group of 16 tokens over the keys of its own 16-token
+// tile.  Returns whether this thread has written a NaN.
+template <int D, int R, bool ONE_GROUP>
+__device__ __forceinline__ bool rows_pass(const RowsArgs& args, int group) {
+  const float *__restrict__ q = args.q, *__restrict__ pages = args.pages;
+  float* __restrict__ out = args.out;
+  const float *__restrict__ slopes = args.slopes, *__restrict__ log_rates = args.log_rates, *__restrict__ sinks = args.sinks;
+  const int nq = args.nq, nkv = args.nkv, page_size = args.page_size, num_pages = args.num_pages;
+  const int window = args.window, keep_first = args.keep_first;
+  const float scale = args.scale, softcap = args.softcap;
+  int* err = args.err;
   typedef RowsShare<D, R> Share;
   extern __shared__ __align__(16) float rows_smem[];
   Share& sh = *reinterpret_cast<Share*>(rows_smem);
-  const int* w = work + (int64_t)blockIdx.x * 8;
+  const int* w = args.work + (int64_t)blockIdx.x * 8;
   const int req_row = w[0], tok0 = w[1], ntok = w[2], pos0 = w[3];
-  if (ntok == 0) return;                     // padding item of a recorded launch
-  int split_begin = w[4], split_end = w[5], leading = w[7];
   const int h = (int)blockIdx.y, kvh = h / (nq / nkv);
   const int tid = threadIdx.x, mg = tid >> 3, sub = tid & 7;
-  const int* table_row = block_table + (int64_t)req_row * table_stride;
-  int pos_last = pos0 + ntok - 1;
-  int key_lo_tile = ls_first_key(pos0, window);
+  const int* table_row = args.block_table + (int64_t)req_row * args.table_stride;
+  // (a group's bounds: what the plan of 16-token tiles has)
+  const int first = ONE_GROUP ? pos0 + 16 * group : pos0;
+  const int pos_last = ONE_GROUP ? min(first + 15, pos0 + ntok - 1) : pos0 + ntok - 1;
+  const int key_lo_tile = ls_first_key(first, window);
+  const int split_begin = ONE_GROUP ? key_lo_tile / LS_SPLIT : w[4];
+  const int split_end = ONE_GROUP ? pos_last / LS_SPLIT + 1 : w[5];
+  const int leading = ONE_GROUP ? min((keep_first + LS_SPLIT - 1) / LS_SPLIT, split_begin) : w[7];
   const float slope = slopes != nullptr ? slopes[h] : 0.f;
   const float log_rate = log_rates != nullptr ? log_rates[h] : 0.f;
 
@@ -108,15 +124,12 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ pag
     }
   };
 
-  // pass 0: all rows of the item; pass g + 1, after a NaN: the rows of group g (rows 16 g .. 16 g + 15)
-#pragma unroll 1
-  for (int pass = 0;; ++pass) {
   Cursor cur;
   cur.turn = split_begin - leading;
   enter(cur);
   bool more = settle(cur);
   if (more) fetch(cur, 0);
-  for (int i = tid; pass == 0 && i < Share::ROWS * (D / 4); i += 128) {
+  for (int i = tid; i < Share::ROWS * (D / 4); i += 128) {
     const int r = i / (D / 4), c4 = 4 * (i - r * (D / 4));
     copy16_or_zero(&sh.q[r][c4], r < ntok ? q + ((int64_t)(tok0 + r) * nq + h) * D + c4 : nullptr);
   }
@@ -264,7 +277,7 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ pag
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const int m = mg + 16 * i;
-    if (m >= ntok || (pass > 0 && i != pass - 1)) continue;
+    if (m >= ntok || (ONE_GROUP && i != group)) continue;
     if (sinks != nullptr) {
       // a sink: one more term exp(sinks[head]) in the softmax's denominator, with no value
       float alpha, beta, m_new;
@@ -285,23 +298,28 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ pag
       nan |= !(y.x == y.x && y.y == y.y && y.z == y.z && y.w == y.w);
     }
   }
-  if (pass == 0 && !__syncthreads_or(nan)) return;
-  if (16 * pass >= ntok) return;
-  // the next group's bounds, as the plan of 16-token tiles has them
-  const int first = pos0 + 16 * pass;
-  pos_last = min(first + 15, pos0 + ntok - 1);
-  key_lo_tile = ls_first_key(first, window);
-  split_begin = key_lo_tile / LS_SPLIT;
-  split_end = pos_last / LS_SPLIT + 1;
-  leading = min((keep_first + LS_SPLIT - 1) / LS_SPLIT, split_begin);
+  return nan;
+}
+
+// (not inlined: the registers and the code of the usual pass stay its own)
+template <int D, int R>
+__device__ __noinline__ void rows_again(const RowsArgs& args, int ntok) {
+  for (int group = 0; 16 * group < ntok; ++group) {
+    __syncthreads();                          // everyone is done with the queries of the pass before
+    rows_pass<D, R, true>(args, group);
   }
 }
 
 template <int D, int R>
-int launch_rows(const float* q, const float* pages, float* out, const int* work, int n_work, const int* block_table,
-                int table_stride, int nq, int nkv, int page_size, int num_pages, int window, int keep_first, float scale,
-                float softcap, const float* slopes, const float* log_rates, const float* sinks, int* err,
-                cudaStream_t stream) {
+__global__ void __launch_bounds__(128, 2) attention_rows_kernel(const __grid_constant__ RowsArgs args) {
+  ls_dependency_sync();
+  const int ntok = args.work[(int64_t)blockIdx.x * 8 + 2];
+  if (ntok == 0) return;                     // padding item of a recorded launch
+  if (__syncthreads_or(rows_pass<D, R, false>(args, 0))) rows_again<D, R>(args, ntok);
+}
+
+template <int D, int R>
+int launch_rows(const RowsArgs& args, int n_work, cudaStream_t stream) {
   constexpr int smem = (int)sizeof(RowsShare<D, R>);
   static bool configured = false;
   if (!configured) {
@@ -310,8 +328,7 @@ int launch_rows(const float* q, const float* pages, float* out, const int* work,
     configured = true;
   }
   LS_COUNT(LS_K_ATTENTION_ROWS);
-  ls_launch(attention_rows_kernel<D, R>, dim3(n_work, nq), 128, smem, stream, q, pages, out, work, block_table, table_stride,
-            nq, nkv, page_size, num_pages, window, keep_first, scale, softcap, slopes, log_rates, sinks, err);
+  ls_launch(attention_rows_kernel<D, R>, dim3(n_work, args.nq), 128, smem, stream, args);
   return ls_launch_status();
 }
 
@@ -360,9 +377,9 @@ LS_API int ls_attention_rows(const float* q, const float* pages, float* out, con
   if (keep_first < 0 || (log_rates != nullptr && slopes == nullptr)) return LS_E_SIZE;
   if (nq <= 0 || nkv <= 0 || nq % nkv || nq > 65535 || page_size <= 0 || LS_SPLIT % page_size) return LS_E_SIZE;
   if (((uintptr_t)pages & 15) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15)) return LS_E_ALIGN;
-#define LS_ROWS(D, R)                                                                                                   \
-  return launch_rows<D, R>(q, pages, out, work, n_work, block_table, table_stride, nq, nkv, page_size, num_pages, window, \
-                           keep_first, scale, softcap, slopes, log_rates, sinks, err, stream)
+  const RowsArgs args = {q, pages, out, work, block_table, table_stride, nq, nkv, page_size, num_pages, window, keep_first,
+                         scale, softcap, slopes, log_rates, sinks, err};
+#define LS_ROWS(D, R) return launch_rows<D, R>(args, n_work, stream)
   if (d == 128 && tile_tokens == 64) LS_ROWS(128, 4);
   if (d == 128 && tile_tokens == 32) LS_ROWS(128, 2);
   if (d == 64 && tile_tokens == 64) LS_ROWS(64, 4);
