@@ -338,12 +338,26 @@ class DecodeGraphs:
             r.rt.exact_sizes = False
             if collecting:
                 gc.enable()
+        ctx.recorded_portions = getattr(ctx, "_portion_list", None)      # (lives as long as the graphs that read it)
         recorded = K.LAUNCHES[0] - before
         K.LAUNCHES[0] = before               # recording launches nothing
         # the last step's result is the logits: the graph's own buffer when that step is
         # recorded, else what the step returns at every replay
         logits = h if pieces[-1][0] is not None else None
         return pieces, ctx, stream, logits, recorded
+
+    @staticmethod
+    def _play(pieces, ctx, h):
+        for graph, fns in pieces:
+            if graph is not None:
+                graph.replay()
+            else:
+                # what a part keeps on the context of a step (recurrent.portion_list) is this step's: a recorded run has its own
+                # in its graph, and what the steps below kept at the replay before says nothing about this one
+                ctx._portion_list = None
+                for fn in fns:
+                    h = fn(h, ctx)
+        return h
 
     # -- steps that mix portions of prompts and decoded tokens --------------
     def mixed_key_for(self, entries) -> tuple | None:
@@ -413,12 +427,7 @@ class DecodeGraphs:
         pieces, ctx, h, logits, recorded = self.mixed[key]
         self.mixed.move_to_end(key)
         ctx.fill(entries, slots)
-        for graph, fns in pieces:
-            if graph is not None:
-                graph.replay()
-            else:
-                for fn in fns:
-                    h = fn(h, ctx)
+        h = self._play(pieces, ctx, h)
         K.LAUNCHES[0] += recorded
         self.mixed_replays += 1
         return (h if logits is None else logits)[:ctx.wanted]
@@ -434,12 +443,7 @@ class DecodeGraphs:
         ctx.fill(entries, slots)
         if tokens_device is not None:
             ctx.token_ids[:len(entries)].copy_(tokens_device, non_blocking=True)
-        for graph, fns in pieces:
-            if graph is not None:
-                graph.replay()
-            else:
-                for fn in fns:
-                    h = fn(h, ctx)
+        h = self._play(pieces, ctx, h)
         K.LAUNCHES[0] += recorded
         self.replays += 1
         return (h if logits is None else logits)[:len(entries)]

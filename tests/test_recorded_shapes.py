@@ -79,3 +79,28 @@ def test_a_class_stops_recording_and_the_other_goes_on(graphs):
     assert recorded == G.MIXED_RECORDINGS
     assert not any(see(graphs, key_of(graphs, [200])) for _ in range(5))
     assert [see(graphs, key_of(graphs, [2048])) for _ in range(3)] == [False, False, True]
+
+
+def test_steps_called_between_replays_look_their_portions_up_at_every_replay(graphs, monkeypatch):
+    """A part that is not recorded (a norm of a user's own, say) takes the recurrent mixer behind it out of the recording with
+    it: the list of portions that the mixer keeps on the context is then made for every step, also where a recorded run
+    made one in its graph."""
+    from lockstep_b200.parts import recurrent
+
+    monkeypatch.setattr(recurrent.K, "find_portions", lambda token_slot, out, cap, err: out[:len(token_slot)].copy_(token_slot))
+    seen = []
+
+    def mixer(h, ctx):
+        out, _ = recurrent.portion_list(ctx, torch.zeros(4, 1), SimpleNamespace(device="cpu", err=None))
+        seen.append(out[:2].tolist())
+        return h
+
+    ctx = SimpleNamespace(token_slot=torch.zeros(2, dtype=torch.int32), wanted=2, _portion_list=(torch.full((7,), -1), 2))
+    ctx.fill = lambda entries, slots: ctx.token_slot.copy_(torch.tensor(slots, dtype=torch.int32))
+    recorded = SimpleNamespace(replay=lambda: None)
+    logits = torch.zeros(2, 3)
+    for table, replay in ((graphs.graphs, graphs.replay), (graphs.mixed, graphs.replay_mixed)):
+        table["key"] = ([(recorded, None), (None, [mixer, mixer]), (recorded, None)], ctx, None, logits, 0)
+        for slots in ([0, 1], [2, 3]):
+            replay("key", [None, None], slots)
+    assert seen == 2 * [[0, 1], [0, 1], [2, 3], [2, 3]]
