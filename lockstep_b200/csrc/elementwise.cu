@@ -97,7 +97,7 @@ __device__ __forceinline__ void ls_store4(TO* p, float a, float b, float c, floa
 // 1,024 to 4,096 elements), so that a row's reads are in flight together, and EARLY asks
 // for the gains, which no kernel writes, before the wait on the kernel before; with many rows
 // the registers of more than 8 groups and their gains would cost more rows an SM than that
-// saves (2,048 rows of 2,560 with 32 groups: 13.7 us, with 16 and late gains 8.0).  Back to back,
+// saves (2,048 rows of 2,560 with 32 groups: 13.7 us, by rmsnorm_rows_kernel below 8.0).  Back to back,
 // 6 rows of 1,024 / 2,560 / 4,096: 1.6 / 3.3 / 4.6 us (with 16 groups and late gains 3.2 / 5.9 / 9.0);
 // 2,048 rows of 1,024: 2.4 us (4.0), 12.6 MB read and written at 5.2 TB/s.
 // y[0..4) = x * rstd * gain, in one access each for the gains and the outputs where `vec`
@@ -189,6 +189,73 @@ rmsnorm_kernel(const float* __restrict__ x, const int* __restrict__ row_index,
   }
 }
 
+// The same for many rows of more than 1,024 elements: 16 groups kept, gains read where they are used.  A kernel of
+// its own, since as an instance of the one above its loops over the rest of a row came out 3 to 35 % slower (2,048 rows
+// of 4,096 / 8,192 bfloat16 12.1 / 36.0 us, there 13.3 / 42.3; 1,024 rows of 8,192 float32 25.4, there 34.0).
+template <typename TO, typename TG>
+__global__ void __launch_bounds__(128)
+rmsnorm_rows_kernel(const float* __restrict__ x, const int* __restrict__ row_index,
+                    const TG* __restrict__ gain_all, TO* __restrict__ y, int rows, int width, int src_rows,
+                    float eps, int parts, int64_t x_ld, int* err) {
+  ls_dependency_sync();
+  constexpr int KEEP = 64;                    // floats a lane keeps: 16 float4
+  const int lane = threadIdx.x & 31;
+  // a row of `parts` equal consecutive parts, each normalised by its own root mean square, is
+  // `parts` rows of `width` elements to this kernel (the gain runs over the whole row)
+  const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (unit >= rows * parts) return;
+  const int r = unit / parts, part = unit - r * parts;
+  int src = row_index ? row_index[r] : r;
+  if (src < 0 || src >= src_rows) {
+    if (lane == 0) ls_record_fault(err, LS_DEV_ROW_RANGE, r);
+    src = 0;
+  }
+  // (x_ld: the source rows' pitch, where the normed columns are the first of a wider row)
+  const float* xr = x + (int64_t)src * x_ld + (int64_t)part * width;
+  TO* yr = y + ((int64_t)r * parts + part) * width;
+  const TG* gain = gain_all + (int64_t)part * width;
+  const bool vec = (width & 3) == 0 && ((uintptr_t)xr & 15) == 0;
+  // four outputs an access where the outputs and the gains allow it (this changes no sum)
+  const bool vec_out = ((uintptr_t)y & (4 * sizeof(TO) - 1)) == 0 && ((uintptr_t)gain & (4 * sizeof(TG) - 1)) == 0;
+  float keep[KEEP];
+  float ss = 0.f;
+  if (vec) {
+    const int groups = width >> 2;
+#pragma unroll
+    for (int i = 0; i < KEEP / 4; ++i) {
+      const int g = lane + 32 * i;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (g < groups) v = *reinterpret_cast<const float4*>(xr + 4 * g);
+      keep[4 * i + 0] = v.x; keep[4 * i + 1] = v.y; keep[4 * i + 2] = v.z; keep[4 * i + 3] = v.w;
+      ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
+    }
+    for (int g = lane + 32 * (KEEP / 4); g < groups; g += 32) {
+      const float4 v = *reinterpret_cast<const float4*>(xr + 4 * g);
+      ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
+    }
+  } else {
+    for (int i = lane; i < width; i += 32) ss = fmaf(xr[i], xr[i], ss);
+  }
+  ss = ls_warp_sum(ss);
+  const float rstd = 1.0f / sqrtf(ss / (float)width + eps);
+  if (vec) {
+    const int groups = width >> 2;
+#pragma unroll
+    for (int i = 0; i < KEEP / 4; ++i) {
+      const int g = lane + 32 * i;
+      if (g < groups) rmsnorm_out4<TO, TG>(yr + 4 * g, gain + 4 * g, keep + 4 * i, rstd, vec_out);
+    }
+    for (int g = lane + 32 * (KEEP / 4); g < groups; g += 32) {
+      const float4 v = *reinterpret_cast<const float4*>(xr + 4 * g);
+      const float four[4] = {v.x, v.y, v.z, v.w};
+      rmsnorm_out4<TO, TG>(yr + 4 * g, gain + 4 * g, four, rstd, vec_out);
+    }
+  } else {
+    for (int i = lane; i < width; i += 32)
+      yr[i] = ls_from_float<TO>(xr[i] * rstd * ls_to_float<TG>(gain[i]));
+  }
+}
+
 LS_API int ls_rmsnorm(const float* x, const int* row_index, const void* gain, int gain_dtype,
                       void* y, int y_dtype, int rows, int row_width, int src_rows, float eps,
                       int parts, int64_t x_ld, int* err, cudaStream_t stream) {
@@ -206,7 +273,9 @@ LS_API int ls_rmsnorm(const float* x, const int* row_index, const void* gain, in
 #define LS_RMS(TO, TG)                                              \
   do {                                                              \
     if (width <= 1024) LS_RMS_AS(TO, TG, 8, true);                  \
-    else if (warps > 1) LS_RMS_AS(TO, TG, 16, false);               \
+    else if (warps > 1)                                             \
+      LS_COUNT(LS_K_RMSNORM), ls_launch(rmsnorm_rows_kernel<TO, TG>, blocks, warps * 32, 0, stream, x, row_index, \
+                                        (const TG*)gain, (TO*)y, rows, width, src_rows, eps, parts, x_ld, err);   \
     else if (width <= 2048) LS_RMS_AS(TO, TG, 16, true);            \
     else if (width <= 3072) LS_RMS_AS(TO, TG, 24, true);            \
     else LS_RMS_AS(TO, TG, 32, (sizeof(TG) == 2));                  \
