@@ -1950,8 +1950,17 @@ LS_API int ls_gemm_nt_tc_rmsnorm(const float* h, const int* row_index, int src_r
 // product (us, inside / apart): 8 rows of 1,024, 4,096 features 6.1 / 6.2, 16 rows 8.2 / 7.0, 32 rows 12.5 / 8.3; 8 rows
 // of 2,048 with a share of 512 columns 8.2 / 8.8, of 1,024 columns 11.5 / 10.7; 8 rows of 2,560 20.5 / 15.6; a norm in
 // two parts, 2 trips for the sums and a division a group: 8 rows 14.0 / 9.9, 1 row 11.9 / 8.4.
+// Rows of more than 2,048 elements: what counts is whether the product's clusters run all at one time, which 14 of eight blocks do.
+// 1,024 to 1,792 features 1 / 8 rows inside take 0.79 to 0.90 / 0.90 to 0.99 of apart at 2,304 to 4,096 elements, 0.72 / 0.80 at 5,120,
+// 0.61 / 0.66 at 8,192 (a norm of one row is a kernel of one warp), 2,048 features 1.07 to 1.11 / 1.15 to 1.19 at 2,304 to 4,096; 9 and 16
+// rows 1.2 to 1.3 up to 4,096 elements, 1.04 to 1.12 at 5,120, 0.91 to 0.97 at 8,192.  At 8,192 elements 1 / 8 rows inside are still
+// as fast or faster at 2,048 features (0.89 / 0.95) and 3,072 (0.98 / 1.01; 144 blocks).
 LS_API int ls_gemm_tc_norm_inside(int T, int N, int K, int epilogue, int parts) {
-  return T <= 8 && parts == 1 && K <= 2048 && make_plan(T, N, K, epilogue).kb_per_share <= 8 ? 1 : 0;
+  if (T > 16 || parts != 1) return 0;
+  const Plan plan = make_plan(T, N, K, epilogue);
+  if (K <= 2048) return T <= 8 && plan.kb_per_share <= 8 ? 1 : 0;
+  const int blocks = (N + 127) / 128 * plan.shares;
+  return (T <= 8 || K >= 8192) && (blocks <= 14 * 8 || (T <= 8 && K >= 8192 && blocks <= 144)) ? 1 : 0;
 }
 
 // The q/k/v projection of few tokens with its heads finished in the epilogue: what

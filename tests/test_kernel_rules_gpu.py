@@ -367,3 +367,26 @@ def test_rows_normed_inside_the_product_or_before_it_have_the_same_bits(width, g
         outs.append(out[3].clone())
     k.raise_on_fault(err)
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("width,features,t,inside", [(2304, 1024, 1, True), (2560, 1792, 8, True), (2560, 1024, 9, False),
+                                                     (4096, 256, 3, True), (4096, 2048, 8, False), (5120, 640, 8, True),
+                                                     (8192, 1024, 16, True), (8192, 1024, 17, False), (8192, 2048, 1, True), (8192, 2048, 9, False),
+                                                     (8192, 4096, 2, False)])
+def test_wide_rows_normed_inside_a_product_of_few_blocks_have_the_bits_of_the_kernel_before_it(width, features, t, inside):
+    """Above 2,048 elements the norm rides inside products whose blocks run at one time: 14 clusters of eight."""
+    k = K()
+    g = torch.Generator().manual_seed(width + features)
+    h = (torch.randn(t, width, generator=g) * 2).to(dev())
+    gain = (1 + 0.1 * torch.randn(width, generator=g)).to(torch.bfloat16).to(dev())
+    w = (torch.randn(features, width, generator=g) * 0.05).to(torch.bfloat16).to(dev())
+    err = k.new_error_word(dev())
+    assert k.norm_inside_pays(t, features, w) == inside
+    apart, rows = torch.empty(t, features, dtype=torch.bfloat16, device=dev()), torch.empty(t, width, dtype=torch.bfloat16, device=dev())
+    k.rmsnorm(h, gain, rows, 1e-6, err)
+    k.gemm_nt(rows, w, apart, err=err)
+    out = torch.empty_like(apart)
+    if inside:
+        assert k.gemm_nt_tc_rmsnorm(h, gain, 1e-6, w, out, k.EPILOGUE_STORE, err)
+        assert torch.equal(out, apart)
+    k.raise_on_fault(err)
