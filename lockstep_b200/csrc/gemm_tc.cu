@@ -1953,14 +1953,16 @@ LS_API int ls_gemm_nt_tc_rmsnorm(const float* h, const int* row_index, int src_r
 // Rows of more than 2,048 elements: what counts is whether the product's clusters run all at one time, which 14 of eight blocks do.
 // 1,024 to 1,792 features 1 / 8 rows inside take 0.79 to 0.90 / 0.90 to 0.99 of apart at 2,304 to 4,096 elements, 0.72 / 0.80 at 5,120,
 // 0.61 / 0.66 at 8,192 (a norm of one row is a kernel of one warp), 2,048 features 1.07 to 1.11 / 1.15 to 1.19 at 2,304 to 4,096; 9 and 16
-// rows 1.2 to 1.3 up to 4,096 elements, 1.04 to 1.12 at 5,120, 0.91 to 0.97 at 8,192.  At 8,192 elements 1 / 8 rows inside are still
-// as fast or faster at 2,048 features (0.89 / 0.95) and 3,072 (0.98 / 1.01; 144 blocks).
+// rows 1.2 to 1.3 up to 4,096 elements, 1.04 to 1.12 at 5,120, 0.91 to 0.97 at 8,192.  The deeper the product, the less
+// another round of its clusters matters beside the norm: at 6,144 elements 2,048 / 4,096 features (128 blocks) 0.96 to 1.00 / 0.83 to 0.89,
+// 3,072 / 6,144 (144 blocks) 1.00 to 1.05 / 1.16 to 1.20; at 8,192 2,048 / 3,072 / 4,096 features 0.90 to 0.94 / 0.96 to 1.01 / 0.74 to 0.78.
 LS_API int ls_gemm_tc_norm_inside(int T, int N, int K, int epilogue, int parts) {
   if (T > 16 || parts != 1) return 0;
   const Plan plan = make_plan(T, N, K, epilogue);
   if (K <= 2048) return T <= 8 && plan.kb_per_share <= 8 ? 1 : 0;
   const int blocks = (N + 127) / 128 * plan.shares;
-  return (T <= 8 || K >= 8192) && (blocks <= 14 * 8 || (T <= 8 && K >= 8192 && blocks <= 144)) ? 1 : 0;
+  if (T > 8) return K >= 8192 && blocks <= 14 * 8 ? 1 : 0;
+  return blocks <= (K >= 8192 ? 144 : K >= 6144 ? 128 : 14 * 8) ? 1 : 0;
 }
 
 // The q/k/v projection of few tokens with its heads finished in the epilogue: what

@@ -372,9 +372,9 @@ def test_rows_normed_inside_the_product_or_before_it_have_the_same_bits(width, g
 @pytest.mark.parametrize("width,features,t,inside", [(2304, 1024, 1, True), (2560, 1792, 8, True), (2560, 1024, 9, False),
                                                      (4096, 256, 3, True), (4096, 2048, 8, False), (5120, 640, 8, True),
                                                      (8192, 1024, 16, True), (8192, 1024, 17, False), (8192, 2048, 1, True), (8192, 2048, 9, False),
-                                                     (8192, 4096, 2, False)])
+                                                     (8192, 4096, 2, True), (6144, 2048, 8, True), (6144, 3072, 1, False)])
 def test_wide_rows_normed_inside_a_product_of_few_blocks_have_the_bits_of_the_kernel_before_it(width, features, t, inside):
-    """Above 2,048 elements the norm rides inside products whose blocks run at one time: 14 clusters of eight."""
+    """Above 2,048 elements the norm rides inside products whose blocks run at one time (14 clusters of eight), or nearly."""
     k = K()
     g = torch.Generator().manual_seed(width + features)
     h = (torch.randn(t, width, generator=g) * 2).to(dev())
