@@ -281,7 +281,10 @@ int launch_skinny_as(const float* A, const float* W, float* C, int M, int N, int
 
 // Which thread makes an element changes no bit.  Narrow (a feature a thread, 8 features a block): a weight of
 // 1,024 rows then lies on 128 SMs (16 a block: K = 3,072, 3 tokens, 22 us against 15).  Middle: two features a
-// thread, to 16 tokens.  Wide, more than eight blocks of 16 features an SM: two features a thread and the tokens on as
+// thread, to 8 tokens.  5 to 8 tokens in blocks of 16 features take 100 KB of stages each, two an SM, and above 32 features an
+// SM would start another round over the device, so there blocks hold 32 (8 tokens of 4,736 / 4,800 / 6,144 / 9,472 features and K = 1,024:
+// in blocks of 16 11.3 / 19.2 / 19.8 / 21.8 us, of 32 13.3 / 14.0 / 14.6 / 15.5).  17 to 32 tokens on four lanes, eight a thread, a feature each (32
+// tokens of 2,560 / 6,144 / 8,192 features 26.1 / 51.1 / 51.3 us; with two features a thread 27.0 / 53.3 / 54.2).  Wide, more than eight blocks of 16 features an SM: two features a thread and the tokens on as
 // few lanes as their number allows, since what is read from shared memory bounds it (8 tokens of a head: 185 us, a
 // token a lane 265).
 template <bool GLU>
@@ -293,14 +296,15 @@ int launch_skinny(const float* A, const float* W, float* C, int M, int N, int K,
     if (M <= 4) LS_SKINNY(1, 1, 4, 1, 256);
     if (M <= 8) LS_SKINNY(1, 1, 8, 2, 256);
     if (M <= 16) LS_SKINNY(1, 2, 8, 2, 128);
-    LS_SKINNY(1, 4, 8, 2, 128);
+    LS_SKINNY(1, 4, 8, 2, 64);
   }
   if (GLU || N <= 16 * 8 * ls_sm_count()) {
     if (M <= 4) LS_SKINNY(2, 1, 4, 1, 256);
+    if (M <= 8 && !GLU && N > 32 * ls_sm_count()) LS_SKINNY(2, 2, 4, 2, 128);
     if (M <= 8) LS_SKINNY(2, 2, 4, 1, 256);
     if (M <= 16) LS_SKINNY(1, 2, 8, 4, 128);
     if (GLU) LS_SKINNY(1, 4, 8, 4, 128);
-    LS_SKINNY(2, 8, 4, 1, 64);
+    LS_SKINNY(1, 8, 4, 2, 64);
   }
   if constexpr (!GLU) {
     if (M <= 4) LS_SKINNY(2, 4, 1, 2, 32);
@@ -321,7 +325,7 @@ bool skinny_applies(const void* A, const void* W, int a_dtype, int c_dtype, int 
 // ---------------------------------------------------------------------------
 // Many tokens, float32: the prompt's products on the true 32-bit path.  A block owns TM tokens x WR
 // rows of W (silu-mul: the gate rows and the up rows of WR / 2 features), a thread 8 x WR / 16 of
-// them as 4 x 4 corners.  FMAs go out two lanes an instruction (two columns, one token).  The next
+// them as 4 x 4 corners.  FMAs go out two lanes an instruction (PAIRS: two columns, one token) or one.  The next
 // k-block is on its way from memory to registers while this one is multiplied.  Every element is
 // still one accumulator and one ascending chain fmaf(a, w, acc), so the bits are those of the two
 // kernels above.  What bounds it: FMAs and, beside them, what threads read from shared memory (an SM
@@ -331,7 +335,7 @@ bool skinny_applies(const void* A, const void* W, int a_dtype, int c_dtype, int 
 // ---------------------------------------------------------------------------
 constexpr int LK = 16;
 
-template <int EPI, int TM, int WR>
+template <int EPI, int TM, int WR, bool PAIRS>
 __global__ void __launch_bounds__(2 * TM, 256 / TM)
 gemm_nt_large_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N,
                      int K, int64_t lda, int64_t ldw, int64_t ldc) {
@@ -413,7 +417,14 @@ gemm_nt_large_kernel(const float* __restrict__ A, const float* __restrict__ W, f
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < WC / 2; ++j) ls_fma_pair(pair[i][j], a[i], w[j]);
+        for (int j = 0; j < WC / 2; ++j) {
+          if constexpr (PAIRS) {
+            ls_fma_pair(pair[i][j], a[i], w[j]);
+          } else {
+            pair[i][j].x = fmaf(a[i], w[j].x, pair[i][j].x);
+            pair[i][j].y = fmaf(a[i], w[j].y, pair[i][j].y);
+          }
+        }
     }
     if (more) {
       stage(buf ^ 1);
@@ -451,7 +462,7 @@ gemm_nt_large_kernel(const float* __restrict__ A, const float* __restrict__ W, f
   }
 }
 
-template <int EPI, int TM, int WR>
+template <int EPI, int TM, int WR, bool PAIRS = true>
 int launch_large_as(const float* A, const float* W, float* C, int M, int N, int K, int64_t lda, int64_t ldw,
                     int64_t ldc, cudaStream_t stream) {
   constexpr int FN = EPI == 2 ? WR / 2 : WR;
@@ -460,7 +471,7 @@ int launch_large_as(const float* A, const float* W, float* C, int M, int N, int 
   for (; M > 0; M -= MOST, A += (int64_t)MOST * lda, C += (int64_t)MOST * ldc) {
     const int rows = M < MOST ? M : MOST;
     LS_COUNT(LS_K_GEMM_SIMT_MANY);
-    ls_launch(gemm_nt_large_kernel<EPI, TM, WR>, dim3((N + FN - 1) / FN, (rows + TM - 1) / TM), 2 * TM, 0, stream, A, W, C, rows, N,
+    ls_launch(gemm_nt_large_kernel<EPI, TM, WR, PAIRS>, dim3((N + FN - 1) / FN, (rows + TM - 1) / TM), 2 * TM, 0, stream, A, W, C, rows, N,
               K, lda, ldw, ldc);
   }
   return ls_launch_status();
@@ -472,14 +483,19 @@ int launch_large(const float* A, const float* W, float* C, int M, int N, int K, 
   // The tile's size changes no sum.  Tiles of 64 x 128 (four blocks an SM) where there are three or more an SM:
   // 1,800 tokens of 4,096 features 334 us (64 x 64: 373, 128 x 64: 385).  With fewer tiles the trip to memory of
   // a k-block bounds a block, and more and smaller tiles are faster, 64 x 64 (600 tokens of 4,096 features 167 us,
-  // 64 x 128: 195), except where 128 x 64 is just one round of two blocks an SM (1,800 tokens of 1,024
-  // features and K = 2,048: 234 us, 64 x 64: 246).
+  // 64 x 128: 195), up to two of them an SM; with more, tiles of 128 x 64 where they are at most two an SM (1,500 / 1,800
+  // tokens of 1,024 features, K = 1,024: 114 / 114 us, 64 x 64: 118 / 122; 400 tokens of 2,560 features, 280 tiles of 64 x 64, K = 2,560:
+  // 278 us, 64 x 64: 238).  These do their FMAs one by one from K = 4,096 on (800 tokens of 2,560 features, K = 9,728: 1,100
+  // us, in pairs 1,195; 512 of 4,096, K = 4,096: 478 and 493) and in pairs below (2,048 of 1,024, K = 3,072: 349 and 335).
   const long long sms = ls_sm_count(), rows64 = (M + 63LL) / 64, rows128 = (M + 127LL) / 128;
   if (rows128 > 65535) return LS_E_SIZE;
   if constexpr (EPI != 2) {
-    const long long tall = rows128 * ((N + 63) / 64);
+    const long long columns = (N + 63) / 64;
     if (rows64 * ((N + 127) / 128) < 3 * sms) {
-      if (2 * tall >= 3 * sms && tall <= 2 * sms) return launch_large_as<EPI, 128, 64>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+      if (rows64 * columns > 2 * sms && rows128 * columns <= 2 * sms) {
+        if (K >= 4096) return launch_large_as<EPI, 128, 64, false>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+        return launch_large_as<EPI, 128, 64>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+      }
       return launch_large_as<EPI, 64, 64>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     }
   }
