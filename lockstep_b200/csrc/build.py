@@ -31,7 +31,8 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC"]
 # library name -> sources.  "core" holds the kernels that take every size; the
 # others hold the tensor-core kernels for the sizes they are specialised for.
 LIBRARIES: dict[str, list[str]] = {
-    "core": ["elementwise.cu", "rowwise.cu", "gemm_simt.cu", "attention_simt.cu", "attention_rows.cu", "sampling.cu"],
+    "core": ["elementwise.cu", "rowwise.cu", "gemm_simt.cu", "attention_simt.cu", "attention_rows.cu", "attention_split.cu",
+             "sampling.cu"],
     "tc": ["gemm_tc.cu", "attention_decode_mma.cu", "attention_prefill_tc.cu"],
     # mixers with a carried state, routed experts, projections with heads of unequal sizes:
     # loaded when a model first builds a part that needs them

@@ -82,6 +82,8 @@ _SIGNATURES = {
         "ls_attention_rows_tile_class": [c_int, c_int, c_int, c_int],
         "ls_attention_rows": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int,
                               c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
+        "ls_attention_split": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
+                               c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
         "ls_attention_decode": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int,
                                 c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
                                 c_void_p, c_void_p, c_void_p, c_void_p],
@@ -637,6 +639,22 @@ def attention_rows(q, pages, out, work, n_work, tile_tokens, block_table, nq, nk
     if status in (-2, -3):
         return False
     _check(status, "attention_rows")
+    return True
+
+
+def attention_split(q, pages, part_acc, part_ml, work, n_work, block_table, nq, nkv, d, window, scale, err,
+                    keep_first: int = 0) -> bool:
+    """``attention_tile`` of single tokens' splits for float32, with the same bits (csrc/attention_split.cu): plain scores, groups of
+    1, 2, 4 or 8 heads of up to 128 elements.  Returns False, having launched nothing, for sizes and addresses it does
+    not take."""
+    status = library().ls_attention_split(
+        _dev(q, "q", torch.float32), _dev(pages, "pages", torch.float32), _dev(part_acc, "part_acc", torch.float32),
+        _dev(part_ml, "part_ml", torch.float32), _dev(work, "work", torch.int32), n_work,
+        _dev(block_table, "block_table", torch.int32), block_table.shape[-1], nq, nkv, d, pages.shape[3], pages.shape[0],
+        int(window), int(keep_first), float(scale), _dev(err, "err", torch.int32), _stream())
+    if status in (-2, -3):
+        return False
+    _check(status, "attention_split")
     return True
 
 

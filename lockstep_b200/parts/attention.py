@@ -147,6 +147,9 @@ def attend(rt: Runtime, q, ctx, cache, nq: int, nkv: int, d: int, mask, scale: f
                                       plan.n_split, cache.block_table, nq, nkv, d, window,
                                       scale, rt.err, extras.slopes, extras.log_rates, softcap=extras.softcap,
                                       keep_first=keep)
+        if exact and q.dtype == torch.float32 and extras.slopes is None and not extras.softcap:
+            done = K.attention_split(q, cache.pages, part_acc, part_ml, plan.split_work, plan.n_split, cache.block_table,
+                                     nq, nkv, d, window, scale, rt.err, keep_first=keep)
         if not done:
             K.attention_tile(q, cache.pages, None, part_acc, part_ml, plan.split_work,
                              plan.n_split, cache.block_table, nq, nkv, d, window,

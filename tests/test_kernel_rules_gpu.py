@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -389,3 +390,37 @@ def test_wide_rows_normed_inside_a_product_of_few_blocks_have_the_bits_of_the_ke
         assert k.gemm_nt_tc_rmsnorm(h, gain, 1e-6, w, out, k.EPILOGUE_STORE, err)
         assert torch.equal(out, apart)
     k.raise_on_fault(err)
+
+
+@pytest.mark.parametrize("nq,nkv,d,page,mask", [(4, 2, 128, 16, 0), (3, 3, 16, 8, 0), (8, 2, 64, 64, 100), (8, 1, 128, 32, (300, 40)),
+                                                (2, 1, 112, 16, -96), (4, 4, 128, 128, 0)])
+def test_float32_splits_of_single_tokens_have_the_bits_of_the_tile_kernel(nq, nkv, d, page, mask):
+    """Partials of every split of single tokens at the edges of tiles and splits, an infinity and a NaN among older values,
+    against the tile kernel's, bit for bit."""
+    from lockstep_b200.engine.batch import mask_parts, plan_attention
+
+    k = K()
+    g = torch.Generator().manual_seed(nq * d + page)
+    places = [0, 1, 30, 31, 32, 33, 127, 255, 256, 257, 511, 512, 700, 767]
+    count = -(-768 // page)
+    pages = torch.randn(count * len(places), 2, nkv, page, d, generator=g)
+    table = torch.randperm(count * len(places), generator=g).to(torch.int32).view(len(places), count).contiguous()
+    for key, value in ((3, math.inf), (763, math.nan)):          # of the last request alone
+        pages[int(table[-1, key // page]), 1, 0, key % page, 5:9] = value
+    q = torch.randn(len(places), nq * d, generator=g).to(dev())
+    pages, table = pages.to(dev()), table.to(dev())
+    _, split, _, n_slots = plan_attention([(i, i, p, 1) for i, p in enumerate(places)], mask, k.attention_split_size())
+    work = torch.from_numpy(np.concatenate([split, np.zeros((3, 8), dtype=np.int32)])).to(dev())      # null items at the end
+    window, keep = mask_parts(mask)
+    err, got = k.new_error_word(dev()), []
+    for kernel in (k.attention_split, k.attention_tile):
+        acc = torch.full((n_slots, nq, d), 7.0, device=dev())
+        ml = torch.full((n_slots, nq, 2), 7.0, device=dev())
+        if kernel is k.attention_split:
+            assert kernel(q, pages, acc, ml, work, len(work), table, nq, nkv, d, window, d ** -0.5, err, keep_first=keep)
+        else:
+            kernel(q, pages, None, acc, ml, work, len(work), table, nq, nkv, d, window, d ** -0.5, err, keep_first=keep)
+        got.append((acc.view(torch.int32), ml.view(torch.int32), acc.isnan()))
+    k.raise_on_fault(err)
+    assert bool(got[0][2].any()) and torch.equal(got[0][2], got[1][2])
+    assert torch.equal(got[0][0][~got[0][2]], got[1][0][~got[0][2]]) and torch.equal(got[0][1], got[1][1])
