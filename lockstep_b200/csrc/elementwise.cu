@@ -322,120 +322,128 @@ __global__ void qk_norm_rope_store_kernel(const T* __restrict__ qkv, const LsQkv
     ls_qkv_head_store<T>(args, reinterpret_cast<const T*>(row_smem) + head * args.d, t, head, lane, err);
 }
 
-// The same for bfloat16 heads of D = 64 or 128 elements that are rotated whole, at a fraction
-// of the instructions: what belongs to the token (position, page, cosines, sines, gains) is
-// looked up once per token and not once per head, a lane keeps its four (two) elements of a
-// head in registers and writes the results over the staged row, and the row leaves in 16-byte
-// pieces.  Every sum and product is ls_norm_rope_head's, in its order: the bits are the same.
+// The same for bfloat16 heads of D = 64 or 128 elements that are rotated whole.  What bounds it is instruction issue, so
+// half a warp has a head and a lane two neighbouring elements of every 32 (2 l + 32 j and 2 l + 1 + 32 j), read,
+// packed and written two at a time: the sum of squares keeps ls_norm_rope_head's chains (one for each of the
+// 32 residues, two a lane) and its tree, whose last step joins a lane's own two.  What belongs to the token (position,
+// page, cosines, sines, gains) is looked up once per lane, before the wait on the kernel before; the head goes from memory to
+// memory through registers, the next one asked for before this one is worked on.  Every sum and product is
+// ls_norm_rope_head's, in its order: the bits are the same.  (A warp a head, a lane single elements, the row staged in shared
+// memory: 2.3 us a layer more for 2,048 tokens of 16 query and 8 key heads of 128, 1.6 us more for 173.)
 template <int D>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128)
 qk_norm_rope_store_whole_kernel(const __nv_bfloat16* __restrict__ qkv, const LsQkvStore args, int tokens, int* err) {
   typedef __nv_bfloat16 bf16;
-  constexpr int PER_LANE = D / 32;                // a lane's elements of a head: lane, lane + 32, ...
-  constexpr int VEC = D / 8;                      // 16-byte pieces of a head
+  constexpr int J = D / 32;                       // a lane's pairs of a head
   ls_dependency_trigger();
-  extern __shared__ uint4 row_smem[];
   const int t = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int half = lane >> 4, l = lane & 15;      // this lane's head of the warp's two, and its place there
   const int nq = args.nq, nkv = args.nkv;
-  const int heads_total = nq + 2 * nkv;
-  // weights first: they do not wait for the kernel before
-  float gq[PER_LANE], gk[PER_LANE];
+  // the token's place (the same in every thread) and constants
+  const int pos = args.positions[t];
+  const bool pos_ok = pos >= 0 && pos < args.max_positions;
+  int page = 0;
+  bool page_ok = false;
+  if (args.write_cache && pos_ok) {
+    page = args.block_table[(int64_t)args.token_req[t] * args.table_stride + pos / args.page_size];
+    page_ok = page >= 0 && page < args.num_pages;
+  }
   const bool normed = args.q_gain != nullptr;
+  float2 gq[J], gk[J], cs[J / 2], sn[J / 2];
 #pragma unroll
-  for (int j = 0; j < PER_LANE; ++j) {
-    gq[j] = gk[j] = 1.f;
+  for (int j = 0; j < J; ++j) {
+    gq[j] = gk[j] = make_float2(1.f, 1.f);
     if (normed) {
-      const int i = lane + 32 * j;
+      const int i = 2 * l + 32 * j;
       if (args.gain_bf16) {
-        gq[j] = __bfloat162float(reinterpret_cast<const bf16*>(args.q_gain)[i]);
-        gk[j] = __bfloat162float(reinterpret_cast<const bf16*>(args.k_gain)[i]);
+        gq[j] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(reinterpret_cast<const bf16*>(args.q_gain) + i));
+        gk[j] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(reinterpret_cast<const bf16*>(args.k_gain) + i));
       } else {
-        gq[j] = reinterpret_cast<const float*>(args.q_gain)[i];
-        gk[j] = reinterpret_cast<const float*>(args.k_gain)[i];
+        gq[j] = *reinterpret_cast<const float2*>(reinterpret_cast<const float*>(args.q_gain) + i);
+        gk[j] = *reinterpret_cast<const float2*>(reinterpret_cast<const float*>(args.k_gain) + i);
       }
     }
   }
-  // the token's place (the same in every thread): from the step's inputs and constants alone, so up to 512 tokens
-  // it is looked up before the wait on the kernel before (64 decoded tokens 5.9 -> 4.3 us a launch in their step).
-  // Launched after itself, 16 query and 8 key heads of 128, before / after the wait: 64 tokens 2.6 / 3.1 us, 512 4.8 / 5.5, 640
-  // 5.8 / 6.5, 1,024 6.1 / 6.7, 2,048 10.2 / 10.7.  Above the line a step does not show it: without the line 2,048 tokens
-  // took 3.47 ms (3.49 with it), 8,192 tokens 21.27 (21.23).
-  int pos = 0, page = 0;
-  bool pos_ok = false, page_ok = false;
-  float cs[PER_LANE / 2], sn[PER_LANE / 2];
-  auto look_up = [&]() {
-    pos = args.positions[t];
-    pos_ok = pos >= 0 && pos < args.max_positions;
-    if (args.write_cache && pos_ok) {
-      page = args.block_table[(int64_t)args.token_req[t] * args.table_stride + pos / args.page_size];
-      page_ok = page >= 0 && page < args.num_pages;
-    }
 #pragma unroll
-    for (int j = 0; j < PER_LANE / 2; ++j) {
-      cs[j] = sn[j] = 0.f;
-      if (pos_ok) {
-        cs[j] = args.cos_table[(int64_t)pos * (D / 2) + lane + 32 * j];
-        sn[j] = args.sin_table[(int64_t)pos * (D / 2) + lane + 32 * j];
-      }
+  for (int j = 0; j < J / 2; ++j) {
+    cs[j] = sn[j] = make_float2(0.f, 0.f);
+    if (pos_ok) {
+      cs[j] = *reinterpret_cast<const float2*>(args.cos_table + (int64_t)pos * (D / 2) + 2 * l + 32 * j);
+      sn[j] = *reinterpret_cast<const float2*>(args.sin_table + (int64_t)pos * (D / 2) + 2 * l + 32 * j);
     }
-  };
-  const bool early = gridDim.x <= 512;
-  if (early) look_up();
+  }
   ls_dependency_wait();
-  const uint4* row = reinterpret_cast<const uint4*>(qkv + (int64_t)t * heads_total * D);
-  for (int i = threadIdx.x; i < heads_total * VEC; i += blockDim.x) row_smem[i] = row[i];
-  if (!early) look_up();
   if (threadIdx.x == 0) {
     if (!pos_ok) ls_record_fault(err, LS_DEV_POSITION_RANGE, t);
     else if (args.write_cache && !page_ok) ls_record_fault(err, LS_DEV_PAGE_RANGE, t);
   }
-  __syncthreads();
-  bf16* staged = reinterpret_cast<bf16*>(row_smem);
-  if (pos_ok) {
-    const int normed_heads = args.write_cache && page_ok ? nq + nkv : nq;      // v heads leave as they came
-    for (int head = warp; head < normed_heads; head += 8) {
-      bf16* h = staged + head * D;
-      const float* gain = head < nq ? gq : gk;
-      float v[PER_LANE];
-      float rstd = 1.f;
+  if (!pos_ok) return;                            // a bad position writes nothing
+  const bool caches = args.write_cache && page_ok;
+  const int slot = caches ? pos % args.page_size : 0;
+  const bf16* row = qkv + (int64_t)t * (nq + 2 * nkv) * D;
+  bf16* pages = reinterpret_cast<bf16*>(args.pages) + ((int64_t)page * 2 * nkv * args.page_size + slot) * D;   // k head 0 of the token
+  const int64_t line = (int64_t)args.page_size * D;
+  const int heads = caches ? nq + nkv : nq;       // the heads that are normed and rotated
+  const int steps = (heads + 1) >> 1;
+
+  auto load = [&](int step, __nv_bfloat162* x) {
+    const int head = 2 * step + half;
 #pragma unroll
-      for (int j = 0; j < PER_LANE; ++j) v[j] = __bfloat162float(h[lane + 32 * j]);
-      if (normed) {
-        float ss = 0.f;
+    for (int j = 0; j < J; ++j)
+      if (head < heads) x[j] = *reinterpret_cast<const __nv_bfloat162*>(row + head * D + 2 * l + 32 * j);
+  };
+  __nv_bfloat162 x[J], next[J];
 #pragma unroll
-        for (int j = 0; j < PER_LANE; ++j) ss = fmaf(v[j], v[j], ss);
-        ss = ls_warp_sum(ss);
-        rstd = 1.0f / sqrtf(ss / (float)D + args.eps);
-      }
-#pragma unroll
-      for (int j = 0; j < PER_LANE / 2; ++j) {
-        float lo = __fmul_rn(v[j], rstd);
-        float hi = __fmul_rn(v[j + PER_LANE / 2], rstd);
-        if (normed) {
-          lo = __fmul_rn(lo, gain[j]);
-          hi = __fmul_rn(hi, gain[j + PER_LANE / 2]);
-        }
-        h[lane + 32 * j] = __float2bfloat16_rn(__fsub_rn(__fmul_rn(lo, cs[j]), __fmul_rn(hi, sn[j])));
-        h[lane + 32 * j + D / 2] = __float2bfloat16_rn(__fadd_rn(__fmul_rn(hi, cs[j]), __fmul_rn(lo, sn[j])));
-      }
-    }
+  for (int j = 0; j < J; ++j) next[j] = __nv_bfloat162(__float2bfloat16(0.f), __float2bfloat16(0.f));
+  int step = warp;
+  if (step < steps) load(step, next);
+  // the value heads leave as they came, 16 bytes at a time
+  if (caches) {
+    constexpr int VEC = D / 8;
+    const uint4* v = reinterpret_cast<const uint4*>(row + (nq + nkv) * D);
+    for (int i = threadIdx.x; i < nkv * VEC; i += 128)
+      reinterpret_cast<uint4*>(pages + (nkv + i / VEC) * line)[i % VEC] = v[i];
   }
-  __syncthreads();
-  // out: q heads side by side into q_out's row; k and v heads each to its line of the page
-  const int first = pos_ok ? 0 : nq * VEC;                                  // a bad position writes nothing
-  const int last = args.write_cache && page_ok ? heads_total * VEC : nq * VEC;
-  uint4* q_dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(args.q_out) + (int64_t)t * nq * D);
-  const int slot = args.write_cache && page_ok ? pos % args.page_size : 0;
-  for (int i = first + threadIdx.x; i < last; i += blockDim.x) {
-    const int head = i / VEC, piece = i % VEC;
-    if (head < nq) {
-      q_dst[i] = row_smem[i];
-    } else {
-      const int is_v = head >= nq + nkv ? 1 : 0;
-      const int kvh = head - nq - is_v * nkv;
-      const int64_t line = (((int64_t)page * 2 + is_v) * nkv + kvh) * args.page_size + slot;
-      reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(args.pages) + line * D)[piece] = row_smem[i];
+  for (; step < steps; step += 4) {
+#pragma unroll
+    for (int j = 0; j < J; ++j) x[j] = next[j];
+    if (step + 4 < steps) load(step + 4, next);
+    const int head = 2 * step + half;
+    float2 v[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) v[j] = __bfloat1622float2(x[j]);
+    float rstd = 1.f;
+    if (normed) {
+      float a = 0.f, b = 0.f;
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        a = fmaf(v[j].x, v[j].x, a);
+        b = fmaf(v[j].y, v[j].y, b);
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+      }
+      rstd = 1.0f / sqrtf((a + b) / (float)D + args.eps);
+    }
+    if (head >= heads) continue;
+    const bool is_q = head < nq;
+    bf16* dst = is_q ? reinterpret_cast<bf16*>(args.q_out) + ((int64_t)t * nq + head) * D : pages + (head - nq) * line;
+#pragma unroll
+    for (int j = 0; j < J / 2; ++j) {
+      const float2 g_lo = is_q ? gq[j] : gk[j], g_hi = is_q ? gq[j + J / 2] : gk[j + J / 2];
+      // (a product with a gain of 1 where there is no norm changes no bit)
+      const float lo0 = __fmul_rn(__fmul_rn(v[j].x, rstd), g_lo.x), lo1 = __fmul_rn(__fmul_rn(v[j].y, rstd), g_lo.y);
+      const float hi0 = __fmul_rn(__fmul_rn(v[j + J / 2].x, rstd), g_hi.x);
+      const float hi1 = __fmul_rn(__fmul_rn(v[j + J / 2].y, rstd), g_hi.y);
+      *reinterpret_cast<__nv_bfloat162*>(dst + 2 * l + 32 * j) =
+          __floats2bfloat162_rn(__fsub_rn(__fmul_rn(lo0, cs[j].x), __fmul_rn(hi0, sn[j].x)),
+                                __fsub_rn(__fmul_rn(lo1, cs[j].y), __fmul_rn(hi1, sn[j].y)));
+      *reinterpret_cast<__nv_bfloat162*>(dst + D / 2 + 2 * l + 32 * j) =
+          __floats2bfloat162_rn(__fadd_rn(__fmul_rn(hi0, cs[j].x), __fmul_rn(lo0, sn[j].x)),
+                                __fadd_rn(__fmul_rn(hi1, cs[j].y), __fmul_rn(lo1, sn[j].y)));
     }
   }
 }
@@ -493,12 +501,13 @@ LS_API int ls_qk_norm_rope_store(const void* qkv, void* q_out, void* pages, int 
   args.interleaved = interleaved ? 1 : 0;
   // whole heads of 64 or 128 bfloat16 in the half layout, rows and targets on 16-byte boundaries: the short kernel
   const bool whole = dtype == LS_BF16 && (d == 64 || d == 128) && rot_dim == d && !interleaved && (q_gain == nullptr) == (k_gain == nullptr) &&
-                     (((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)pages) & 15) == 0 && smem <= 48 * 1024;
+                     (((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)pages) & 15) == 0 &&
+                     (((uintptr_t)q_gain | (uintptr_t)k_gain | (uintptr_t)cos_table | (uintptr_t)sin_table) & 7) == 0;
   if (whole) {
     if (d == 64)
-      LS_COUNT(LS_K_QK_NORM_ROPE_WHOLE), ls_launch(qk_norm_rope_store_whole_kernel<64>, grid, 256, smem, stream, (const __nv_bfloat16*)qkv, args, tokens, err);
+      LS_COUNT(LS_K_QK_NORM_ROPE_WHOLE), ls_launch(qk_norm_rope_store_whole_kernel<64>, grid, 128, 0, stream, (const __nv_bfloat16*)qkv, args, tokens, err);
     else
-      LS_COUNT(LS_K_QK_NORM_ROPE_WHOLE), ls_launch(qk_norm_rope_store_whole_kernel<128>, grid, 256, smem, stream, (const __nv_bfloat16*)qkv, args, tokens, err);
+      LS_COUNT(LS_K_QK_NORM_ROPE_WHOLE), ls_launch(qk_norm_rope_store_whole_kernel<128>, grid, 128, 0, stream, (const __nv_bfloat16*)qkv, args, tokens, err);
     return ls_launch_status();
   }
   if (dtype == LS_F32)

@@ -424,3 +424,35 @@ def test_float32_splits_of_single_tokens_have_the_bits_of_the_tile_kernel(nq, nk
     k.raise_on_fault(err)
     assert bool(got[0][2].any()) and torch.equal(got[0][2], got[1][2])
     assert torch.equal(got[0][0][~got[0][2]], got[1][0][~got[0][2]]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("nq,nkv,d,gain,cache", [(16, 8, 128, torch.bfloat16, True), (3, 1, 128, torch.float32, True), (2, 1, 64, torch.bfloat16, True),
+                                                 (7, 7, 64, None, True), (5, 1, 128, torch.bfloat16, False), (200, 8, 128, torch.bfloat16, True)])
+def test_whole_heads_have_the_bits_of_the_general_kernel(nq, nkv, d, gain, cache):
+    """Odd and even numbers of heads, of 64 and 128 elements, with and without gains and cache, against the kernel that takes any
+    alignment (rows that start 8 bytes off)."""
+    k = K()
+    g = torch.Generator().manual_seed(nq + d)
+    tokens, page, num_pages = 37, 16, 5
+    raw = torch.randn(tokens * (nq + 2 * nkv) * d + 8, generator=g).bfloat16().to(dev())
+    gains = [None, None] if gain is None else [(1 + 0.1 * torch.randn(d, generator=g)).to(gain).to(dev()) for _ in range(2)]
+    ang = torch.rand(80, d // 2, generator=g) * 6
+    cos, sin = ang.cos().to(dev()), ang.sin().to(dev())
+    positions = torch.arange(tokens, dtype=torch.int32, device=dev()) + 11
+    table = torch.tensor([[4, 2, 0, 1, 3]], dtype=torch.int32, device=dev())
+    req = torch.zeros(tokens, dtype=torch.int32, device=dev())
+    err, got, names = k.new_error_word(dev()), [], []
+    for off in (0, 4):
+        qkv = torch.empty_like(raw)[off:off + raw.numel() - 8].view(tokens, -1)
+        qkv.copy_(raw[:-8].view(tokens, -1))
+        q = torch.full((tokens, nq * d), 7.0, dtype=torch.bfloat16, device=dev())
+        pages = torch.full((num_pages, 2, nkv, page, d), 7.0, dtype=torch.bfloat16, device=dev())
+        before = k.kernel_counts()
+        k.qk_norm_rope_store(qkv, q, pages, *gains, cos, sin, positions, req, table, nq, nkv, d, d, 1e-6, cache, err)
+        after = k.kernel_counts()
+        names.append([n for n in after if after[n] > before.get(n, 0)])
+        got.append((q, pages))
+    k.raise_on_fault(err)
+    assert names == [["qk_norm_rope_store_whole"], ["qk_norm_rope_store"]]
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert bool((got[0][1] != 7).any()) == cache
