@@ -467,9 +467,14 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_acc,
                                          const float* __restrict__ part_ml, T* __restrict__ out,
                                          const int* __restrict__ items, int nq, int d, int slot_limit,
                                          const float* __restrict__ sinks, int* err) {
-  ls_dependency_sync();
+  ls_dependency_trigger();
+  // (the items are the step's inputs and the sinks weights, older than the kernel before: read before the wait on it, 0.6 us a
+  // layer of a step of one request)
   const int* it = items + (int64_t)blockIdx.x * 4;
   const int tok = it[0], first = it[1], stride = it[2], n = it[3];
+  const int h = blockIdx.y;
+  const float sink = sinks != nullptr ? sinks[h] : -CUDART_INF_F;
+  ls_dependency_wait();
   if (n == 0) return;                        // padding item of a recorded launch
   if (slot_limit > 0) {                      // see attention_decode_kernel
     const long long last = (long long)first + (long long)stride * (n - 1);
@@ -478,9 +483,8 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_acc,
       return;
     }
   }
-  const int h = blockIdx.y;
   for (int c = threadIdx.x; c < d; c += blockDim.x)
-    out[((int64_t)tok * nq + h) * d + c] = ls_from_float<T>(ls_fold_row(part_acc, part_ml, first, stride, n, nq, h, d, c, sinks != nullptr ? sinks[h] : -CUDART_INF_F));
+    out[((int64_t)tok * nq + h) * d + c] = ls_from_float<T>(ls_fold_row(part_acc, part_ml, first, stride, n, nq, h, d, c, sink));
 }
 
 size_t tile_smem_bytes(int d) {
