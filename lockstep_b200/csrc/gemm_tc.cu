@@ -1603,6 +1603,7 @@ int launch_cluster(const CUtensorMap& mw, const CUtensorMap& mx, void* C, int T,
 }
 
 constexpr int MAX_DYNAMIC_SMEM = 227 * 1024;
+constexpr int FEW_SMEM = 140 * 1024;
 
 template <int BN, int EPI, typename TC, bool NORM>
 int launch_few(const CUtensorMap& mw, const CUtensorMap& mx, const NormArgs& norm, const LsQkvStore& heads, void* C,
@@ -1630,9 +1631,13 @@ int launch_few(const CUtensorMap& mw, const CUtensorMap& mx, const NormArgs& nor
   lay.recv_off = lay.x_off + (uint32_t)x_bytes;
   lay.head_off = lay.recv_off + (uint32_t)recv_bytes;
   lay.bars_off = lay.head_off + (uint32_t)head_bytes;
-  // the whole SM is asked for although less is used: a block of this kernel, resident early,
-  // must not take room from the blocks of the kernel before it (measured: slower otherwise)
-  lay.smem = MAX_DYNAMIC_SMEM;
+  // More than half of an SM's shared memory is asked for, whatever is used: two blocks of these kernels never share an SM, so
+  // that those of a launch spread over the device, while blocks of attention, norms and folds fit beside one and start
+  // before it ends.  (Steps of one request / 8 at a context of 1,500 / 16 at 300 / 32 at 60, ms with 24 / 40 / 40 / 40 decoded tokens
+  // and the prompts: what is used 21.59 / 62.7 / 51.5 / 51.4, 113 KB 21.83 / 62.6 / 51.1 / 51.5, 114 to 140 KB 20.60 / 63.3 / 51.2 / 50.7,
+  // the whole SM 20.59 / 64.6 / 52.2 / 51.4.)
+  const int used = (int)lay.bars_off + bars_bytes + 1024;
+  lay.smem = (uint32_t)(used > FEW_SMEM ? used : FEW_SMEM);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((N + BM - 1) / BM, (T + BN - 1) / BN, plan.shares);
   cfg.blockDim = dim3(192);
