@@ -1,29 +1,28 @@
 // Attention of a portion of a prompt over the paged cache on the 5th-generation
 // tensor cores: bfloat16, head sizes 64 and 128.  A block takes 128 query tokens of
 // one request and one query head (a token is a row of the MMA tile, a lane of
-// tensor memory, and a thread of the softmax warps) and walks the keys in
+// tensor memory, and a thread of a softmax team) and walks the keys in
 // ascending tiles of 128, whose edges lie at multiples of 128 keys whatever the
 // portion, so a row's arithmetic depends on its own position only.
 //
 //   S = Q K^T     tcgen05.mma, Q [128 x d] and the key tile [128 x d] K-major in
 //                 shared memory (TMA, 128-byte swizzle), S in tensor memory
-//   softmax       the threads of a row read it from S with tcgen05.ld: maximum,
+//   softmax       a thread reads its row's 128 scores from S with tcgen05.ld: maximum,
 //                 p = exp2(s * scale * log2 e - m_ref), the running sum l in registers; P
-//                 rounded to bfloat16 goes back to tensor memory (tcgen05.st), two keys a column
+//                 rounded to bfloat16 goes back to tensor memory (tcgen05.st), two keys a column,
+//                 over the scores it came from
 //   PV            tcgen05.mma with P [128 x 128] as the A operand in tensor memory and the
 //                 value tile [128 keys x d] as it lies in the cache (MN-major) in shared
 //                 memory, adding to O in tensor memory over all tiles.  m_ref follows the
 //                 row's maximum lazily (when it has grown by more than 8, a factor 256, the
 //                 row of O is scaled and m_ref moved); O / l does not depend on m_ref.
 //
-// Nineteen warps: warp 0 fetches Q once and the key tiles, warp 18 the value tiles, into
-// two stages each (a lane per page of a tile: look-up and TMA box), warp 1 issues the MMAs
-// (S of the next tile before PV of this one, so the tensor cores work while the
-// softmax runs; S and P have two buffers each in tensor memory), warps 2..17 are the
-// softmax, four threads per row: each has 32 keys of a tile and a quarter of the head's
-// dimensions; they share the row's maximum through shared memory.  (With two threads per
-// row the softmax warps, two to a scheduler, were short of issue slots.)  Every wait is bounded; a wait that runs out records
-// LS_DEV_WAIT_TIMEOUT and the block winds down and frees its tensor memory.
+// Twelve warps: warp 0 issues the MMAs, warp 1 fetches Q and the key tiles, warp 2 the value
+// tiles (a lane per page of a tile: look-up and TMA box), warps 4..7 and 8..11 are two softmax
+// teams that take the tiles in turn, a thread a row.  Tensor memory holds three S tiles and O, so
+// S of the two tiles ahead is made while a tile's exponentials are taken.  Every wait is
+// bounded; a wait that runs out records LS_DEV_WAIT_TIMEOUT and the block winds down and frees
+// its tensor memory.
 #include <cuda.h>
 #include <math_constants.h>
 
@@ -34,25 +33,45 @@ namespace {
 
 constexpr int BLOCK_M = 128;              // query tokens per block
 constexpr int BLOCK_N = 128;              // keys per tile
-constexpr int STAGES = 2;
+constexpr int STAGES = 2;                 // of Q, of keys and of values
+constexpr int S_TILES = 3;                // S tiles in tensor memory
 constexpr int UMMA_K = 16;
 constexpr int HALF_BYTES = 128 * 128;     // 128 rows of 64 elements
 constexpr uint32_t TMEM_COLS = 512;
-constexpr int GROUPS = 4;                 // softmax threads per row (warpgroups of the softmax)
-constexpr int THREADS = (3 + 4 * GROUPS) * 32;
-constexpr int V_WARP = 2 + 4 * GROUPS;    // the warp that fetches the value tiles
+constexpr int MMA_WARP = 0, K_WARP = 1, V_WARP = 2, TEAM_WARP = 4;
+constexpr int THREADS = 12 * 32;
 
-// MN-major operand (the value tile as it lies in the cache: a key is a row of 128 bytes = 64
-// elements of d): blocks of 64 elements of d are `block_stride` bytes apart (leading offset),
-// groups of 8 keys 1024 bytes (stride offset); 128-byte swizzle
-__device__ __forceinline__ uint64_t desc_mn_major(uint32_t saddr, uint32_t block_stride) {
+// A key or value tile lies in groups of 8 keys, a group as its halves of 64 elements, a half as 8
+// rows of 128 bytes (128-byte swizzle): what one TMA box of a page leaves (see encode_pages).
+// MN-major operand (the value tile, d the major dimension): halves 1024 bytes apart (leading offset), groups of 8
+// keys HALVES x 1024 (stride offset)
+template <int HALVES>
+__device__ __forceinline__ uint64_t desc_mn_major(uint32_t saddr) {
   uint64_t d = 0;
   d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)((block_stride >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)(1024 >> 4) << 16;
+  d |= (uint64_t)((HALVES * 1024) >> 4) << 32;
   d |= (uint64_t)1 << 46;
   d |= (uint64_t)2 << 61;
   return d;
+}
+// K-major operand whose groups of 8 rows are GROUP_BYTES apart
+template <int GROUP_BYTES>
+__device__ __forceinline__ uint64_t desc_k_major_groups(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(GROUP_BYTES >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int x0, int x1, int x2, int x3,
+                                            uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(dst), "l"(map), "r"(smem_u32(bar)), "r"(x0), "r"(x1), "r"(x2), "r"(x3)
+      : "memory");
 }
 // the same with the A operand in tensor memory (row = lane, two bfloat16 of neighbouring k a column)
 __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc,
@@ -85,21 +104,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
         "r"(taddr)
       : "memory");
-}
-// N columns (a multiple of 16) of this thread's lane to or from registers
-template <int N>
-__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t* r) {
-  static_assert(N % 16 == 0, "columns in sixteens");
-#pragma unroll
-  for (int c = 0; c + 32 <= N; c += 32) tmem_ld32(taddr + c, r + c);
-  if constexpr (N % 32) tmem_ld16(taddr + N - 16, r + N - 16);
-}
-template <int N>
-__device__ __forceinline__ void tmem_st_cols(uint32_t taddr, const uint32_t* r) {
-  static_assert(N % 16 == 0, "columns in sixteens");
-#pragma unroll
-  for (int c = 0; c + 32 <= N; c += 32) tmem_st32(taddr + c, r + c);
-  if constexpr (N % 32) tmem_st16(taddr + N - 16, r + N - 16);
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // 2^x on the special-function unit, one instruction (inputs here are <= 0 or -inf)
@@ -158,15 +162,25 @@ struct Item {
   __device__ __forceinline__ int tile(int it) const { return it < lead ? it : tile_first + it - lead; }
 };
 
-// HALVES = d / 64.  Shared memory: Q [HALVES][128 rows][128 B]; two stages of K and of V
-// [HALVES][128 keys][128 B]; barriers.  Tensor memory: two S buffers, O, two P buffers (bfloat16).
+// HALVES = d / 64.  Shared memory: two stages of Q [HALVES][128 rows][128 B], of K and of V [16 groups][HALVES][8 keys][128 B];
+// barriers; what the teams hand each other.  Tensor memory: three S tiles (P over the S it came from), O.
 //
 // The kernel is persistent: a block per SM walks the items (work item x head, longest context
 // first) in rounds, round r handing item r * blocks + b to block b, and every other round in the
-// reverse order, so that a block with a long item gets a short one next.  Barriers, stages and
-// buffers count on over the items of a block (tile counter `gt`), the producers run ahead into
-// the next item's Q and first tiles while the softmax of the last tile still runs, and the
-// tensor memory is allocated once: an item after the first does not pay a block's start again.
+// reverse order, so that a block with a long item gets a short one next.  Tiles count on over the items of
+// a block (`g`): tile g is team g & 1's, lies in S tile g % 3 and in stage g & 1 of keys and values.  The
+// MMA warp issues S two tiles ahead, into the next item too, whose Q has a stage of its own.
+//
+// What bounds it: MMAs (1,024 cycles a tile of 128 x 128 with d = 128), exponentials (1,024 on the special-function
+// units), shared memory (160 KB a tile at 128 bytes a cycle) and L2 (64 KB a tile an SM) have to run side by side; a tile
+// takes about 1,800 cycles, paced by the arrival of keys and values.  Measured, 16 query and 8 key heads of 128, pages of 16, with a
+// head a block and four threads a row / two heads a block / now: 2,048 tokens 30.0 / - / 25.1 us, 2,048 after
+// 6,144 148.8 / 148.4 / 113.6 us, 8,192 - / 276 / 244 us (1,126 TFLOP/s).
+// Two teams on different tiles, with no chain between a tile's softmax and the next tile's S.  A row's sums need one
+// order: m_ref of a row goes from team to team with the tiles (through shared memory and a named barrier of the two
+// warps that share the row's quarter of tensor memory, before the exponentials are taken), O is one accumulator and each
+// team keeps the sum l of its own tiles, which the team that has the item's last tile adds up.
+//
 // EXTRAS: the scores may get a bias that grows with the logarithm of the distance of key and query taken
 // off (slopes[head] x ln(1 + log_rates[head] x distance): in the units of the exponentials,
 // slopes[head] x lg2(1 + log_rates[head] x distance), one more special-function instruction a score),
@@ -183,32 +197,32 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             const float* __restrict__ log_rates, const float* __restrict__ sinks, float cap_log2, int* err) {
   ls_dependency_trigger();
   constexpr int D = HALVES * 64;
-  constexpr int KV_BYTES = HALVES * HALF_BYTES;          // K (or V) of one tile; also Q
-  // tensor memory: two S buffers, O, and two P buffers (bfloat16, two keys a column)
-  constexpr uint32_t S_COL = 0, O_COL = 2 * BLOCK_N, P_COL = O_COL + 128, P_COLS = BLOCK_N / 2;
+  constexpr int TILE_BYTES = HALVES * HALF_BYTES;        // K or V of one tile; also Q of one item
+  constexpr int GROUP_BYTES = HALVES * 1024;             // 8 keys of a tile
+  constexpr uint32_t O_COL = S_TILES * BLOCK_N;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t q_smem = base;
-  const uint32_t k_smem = q_smem + KV_BYTES;             // [STAGES]
-  const uint32_t v_smem = k_smem + STAGES * KV_BYTES;    // [STAGES]
-  const uint32_t bars_smem = v_smem + STAGES * KV_BYTES;
-  uint8_t* v_ptr = aligned + (v_smem - base);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(aligned + (bars_smem - base));
-  uint64_t* q_full = bars;             // Q of an item landed
-  uint64_t* k_full = bars + 1;         // [2] keys of a tile landed
-  uint64_t* v_full = bars + 3;         // [2] values landed
-  // (a key stage is free when the S product that read it is done, which is what s_full says; a
-  // value stage when its PV product is done: o_full.  The producers wait on those: a commit of
-  // its own for each cost the issuing warp ≈ 125 cycles a tile)
-  uint64_t* s_full = bars + 9;         // [2] S of a tile is in tensor memory
-  uint64_t* q_free = bars + 13;        // the item's last S product has read Q
-  uint64_t* o_full = bars + 14;        // [2] PV of a tile has been added to O (and its P may be overwritten)
-  uint64_t* p_full = bars + 16;        // [2] P of a tile is in tensor memory
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
+  const uint32_t q_smem = base;                          // [STAGES]
+  const uint32_t k_smem = q_smem + STAGES * TILE_BYTES;  // [STAGES]
+  const uint32_t v_smem = k_smem + STAGES * TILE_BYTES;  // [STAGES]
+  uint8_t* v_ptr = aligned + 2 * STAGES * TILE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(aligned + 3 * STAGES * TILE_BYTES);
+  uint64_t* q_full = bars;             // [2] Q of an item landed
+  uint64_t* q_free = bars + 2;         // [2] the item's last S product has read Q
+  uint64_t* k_full = bars + 4;         // [2] keys of a tile landed
+  uint64_t* v_full = bars + 6;         // [2] values landed
+  uint64_t* k_free = bars + 8;         // [2] the S product has read the keys
+  uint64_t* s_full = bars + 10;        // [3] S of a tile is in tensor memory
+  uint64_t* p_full = bars + 13;        // [3] P of a tile is in tensor memory
+  uint64_t* o_full = bars + 16;        // [2] PV of a tile has been added to O (and has read its values)
+  uint64_t* o_free = bars + 18;        // the item's O has been read
+  uint64_t* l_full = bars + 19;        // [4] the sums of the team without the item's last tile
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 23);
   volatile uint32_t* failed = tmem_slot + 1;
-  float* row_max = reinterpret_cast<float*>(bars + 32);   // [2 tiles][GROUPS][128 rows], then [GROUPS][128] for l
+  float* hand_m = reinterpret_cast<float*>(bars + 32);   // [2 teams][128 rows] m_ref after a team's tile
+  float* hand_l = hand_m + 2 * 128;                      // [4][128 rows] sums handed over at an item's end
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int total_items = n_work * nq;
@@ -254,26 +268,30 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   // one: the first item's first look-up runs under the set-up below
   Item first_item;
   int first_page = 0;
-  const bool producer = warp == 0 || warp == V_WARP;
+  const bool producer = warp == K_WARP || warp == V_WARP;
   if (producer && get_item(0, first_item) == 1) first_page = lookup(first_item, 0);
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    mbar_init(q_free, 1);
     for (int s = 0; s < 2; ++s) {
+      mbar_init(&q_full[s], 1);
+      mbar_init(&q_free[s], 1);
       mbar_init(&k_full[s], 1);
       mbar_init(&v_full[s], 1);
-      mbar_init(&s_full[s], 1);
+      mbar_init(&k_free[s], 1);
       mbar_init(&o_full[s], 1);
     }
-    mbar_init(&p_full[0], 4 * GROUPS);
-    mbar_init(&p_full[1], 4 * GROUPS);
+    for (int s = 0; s < S_TILES; ++s) {
+      mbar_init(&s_full[s], 1);
+      mbar_init(&p_full[s], 4);
+    }
+    for (int s = 0; s < 4; ++s) mbar_init(&l_full[s], 4);
+    mbar_init(o_free, 4);
     *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_kv) : "memory");
   }
-  if (warp == 2) {
+  if (warp == TEAM_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(TMEM_COLS)
                  : "memory");
@@ -285,138 +303,13 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   const uint32_t tmem_base = *tmem_slot;
   ls_dependency_wait();                 // q and this step's keys and values come from the kernel before
 
-  if (producer) {
-    // ---- producers: warp 0 fetches Q and the key tiles, warp V_WARP the value tiles: a key stage
-    // is free two tiles before the value stage of the same tile, and neither waits for the other's ----
-    const bool keys = warp == 0;
-    uint64_t* free_bar = keys ? s_full : o_full;
-    uint64_t* full_bar = keys ? k_full : v_full;
-    const uint32_t dst_base = keys ? k_smem : v_smem;
-    int gt = 0, j = 0;                  // tiles and items of this block so far
-    bool ok = true;
-    for (int round = 0; ok; ++round) {
-      Item I;
-      const int kind = get_item(round, I);
-      if (kind == 0) break;
-      if (kind == 2) continue;
-      int page = round == 0 ? first_page : lookup(I, 0);
-      if (keys && lane == 0) {
-        // Q is free once the last S product of the item before has read it
-        if (j > 0 && (*failed || !mbar_wait(q_free, (uint32_t)(j - 1) & 1u))) {
-          *failed = 1;
-          ls_record_fault(err, LS_DEV_WAIT_TIMEOUT, 810);
-        } else {
-          mbar_expect_tx(q_full, KV_BYTES);
-#pragma unroll
-          for (int hh = 0; hh < HALVES; ++hh)
-            tma_load_2d(q_smem + hh * HALF_BYTES, &map_q, I.h * D + hh * 64, I.tok0, q_full);
-        }
-      }
-      for (int it = 0; it < I.n_tiles; ++it) {
-        const int g = gt + it;
-        const int s = g & 1;
-        const uint32_t phase = (uint32_t)(g >> 1) & 1u;
-        const int c0 = I.tile(it) * BLOCK_N;
-        ok = *failed == 0 && mbar_wait(&free_bar[s], phase ^ 1u);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) {
-          *failed = 1;
-          if (lane == 0) ls_record_fault(err, LS_DEV_WAIT_TIMEOUT, 800 + s);
-          break;
-        }
-        if (lane == 0) mbar_expect_tx(&full_bar[s], KV_BYTES);
-        __syncwarp();
-        if (lane < boxes) {
-          if (page < 0 || page >= num_pages) {
-            ls_record_fault(err, LS_DEV_PAGE_RANGE, c0 + lane * rows_per_box);
-            page = 0;
-          }
-          const int in_page = ((c0 + lane * rows_per_box) % page_size) / rows_per_box * rows_per_box;
-          const int y = ((page * 2 + (keys ? 0 : 1)) * nkv + I.kvh) * page_size + in_page;
-#pragma unroll
-          for (int hh = 0; hh < HALVES; ++hh)
-            tma_load_2d(dst_base + (uint32_t)(s * KV_BYTES + hh * HALF_BYTES + lane * rows_per_box * 128), &map_kv,
-                        hh * 64, y, &full_bar[s]);
-        }
-        page = lookup(I, it + 1);       // after this tile's loads have gone out
-      }
-      gt += I.n_tiles;
-      ++j;
-    }
-  } else if (warp == 1) {
-    // ---- MMA issue: the whole warp walks the loop and one elected lane issues, so that the
-    // instructions' operands are the same in every lane and stay in uniform registers (inside a
-    // branch of one lane every MMA paid for moving them there) ----
-    constexpr uint32_t idesc_s = instr_desc(BLOCK_M, BLOCK_N, false);
-    constexpr uint32_t idesc_o = instr_desc(BLOCK_M, D, true);
-    const bool issuer = elect_one();
-    int gt = 0, j = 0;
-    bool ok = true;
-    for (int round = 0; ok; ++round) {
-      Item I;
-      const int kind = get_item(round, I);
-      if (kind == 0) break;
-      if (kind == 2) continue;
-      ok = __all_sync(0xffffffffu, mbar_wait(q_full, (uint32_t)j & 1u));
-      auto issue_s = [&](int it) {       // S(it) = Q K(it)^T into the S buffer in turn
-        const int g = gt + it;
-        const int s = g & 1;
-        const uint32_t phase = (uint32_t)(g >> 1) & 1u;
-        // (the S buffer is free: the softmax warps had read tile g - 2 before they announced its P,
-        // which this warp waited for before the PV product of that tile)
-        if (!__all_sync(0xffffffffu, mbar_wait(&k_full[s], phase))) return false;
-        fence_after_sync();
-        if (issuer) {
-#pragma unroll
-          for (int k = 0; k < D / UMMA_K; ++k) {
-            const uint32_t koff = (uint32_t)((k >> 2) * HALF_BYTES + (k & 3) * UMMA_K * 2);
-            umma(tmem_base + S_COL + s * BLOCK_N, desc_k_major(q_smem + koff),
-                 desc_k_major(k_smem + s * KV_BYTES + koff), idesc_s, k != 0 ? 1u : 0u);
-          }
-          umma_commit(&s_full[s]);
-          if (it == I.n_tiles - 1) umma_commit(q_free);     // the item's last product with this Q
-        }
-        __syncwarp();
-        return true;
-      };
-      if (ok) ok = issue_s(0);
-      for (int it = 0; it < I.n_tiles && ok; ++it) {
-        const int g = gt + it;
-        const int s = g & 1;
-        const uint32_t phase = (uint32_t)(g >> 1) & 1u;
-        if (it + 1 < I.n_tiles) ok = issue_s(it + 1);
-        if (!ok) break;
-        ok = __all_sync(0xffffffffu, mbar_wait(&p_full[s], phase) && mbar_wait(&v_full[s], phase));
-        if (!ok) break;
-        fence_after_sync();
-        if (issuer) {
-#pragma unroll
-          for (int k = 0; k < BLOCK_N / UMMA_K; ++k) {
-            // P from tensor memory: 16 keys are 8 columns; V: 16 keys are 16 rows of 128 bytes
-            const uint64_t b = desc_mn_major(v_smem + s * KV_BYTES + k * UMMA_K * 128, HALF_BYTES);
-            umma_ts(tmem_base + O_COL, tmem_base + P_COL + s * P_COLS + k * (UMMA_K / 2), b, idesc_o,
-                    (it | k) != 0 ? 1u : 0u);
-          }
-          umma_commit(&o_full[s]);
-        }
-        __syncwarp();
-      }
-      gt += I.n_tiles;
-      ++j;
-    }
-    if (!ok) {
-      *failed = 1;
-      if (issuer) ls_record_fault(err, LS_DEV_WAIT_TIMEOUT, 820);
-    }
-  } else if (warp < V_WARP) {
-    // ---- softmax: GROUPS threads per row (a token, lane `row` of tensor memory): the thread of
-    // group g (warps 2 + 4 g .. 5 + 4 g) has keys 32 g .. 32 g + 31 of a tile and the g-th
-    // quarter of the head's dimensions ----
-    constexpr int HC = BLOCK_N / GROUPS;          // keys of a tile per thread
-    constexpr int HD = D / GROUPS;                // output dimensions per thread
-    constexpr int ROWS = 128 * GROUPS;            // threads of the softmax
+  if (warp >= TEAM_WARP) {
+    // ---- softmax: team 0 (warps 4..7) has the even tiles of the block, team 1 the odd ones; a
+    // thread a row (a token, lane `row` of tensor memory), whose 128 scores lie in registers: the teams take
+    // what the other warpgroup leaves of the block's 3 x 168 registers a thread ----
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    const int team = (warp - TEAM_WARP) >> 2;
     const int quad = warp & 3;
-    const int group = (warp - 2) >> 2;
     const int row = quad * 32 + lane;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
     // O = sum of P V stays in tensor memory, the MMAs of every tile adding to it, in units of
@@ -426,10 +319,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // The quotient O / l does not depend on m_ref.
     constexpr float LAZY = 8.f;
     bool ok = true;
-    int gt = 0;
+    int gt = 0, shared_items = 0;                 // tiles, and items of two or more tiles so far
+    int s_tile = 0;                               // gt % 3
+    uint32_t s_phase = 0;                         // (gt / 3) & 1
 
     // A wait that runs out clears `ok`; the loops still run to their ends, skipping the work, so
-    // that every thread meets the named barrier of every tile of every item.
+    // that every thread meets the named barriers of every tile of every item.
     for (int round = 0;; ++round) {
       Item I;
       const int kind = get_item(round, I);
@@ -439,7 +334,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       const int pos = pos0 + row;
       const int lo = ls_first_key(pos, window);
       const int lo_last = ls_first_key(pos_last, window);
-      float m_ref = -CUDART_INF_F, l_run = 0.f;
+      // m_ref: the row's, as this team knows it; l_run: the sum over this team's tiles, in its units;
+      // m_before: m_ref before the item's last tile, in whose units the other team hands its sum over
+      float m_ref = -CUDART_INF_F, l_run = 0.f, m_before = -CUDART_INF_F;
       float bias_a = 0.f, bias_b = 0.f;
       bool biased = false, linear = false;
       if constexpr (EXTRAS) {
@@ -447,643 +344,408 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           bias_a = slopes[I.h];
           bias_b = log_rates[I.h];
           biased = true;
-        } else if (slopes != nullptr || cap_log2 > 0.f) {
+        } else if (slopes != nullptr || cap_log2 > 0.f || !(scale_log2 > 0.f)) {
           bias_a = slopes != nullptr ? slopes[I.h] * 1.4426950408889634f : 0.f;      // the slope in the exponentials' units
           bias_b = cap_log2 > 0.f ? scale_log2 / cap_log2 : 0.f;                     // score -> score x scale / cap
           biased = linear = true;
         }
       }
+      // (a scale that is not above 0 too, since -inf times it is not what a masked score is to be;)
       // with a bias the scores are put into the exponentials' units as they are read, and no scale is left
       const float scale_eff = biased ? 1.0f : scale_log2;
       for (int it = 0; it < n_tiles; ++it) {
         const int g = gt + it;
-        const int s = g & 1;
-        const int t0 = I.tile(it) * BLOCK_N;                         // first key of the tile
-        const int c0 = t0 + group * HC;                              // first key of this thread
-        if (ok && !mbar_wait(&s_full[s], (uint32_t)(g >> 1) & 1u)) ok = false;
+        const uint32_t s_addr = lane_base + (uint32_t)(s_tile * BLOCK_N);
+        uint64_t* s_bar = &s_full[s_tile];
+        uint64_t* p_bar = &p_full[s_tile];
+        const uint32_t s_par = s_phase;
+        if (++s_tile == S_TILES) {
+          s_tile = 0;
+          s_phase ^= 1u;
+        }
+        if ((g & 1) != team) continue;
+        const int c0 = I.tile(it) * BLOCK_N;                         // first key of the tile
+        if (ok && !mbar_wait(s_bar, s_par)) ok = false;
         fence_after_sync();
-        // this thread's scores into registers; the buffer is free once all have theirs
-        uint32_t sc[HC];
+        uint32_t sc[BLOCK_N];
 #pragma unroll
-        for (int q0 = 0; q0 < HC; q0 += 32) tmem_ld32(lane_base + S_COL + s * BLOCK_N + group * HC + q0, sc + q0);
+        for (int q0 = 0; q0 < BLOCK_N; q0 += 32) tmem_ld32(s_addr + q0, sc + q0);
         tmem_ld_wait();
         if constexpr (EXTRAS) {
           if (biased && linear) {
             const float d0 = (float)(pos - c0);
             const bool capped = cap_log2 > 0.f;
 #pragma unroll
-            for (int jj = 0; jj < HC; ++jj) {
+            for (int jj = 0; jj < BLOCK_N; ++jj) {
               const float dist = fmaxf(d0 - (float)jj, 0.f);
               const float raw = __uint_as_float(sc[jj]);
               const float v = capped ? cap_log2 * tanh_of(raw * bias_b) : raw * scale_log2;
               sc[jj] = __float_as_uint(fmaf(-bias_a, dist, v));
             }
           } else if (biased) {
-            const float d0 = (float)(pos - c0);        // distance of this thread's first key (masked keys: clamped)
+            const float d0 = (float)(pos - c0);        // distance of the tile's first key (masked keys: clamped)
 #pragma unroll
-            for (int jj = 0; jj < HC; ++jj) {
+            for (int jj = 0; jj < BLOCK_N; ++jj) {
               const float dist = fmaxf(d0 - (float)jj, 0.f);
               sc[jj] = __float_as_uint(fmaf(__uint_as_float(sc[jj]), scale_log2, -bias_a * lg2(fmaf(bias_b, dist, 1.0f))));
             }
           }
         }
-        // every key of the tile is seen by every row: no masks (uniform over the block)
-        const bool full_tile = t0 + BLOCK_N - 1 <= pos0 && (t0 >= lo_last || t0 + BLOCK_N <= kept);
-        float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-        if (full_tile) {
+        // every key of the tile is seen by every row: no masks (uniform over the block); elsewhere a masked score
+        // becomes -inf (selects and not branches), whose exponential is 0
+        const bool full_tile = c0 + BLOCK_N - 1 <= pos0 && (c0 >= lo_last || c0 + BLOCK_N <= kept);
+        if (!full_tile) {
+          // (a key's place is kept where place - first < count, as unsigned numbers)
+          const int first = lo - c0 > 0 ? lo - c0 : 0;
+          const uint32_t count = pos - c0 - first + 1 > 0 ? (uint32_t)(pos - c0 - first + 1) : 0u;
+          if (c0 >= lo_last) {                                       // no window within the tile: the diagonal alone
 #pragma unroll
-          for (int jj = 0; jj < HC; jj += 2)
-            mx[(jj >> 1) & 3] = max3(mx[(jj >> 1) & 3], __uint_as_float(sc[jj]), __uint_as_float(sc[jj + 1]));
-        } else {
-          // selects, not branches: a masked score counts as -inf
+            for (int jj = 0; jj < BLOCK_N; ++jj) sc[jj] = jj <= pos - c0 ? sc[jj] : __float_as_uint(-CUDART_INF_F);
+          } else {
+            const int lead = EXTRAS ? min(kept - c0, pos - c0 + 1) : 0;
 #pragma unroll
-          for (int jj = 0; jj < HC; ++jj) {
-            const bool keep = (c0 + jj <= pos) & ((c0 + jj >= lo) | (EXTRAS && c0 + jj < kept));
-            mx[jj & 3] = fmaxf(mx[jj & 3], keep ? __uint_as_float(sc[jj]) : -CUDART_INF_F);
+            for (int jj = 0; jj < BLOCK_N; ++jj) {
+              const bool seen = (uint32_t)(jj - first) < count || (EXTRAS && jj < lead);
+              sc[jj] = seen ? sc[jj] : __float_as_uint(-CUDART_INF_F);
+            }
           }
         }
-        // the row's maximum is that of its threads
-        float tile_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-        row_max[(it & 1) * ROWS + group * 128 + row] = tile_max;
-        asm volatile("bar.sync 1, %0;" ::"n"(ROWS) : "memory");
+        float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
 #pragma unroll
-        for (int o = 0; o < GROUPS; ++o) tile_max = fmaxf(tile_max, row_max[(it & 1) * ROWS + o * 128 + row]);
-        // all threads of a row work out the same m_ref from the same numbers
+        for (int jj = 0; jj < BLOCK_N; jj += 2)
+          mx[(jj >> 1) & 3] = max3(mx[(jj >> 1) & 3], __uint_as_float(sc[jj]), __uint_as_float(sc[jj + 1]));
+        const float tile_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        // m_ref after the tile before, from the other team (an item's first tile meets it too, for the
+        // barrier's sake: a team may not announce two tiles before the other has taken the first)
+        if (g > 0) asm volatile("bar.sync %0, 64;" ::"r"(1 + quad * 2 + ((g - 1) & 1)) : "memory");
+        if (it > 0) {
+          const float m_prev = hand_m[((g - 1) & 1) * 128 + row];
+          // (m_ref is -inf before the first key a row sees; l_run is 0 then)
+          if (m_prev != m_ref) l_run *= m_ref == -CUDART_INF_F ? 0.f : ex2(m_ref - m_prev);
+          m_ref = m_prev;
+        }
+        m_before = m_ref;
         const float m_new = tile_max * scale_eff;
         const bool move = m_new > m_ref + LAZY;                      // true too for the first key a row sees
         const float factor = move ? ((m_ref == -CUDART_INF_F) ? 0.f : ex2(m_ref - m_new)) : 1.f;
         if (move) m_ref = m_new;
-        // this tile's P buffer was read by the PV of two tiles ago (long done); O is scaled only
-        // after the PV of the tile before has been added to it
-        if (ok && g > 1 && !mbar_wait(&o_full[s], (uint32_t)((g - 2) >> 1) & 1u)) ok = false;
+        hand_m[(g & 1) * 128 + row] = m_ref;
+        asm volatile("bar.arrive %0, 64;" ::"r"(1 + quad * 2 + (g & 1)) : "memory");
+        // O is scaled only after the PV of the tile before has been added to it (and before this
+        // tile's P is announced, so before the PV of this tile)
         if (it > 0 && __any_sync(0xffffffffu, move)) {
           if (ok && !mbar_wait(&o_full[(g - 1) & 1], (uint32_t)((g - 1) >> 1) & 1u)) ok = false;
           if (__all_sync(0xffffffffu, ok)) {
             fence_after_sync();
-            uint32_t og[HD];
-            tmem_ld_cols<HD>(lane_base + O_COL + group * HD, og);
-            tmem_ld_wait();
 #pragma unroll
-            for (int c = 0; c < HD; ++c) og[c] = __float_as_uint(__uint_as_float(og[c]) * factor);
-            tmem_st_cols<HD>(lane_base + O_COL + group * HD, og);
-          }
-        }
-        // p = exp2(s * scale - m_ref), rounded to bfloat16, two keys a column, into this thread's
-        // columns of the tile's P buffer in tensor memory, from where the PV product takes it as
-        // its A operand; the sum in four running sums, folded in a fixed order
-        float ps[4] = {0.f, 0.f, 0.f, 0.f};
-        const bool dead = m_ref == -CUDART_INF_F;          // nothing seen yet by this row
-        const float neg_m = dead ? 0.f : -m_ref;
-        uint32_t pk[HC / 2];
-        {
-          const bool plain = full_tile & !dead;             // uniform over the block but for `dead`
-#pragma unroll
-          for (int n0 = 0; n0 < HC; n0 += 8) {
-            float p[8];
-            if (plain) {
-#pragma unroll
-              for (int jj = 0; jj < 8; jj += 2) {
-                p[jj] = __uint_as_float(sc[n0 + jj]);
-                p[jj + 1] = __uint_as_float(sc[n0 + jj + 1]);
-                fma2(p[jj], p[jj + 1], scale_eff, neg_m);
-                p[jj] = ex2(p[jj]);
-                p[jj + 1] = ex2(p[jj + 1]);
-              }
-            } else {
-              // every exponential is taken, masked ones of -inf (which is 0): selects, not branches
-#pragma unroll
-              for (int jj = 0; jj < 8; ++jj) {
-                const int key = c0 + n0 + jj;
-                const bool keep = (key <= pos) & ((key >= lo) | (EXTRAS && key < kept)) & !dead;
-                p[jj] = ex2(keep ? fmaf(__uint_as_float(sc[n0 + jj]), scale_eff, neg_m) : -CUDART_INF_F);
-              }
-            }
-            add2(ps[0], ps[1], p[0], p[1]);
-            add2(ps[2], ps[3], p[2], p[3]);
-            add2(ps[0], ps[1], p[4], p[5]);
-            add2(ps[2], ps[3], p[6], p[7]);
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) pk[(n0 >> 1) + jj] = pack_bf16(p[2 * jj], p[2 * jj + 1]);
-          }
-        }
-        tmem_st_cols<HC / 2>(lane_base + P_COL + s * P_COLS + group * (HC / 2), pk);
-        const float psum = (ps[0] + ps[1]) + (ps[2] + ps[3]);
-        // value rows of keys past the last position were never written: they must not be NaN,
-        // since P is zero there and the MMA multiplies all the same
-        if (t0 + BLOCK_N - 1 > pos_last) {
-          if (ok && !mbar_wait(&v_full[s], (uint32_t)(g >> 1) & 1u)) ok = false;
-          if (ok && group < HALVES && t0 + row > pos_last) {
-            uint4* vrow = reinterpret_cast<uint4*>(v_ptr + s * KV_BYTES + group * HALF_BYTES + row * 128);
-#pragma unroll
-            for (int q8 = 0; q8 < 8; ++q8) vrow[q8] = make_uint4(0u, 0u, 0u, 0u);
-          }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        }
-        tmem_st_wait();
-        fence_before_sync();
-        __syncwarp();
-        if (lane == 0 && ok) mbar_arrive(&p_full[s]);
-        l_run = fmaf(l_run, factor, psum);
-      }
-      // the row's sum is that of its threads (a region of its own: the next item's first tile
-      // writes its maxima while a slow thread may still read these)
-      float* l_part = row_max + 2 * ROWS;
-      l_part[group * 128 + row] = l_run;
-      asm volatile("bar.sync 1, %0;" ::"n"(ROWS) : "memory");
-      float l_row = l_part[row];                     // the same sum in the same order in each of the row's threads
-#pragma unroll
-      for (int o = 1; o < GROUPS; ++o) l_row += l_part[o * 128 + row];
-      if constexpr (EXTRAS) {
-        // the sink, in the units of this row's sums (2^m_ref): every thread of the row adds the same
-        if (sinks != nullptr && m_ref != -CUDART_INF_F) l_row += ex2(fmaf(sinks[I.h], 1.4426950408889634f, -m_ref));
-      }
-      const int g_last = gt + n_tiles - 1;
-      if (ok && !mbar_wait(&o_full[g_last & 1], (uint32_t)(g_last >> 1) & 1u)) ok = false;
-      if (ok) {
-        fence_after_sync();
-        uint32_t og[HD];
-        tmem_ld_cols<HD>(lane_base + O_COL + group * HD, og);
-        tmem_ld_wait();
-        fence_before_sync();                         // the next item's first PV overwrites O after its P
-        if (row < I.ntok) {
-          const float inv = l_row > 0.f ? 1.0f / l_row : 0.f;
-          __nv_bfloat16* dst = out + ((int64_t)(I.tok0 + row) * nq + I.h) * D + group * HD;
-#pragma unroll
-          for (int c = 0; c < HD; c += 8) {
-            uint4 v;
-            v.x = pack_bf16(__uint_as_float(og[c]) * inv, __uint_as_float(og[c + 1]) * inv);
-            v.y = pack_bf16(__uint_as_float(og[c + 2]) * inv, __uint_as_float(og[c + 3]) * inv);
-            v.z = pack_bf16(__uint_as_float(og[c + 4]) * inv, __uint_as_float(og[c + 5]) * inv);
-            v.w = pack_bf16(__uint_as_float(og[c + 6]) * inv, __uint_as_float(og[c + 7]) * inv);
-            *reinterpret_cast<uint4*>(dst + c) = v;
-          }
-        }
-      }
-      // (the bar.sync of the next item's first tile, or of its sums, comes before any thread
-      // writes this region again)
-      gt += n_tiles;
-    }
-    if (!ok) {
-      *failed = 1;
-      if (lane == 0) ls_record_fault(err, LS_DEV_WAIT_TIMEOUT, 840 + quad);
-    }
-  }
-  fence_before_sync();
-  __syncthreads();
-  if (warp == 2) {
-    fence_after_sync();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS)
-                 : "memory");
-  }
-}
-
-
-// ---------------------------------------------------------------------------
-// Two query heads of one key head in a block (group sizes that are even).  The two heads'
-// tiles Q_A and Q_B (the same 128 tokens) share every key and value tile, which is loaded
-// once, and each has a team of eight softmax warps (two threads a row, 64 keys each, read
-// from tensor memory in pieces of 32).  Tensor memory: S_A, S_B, O_A, O_B, 128 columns each;
-// P (bfloat16, two keys a column) is written over the S it came from, keys 0..63 into the
-// first 32 columns and keys 64..127 into columns 64..95, so that a thread only writes over
-// scores it has already taken.  The MMAs of one team run while the other team's softmax
-// does: S_A, S_B | PV_A, S_A', PV_B, S_B' | ... in this order on the tensor pipe, which
-// executes them as issued, so PV_X has read P_X before the next S_X overwrites it.
-// A row's arithmetic is that of the kernel above with two threads a row; it depends on the
-// row's own position only.
-// ---------------------------------------------------------------------------
-constexpr int PAIR_THREADS = 19 * 32;
-constexpr int PAIR_V_WARP = 18;
-
-template <int HALVES>
-__global__ void __launch_bounds__(PAIR_THREADS, 1)
-attention_prefill_tc_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
-                                 __nv_bfloat16* __restrict__ out, const int* __restrict__ work, int n_work,
-                                 const int* __restrict__ block_table, int table_stride, int nq, int nkv, int page_size,
-                                 int num_pages, int window, float scale_log2, int* err) {
-  ls_dependency_trigger();
-  constexpr int D = HALVES * 64;
-  constexpr int KV_BYTES = HALVES * HALF_BYTES;          // K (or V) of one tile; also one head's Q
-  constexpr uint32_t S_COL = 0, O_COL = 2 * BLOCK_N;     // S_X at S_COL + 128 X, O_X at O_COL + 128 X
-
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t q_smem = base;                          // [2 heads]
-  const uint32_t k_smem = q_smem + 2 * KV_BYTES;         // [STAGES]
-  const uint32_t v_smem = k_smem + STAGES * KV_BYTES;    // [STAGES]
-  const uint32_t bars_smem = v_smem + STAGES * KV_BYTES;
-  uint8_t* v_ptr = aligned + (v_smem - base);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(aligned + (bars_smem - base));
-  uint64_t* q_full = bars;             // both heads' Q of an item landed
-  uint64_t* k_full = bars + 1;         // [2] keys of a tile landed
-  uint64_t* v_full = bars + 3;         // [2] values landed
-  uint64_t* k_free = bars + 5;         // [2] both S products have read the stage
-  uint64_t* v_free = bars + 7;         // [2] both PV products have read the stage
-  uint64_t* s_full = bars + 9;         // [2 teams] S of a tile is in tensor memory
-  uint64_t* p_full = bars + 11;        // [2 teams] P of a tile is in tensor memory
-  uint64_t* o_full = bars + 13;        // [2 teams] PV of a tile has been added to O
-  uint64_t* q_free = bars + 15;        // the item's last S product has read Q
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
-  volatile uint32_t* failed = tmem_slot + 1;
-  float* team_mem = reinterpret_cast<float*>(bars + 32);   // per team: maxima [2][2][128], then sums [4][128]
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pairs = nq >> 1;
-  const int total_items = n_work * pairs;
-  const int blocks = (int)gridDim.x;
-
-  // the item of this block in round `round`: 0 none is left, 1 an item, 2 a padding item (nothing to do);
-  // I.h is the first head of the pair
-  auto get_item = [&](int round, Item& I) -> int {
-    const int idx = round * blocks + ((round & 1) ? blocks - 1 - (int)blockIdx.x : (int)blockIdx.x);
-    if (idx >= total_items) return 0;
-    const int wi = idx / pairs;
-    I.h = 2 * (idx - wi * pairs);
-    const int* w = work + (int64_t)wi * 8;
-    I.tok0 = w[1];
-    I.ntok = w[2];
-    I.pos0 = w[3];
-    if (I.ntok == 0) return 2;
-    I.table_row = block_table + (int64_t)w[0] * table_stride;
-    I.kvh = I.h / (nq / nkv);
-    I.pos_last = I.pos0 + I.ntok - 1;
-    I.key_lo = ls_first_key(I.pos0, window);
-    I.tile_first = I.key_lo / BLOCK_N;
-    I.n_tiles = I.pos_last / BLOCK_N + 1 - I.tile_first;
-    return 1;
-  };
-
-  const int rows_per_box = page_size < BLOCK_N ? page_size : BLOCK_N;
-  const int boxes = BLOCK_N / rows_per_box;
-  auto lookup = [&](const Item& I, int it) {
-    int page = 0;
-    if (it < I.n_tiles && lane < boxes) {
-      int key = (I.tile_first + it) * BLOCK_N + lane * rows_per_box;
-      if (key > I.pos_last) key = I.pos_last;
-      if (key < I.key_lo) key = I.key_lo;
-      page = I.table_row[key / page_size];
-    }
-    return page;
-  };
-  Item first_item;
-  int first_page = 0;
-  const bool producer = warp == 0 || warp == PAIR_V_WARP;
-  if (producer && get_item(0, first_item) == 1) first_page = lookup(first_item, 0);
-
-  if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    mbar_init(q_free, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&k_full[s], 1);
-      mbar_init(&v_full[s], 1);
-      mbar_init(&k_free[s], 1);
-      mbar_init(&v_free[s], 1);
-      mbar_init(&s_full[s], 1);
-      mbar_init(&p_full[s], 8);
-      mbar_init(&o_full[s], 1);
-    }
-    *failed = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_kv) : "memory");
-  }
-  if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  fence_before_sync();
-  __syncthreads();
-  fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
-  ls_dependency_wait();
-
-  if (producer) {
-    // ---- producers: warp 0 fetches both heads' Q and the key tiles, warp PAIR_V_WARP the value tiles ----
-    const bool keys = warp == 0;
-    uint64_t* free_bar = keys ? k_free : v_free;
-    uint64_t* full_bar = keys ? k_full : v_full;
-    const uint32_t dst_base = keys ? k_smem : v_smem;
-    int gt = 0, j = 0;
-    bool ok = true;
-    for (int round = 0; ok; ++round) {
-      Item I;
-      const int kind = get_item(round, I);
-      if (kind == 0) break;
-      if (kind == 2) continue;
-      int page = round == 0 ? first_page : lookup(I, 0);
-      if (keys && lane == 0) {
-        if (j > 0 && (*failed || !mbar_wait(q_free, (uint32_t)(j - 1) & 1u))) {
-          *failed = 1;
-          ls_record_fault(err, LS_DEV_WAIT_TIMEOUT, 910);
-        } else {
-          mbar_expect_tx(q_full, 2 * KV_BYTES);
-#pragma unroll
-          for (int x = 0; x < 2; ++x)
-#pragma unroll
-            for (int hh = 0; hh < HALVES; ++hh)
-              tma_load_2d(q_smem + x * KV_BYTES + hh * HALF_BYTES, &map_q, (I.h + x) * D + hh * 64, I.tok0, q_full);
-        }
-      }
-      for (int it = 0; it < I.n_tiles; ++it) {
-        const int g = gt + it;
-        const int s = g & 1;
-        const uint32_t phase = (uint32_t)(g >> 1) & 1u;
-        const int c0 = (I.tile_first + it) * BLOCK_N;
-        ok = *failed == 0 && mbar_wait(&free_bar[s], phase ^ 1u);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) {
-          *failed = 1;
-          if (lane == 0) ls_record_fault(err, LS_DEV_WAIT_TIMEOUT, 900 + s);
-          break;
-        }
-        if (lane == 0) mbar_expect_tx(&full_bar[s], KV_BYTES);
-        __syncwarp();
-        if (lane < boxes) {
-          if (page < 0 || page >= num_pages) {
-            ls_record_fault(err, LS_DEV_PAGE_RANGE, c0 + lane * rows_per_box);
-            page = 0;
-          }
-          const int in_page = ((c0 + lane * rows_per_box) % page_size) / rows_per_box * rows_per_box;
-          const int y = ((page * 2 + (keys ? 0 : 1)) * nkv + I.kvh) * page_size + in_page;
-#pragma unroll
-          for (int hh = 0; hh < HALVES; ++hh)
-            tma_load_2d(dst_base + (uint32_t)(s * KV_BYTES + hh * HALF_BYTES + lane * rows_per_box * 128), &map_kv,
-                        hh * 64, y, &full_bar[s]);
-        }
-        page = lookup(I, it + 1);
-      }
-      gt += I.n_tiles;
-      ++j;
-    }
-  } else if (warp == 1) {
-    // ---- MMA issue (the whole warp walks the loop, one elected lane issues) ----
-    constexpr uint32_t idesc_s = instr_desc(BLOCK_M, BLOCK_N, false);
-    constexpr uint32_t idesc_o = instr_desc(BLOCK_M, D, true);
-    const bool issuer = elect_one();
-    int gt = 0, j = 0;
-    bool ok = true;
-    for (int round = 0; ok; ++round) {
-      Item I;
-      const int kind = get_item(round, I);
-      if (kind == 0) break;
-      if (kind == 2) continue;
-      ok = __all_sync(0xffffffffu, mbar_wait(q_full, (uint32_t)j & 1u));
-      // S_x(it) = Q_x K(it)^T; the keys are waited for by the first head's product
-      auto issue_s = [&](int x, int it) {
-        const int g = gt + it;
-        const int s = g & 1;
-        if (x == 0) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&k_full[s], (uint32_t)(g >> 1) & 1u))) return false;
-          fence_after_sync();
-        }
-        if (issuer) {
-#pragma unroll
-          for (int k = 0; k < D / UMMA_K; ++k) {
-            const uint32_t koff = (uint32_t)((k >> 2) * HALF_BYTES + (k & 3) * UMMA_K * 2);
-            umma(tmem_base + S_COL + x * BLOCK_N, desc_k_major(q_smem + x * KV_BYTES + koff),
-                 desc_k_major(k_smem + s * KV_BYTES + koff), idesc_s, k != 0 ? 1u : 0u);
-          }
-          umma_commit(&s_full[x]);
-          if (x == 1) {
-            umma_commit(&k_free[s]);
-            if (it == I.n_tiles - 1) umma_commit(q_free);
-          }
-        }
-        __syncwarp();
-        return true;
-      };
-      // O_x += P_x(it) V(it); the values are waited for by the first head's product
-      auto issue_pv = [&](int x, int it) {
-        const int g = gt + it;
-        const int s = g & 1;
-        bool got = mbar_wait(&p_full[x], (uint32_t)g & 1u);
-        if (x == 0) got = got && mbar_wait(&v_full[s], (uint32_t)(g >> 1) & 1u);
-        if (!__all_sync(0xffffffffu, got)) return false;
-        fence_after_sync();
-        if (issuer) {
-#pragma unroll
-          for (int k = 0; k < BLOCK_N / UMMA_K; ++k) {
-            // 16 keys are 8 columns of P: keys 0..63 at columns 0..31 of S_x, keys 64..127 at 64..95
-            const uint32_t pcol = (uint32_t)(k < 4 ? k * 8 : 64 + (k - 4) * 8);
-            const uint64_t b = desc_mn_major(v_smem + s * KV_BYTES + k * UMMA_K * 128, HALF_BYTES);
-            umma_ts(tmem_base + O_COL + x * 128, tmem_base + S_COL + x * BLOCK_N + pcol, b, idesc_o,
-                    (it | k) != 0 ? 1u : 0u);
-          }
-          umma_commit(&o_full[x]);
-          if (x == 1) umma_commit(&v_free[s]);
-        }
-        __syncwarp();
-        return true;
-      };
-      if (ok) ok = issue_s(0, 0);
-      if (ok) ok = issue_s(1, 0);
-      for (int it = 0; it < I.n_tiles && ok; ++it) {
-        ok = issue_pv(0, it);
-        if (ok && it + 1 < I.n_tiles) ok = issue_s(0, it + 1);
-        if (ok) ok = issue_pv(1, it);
-        if (ok && it + 1 < I.n_tiles) ok = issue_s(1, it + 1);
-      }
-      gt += I.n_tiles;
-      ++j;
-    }
-    if (!ok) {
-      *failed = 1;
-      if (issuer) ls_record_fault(err, LS_DEV_WAIT_TIMEOUT, 920);
-    }
-  } else if (warp < PAIR_V_WARP) {
-    // ---- softmax: team x = (warp - 2) / 8 has head I.h + x; two threads a row: `sub` has keys
-    // 64 sub .. 64 sub + 63 of a tile (read in pieces of 32) and half of the head's dimensions ----
-    constexpr int HC = 32;                        // scores in registers at a time
-    const int team = (warp - 2) >> 3;
-    const int sub = ((warp - 2) >> 2) & 1;
-    const int quad = warp & 3;
-    const int row = quad * 32 + lane;
-    const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
-    const uint32_t s_col = lane_base + S_COL + team * BLOCK_N;
-    const uint32_t o_col = lane_base + O_COL + team * 128 + sub * (D / 2);
-    float* tmax = team_mem + team * 1024;         // [parity][sub][128]: the two threads of a row exchange their maxima
-    float* l_part = tmax + 512;                   // [quarter][128]
-    constexpr float LAZY = 8.f;
-    bool ok = true;
-    int gt = 0;
-    // A wait that runs out clears `ok`; the loops still run to their ends, skipping the work, so
-    // that every thread meets the named barriers of every tile of every item.
-    for (int round = 0;; ++round) {
-      Item I;
-      const int kind = get_item(round, I);
-      if (kind == 0) break;
-      if (kind == 2) continue;
-      const int pos0 = I.pos0, pos_last = I.pos_last, tile_first = I.tile_first, n_tiles = I.n_tiles;
-      const int pos = pos0 + row;
-      const int lo = ls_first_key(pos, window);
-      const int lo_last = ls_first_key(pos_last, window);
-      // the sum of a row's weights is kept per quarter of a tile's keys (32 sub .. + 31), as the
-      // kernel with four threads a row keeps it, so that both give the same bits
-      float m_ref = -CUDART_INF_F, l_run[2] = {0.f, 0.f};
-      for (int it = 0; it < n_tiles; ++it) {
-        const int g = gt + it;
-        const int s = g & 1;                       // stage of the tile's keys and values
-        const int c0 = (tile_first + it) * BLOCK_N + sub * 64;        // first key of this thread
-        if (ok && !mbar_wait(&s_full[team], (uint32_t)g & 1u)) ok = false;
-        fence_after_sync();
-        const bool full_tile = (tile_first + it) * BLOCK_N + BLOCK_N - 1 <= pos0 && (tile_first + it) * BLOCK_N >= lo_last;
-        // ---- the row's maximum over the tile ----
-        float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-#pragma unroll
-        for (int piece = 0; piece < 2; ++piece) {
-          uint32_t sc[HC];
-          tmem_ld32(s_col + sub * 64 + piece * HC, sc);
-          tmem_ld_wait();
-          if (full_tile) {
-#pragma unroll
-            for (int jj = 0; jj < HC; jj += 2)
-              mx[(jj >> 1) & 3] = max3(mx[(jj >> 1) & 3], __uint_as_float(sc[jj]), __uint_as_float(sc[jj + 1]));
-          } else {
-            // selects, not branches: a masked score counts as -inf
-#pragma unroll
-            for (int jj = 0; jj < HC; ++jj) {
-              const int key = c0 + piece * HC + jj;
-              const bool keep = (key <= pos) & (key >= lo);
-              mx[jj & 3] = fmaxf(mx[jj & 3], keep ? __uint_as_float(sc[jj]) : -CUDART_INF_F);
-            }
-          }
-        }
-        float tile_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-        const int par = it & 1;
-        tmax[par * 256 + sub * 128 + row] = tile_max;
-        if (team == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
-        else asm volatile("bar.sync 2, 256;" ::: "memory");
-        tile_max = fmaxf(tmax[par * 256 + row], tmax[par * 256 + 128 + row]);
-        // both threads of a row work out the same m_ref from the same numbers
-        const float m_new = tile_max * scale_log2;
-        const bool move = m_new > m_ref + LAZY;                      // true too for the first key a row sees
-        const float factor = move ? ((m_ref == -CUDART_INF_F) ? 0.f : ex2(m_ref - m_new)) : 1.f;
-        if (move) m_ref = m_new;
-        // O is scaled only after the PV of the tile before has been added to it (and before this
-        // tile's P is announced, so before the PV of this tile)
-        if (it > 0 && __any_sync(0xffffffffu, move)) {
-          if (ok && !mbar_wait(&o_full[team], (uint32_t)(g - 1) & 1u)) ok = false;
-          if (__all_sync(0xffffffffu, ok)) {
-            fence_after_sync();
-#pragma unroll
-            for (int piece = 0; piece < D / 64; ++piece) {            // this thread's half of the row, 32 columns at a time
+            for (int c = 0; c < D; c += 32) {
               uint32_t og[32];
-              tmem_ld32(o_col + piece * 32, og);
+              tmem_ld32(lane_base + O_COL + c, og);
               tmem_ld_wait();
 #pragma unroll
-              for (int c = 0; c < 32; ++c) og[c] = __float_as_uint(__uint_as_float(og[c]) * factor);
-              tmem_st32(o_col + piece * 32, og);
+              for (int e = 0; e < 32; ++e) og[e] = __float_as_uint(__uint_as_float(og[e]) * factor);
+              tmem_st32(lane_base + O_COL + c, og);
             }
           }
         }
-        // ---- p = exp2(s * scale - m_ref), rounded to bfloat16, two keys a column, written over
-        // scores this thread has already taken ----
+        // p = exp2(s * scale - m_ref), rounded to bfloat16, two keys a column, written over scores this
+        // thread has taken, from where the PV product takes it as its A operand; the sum in four
+        // running sums, folded in a fixed order
+        float ps[4] = {0.f, 0.f, 0.f, 0.f};
         const bool dead = m_ref == -CUDART_INF_F;          // nothing seen yet by this row
-        const float neg_m = dead ? 0.f : -m_ref;
-        const bool plain = full_tile & !dead;               // uniform over the block but for `dead`
+        const float add = dead ? 0.f : -m_ref;
 #pragma unroll
-        for (int piece = 0; piece < 2; ++piece) {
-          uint32_t sc[HC];
-          tmem_ld32(s_col + sub * 64 + piece * HC, sc);
-          tmem_ld_wait();
-          uint32_t pk[HC / 2];
-          float ps[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int n0 = 0; n0 < BLOCK_N; n0 += 32) {
+          uint32_t pk[16];
 #pragma unroll
-          for (int n0 = 0; n0 < HC; n0 += 8) {
-            float p[8];
-            if (plain) {
+          for (int jj = 0; jj < 32; jj += 4) {
+            float p[4];
 #pragma unroll
-              for (int jj = 0; jj < 8; jj += 2) {
-                p[jj] = __uint_as_float(sc[n0 + jj]);
-                p[jj + 1] = __uint_as_float(sc[n0 + jj + 1]);
-                fma2(p[jj], p[jj + 1], scale_log2, neg_m);
-                p[jj] = ex2(p[jj]);
-                p[jj + 1] = ex2(p[jj + 1]);
-              }
-            } else {
-              // every exponential is taken, masked ones of -inf (which is 0): selects, not branches
+            for (int e = 0; e < 4; ++e) p[e] = __uint_as_float(sc[n0 + jj + e]);
+            fma2(p[0], p[1], scale_eff, add);
+            fma2(p[2], p[3], scale_eff, add);
 #pragma unroll
-              for (int jj = 0; jj < 8; ++jj) {
-                const int key = c0 + piece * HC + n0 + jj;
-                const bool keep = (key <= pos) & (key >= lo) & !dead;
-                p[jj] = ex2(keep ? fmaf(__uint_as_float(sc[n0 + jj]), scale_log2, neg_m) : -CUDART_INF_F);
-              }
-            }
+            for (int e = 0; e < 4; ++e) p[e] = ex2(p[e]);
             add2(ps[0], ps[1], p[0], p[1]);
             add2(ps[2], ps[3], p[2], p[3]);
-            add2(ps[0], ps[1], p[4], p[5]);
-            add2(ps[2], ps[3], p[6], p[7]);
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) pk[(n0 >> 1) + jj] = pack_bf16(p[2 * jj], p[2 * jj + 1]);
+            pk[jj >> 1] = pack_bf16(p[0], p[1]);
+            pk[(jj >> 1) + 1] = pack_bf16(p[2], p[3]);
           }
-          tmem_st16(s_col + sub * 64 + piece * (HC / 2), pk);
-          l_run[piece] = fmaf(l_run[piece], factor, (ps[0] + ps[1]) + (ps[2] + ps[3]));
+          tmem_st16(s_addr + (n0 >> 1), pk);
+        }
+        float psum = (ps[0] + ps[1]) + (ps[2] + ps[3]);
+        if (__any_sync(0xffffffffu, dead && psum != 0.f)) {
+          // (a row that has seen scores that are no numbers and nothing else weighs nothing)
+          tmem_st_wait();
+#pragma unroll
+          for (int c = 0; c < BLOCK_N / 2; c += 32) {
+            uint32_t pk[32];
+            tmem_ld32(s_addr + c, pk);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) pk[e] = dead ? 0u : pk[e];
+            tmem_st32(s_addr + c, pk);
+          }
+          if (dead) psum = 0.f;
         }
         // value rows of keys past the last position were never written: they must not be NaN,
         // since P is zero there and the MMA multiplies all the same
-        if ((tile_first + it) * BLOCK_N + BLOCK_N - 1 > pos_last) {
-          if (ok && !mbar_wait(&v_full[s], (uint32_t)(g >> 1) & 1u)) ok = false;
-          if (ok && sub < HALVES && (tile_first + it) * BLOCK_N + row > pos_last) {
-            uint4* vrow = reinterpret_cast<uint4*>(v_ptr + s * KV_BYTES + sub * HALF_BYTES + row * 128);
+        if (c0 + BLOCK_N - 1 > pos_last) {
+          if (ok && !mbar_wait(&v_full[g & 1], (uint32_t)(g >> 1) & 1u)) ok = false;
+          if (ok && c0 + row > pos_last) {
+            uint4* vrow = reinterpret_cast<uint4*>(v_ptr + (g & 1) * TILE_BYTES + (row >> 3) * GROUP_BYTES + (row & 7) * 128);
 #pragma unroll
-            for (int q8 = 0; q8 < 8; ++q8) vrow[q8] = make_uint4(0u, 0u, 0u, 0u);
+            for (int hh = 0; hh < HALVES; ++hh)
+#pragma unroll
+              for (int q8 = 0; q8 < 8; ++q8) vrow[hh * 64 + q8] = make_uint4(0u, 0u, 0u, 0u);
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
         tmem_st_wait();
         fence_before_sync();
         __syncwarp();
-        if (lane == 0 && ok) mbar_arrive(&p_full[team]);
+        if (lane == 0 && ok) mbar_arrive(p_bar);
+        l_run = fmaf(l_run, factor, psum);
       }
-      // ---- the item's end: the row's sum is that of its four quarters in order; each thread
-      // writes half of the row out ----
-      l_part[(sub * 2) * 128 + row] = l_run[0];
-      l_part[(sub * 2 + 1) * 128 + row] = l_run[1];
-      if (team == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
-      else asm volatile("bar.sync 2, 256;" ::: "memory");
-      float l_row = l_part[row];
-#pragma unroll
-      for (int o = 1; o < 4; ++o) l_row += l_part[o * 128 + row];
+      // ---- the item's end: the team that had the last tile takes the other's sum and writes the
+      // rows out, while the other goes on to the next item ----
       const int g_last = gt + n_tiles - 1;
-      if (ok && !mbar_wait(&o_full[team], (uint32_t)g_last & 1u)) ok = false;
-      if (ok) {
-        fence_after_sync();
-        const float inv = l_row > 0.f ? 1.0f / l_row : 0.f;
-        __nv_bfloat16* dst = out + ((int64_t)(I.tok0 + row) * nq + I.h + team) * D + sub * (D / 2);
+      const int lb = shared_items & 3;
+      const uint32_t l_par = (uint32_t)(shared_items >> 2) & 1u;
+      if ((g_last & 1) != team) {
+        if (n_tiles > 1) {
+          hand_l[lb * 128 + row] = l_run;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&l_full[lb]);
+        }
+      } else {
+        float l_row = l_run;
+        if (n_tiles > 1) {
+          if (ok && !mbar_wait(&l_full[lb], l_par)) ok = false;
+          // (rounded one by one: the same sum whichever team has the last tile)
+          if (m_before != -CUDART_INF_F)
+            l_row = __fadd_rn(__fmul_rn(hand_l[lb * 128 + row], ex2(m_before - m_ref)), l_row);
+        }
+        if constexpr (EXTRAS) {
+          // the sink, in the units of this row's sums (2^m_ref)
+          if (sinks != nullptr && m_ref != -CUDART_INF_F) l_row += ex2(fmaf(sinks[I.h], 1.4426950408889634f, -m_ref));
+        }
+        if (ok && !mbar_wait(&o_full[g_last & 1], (uint32_t)(g_last >> 1) & 1u)) ok = false;
+        if (__all_sync(0xffffffffu, ok)) {
+          fence_after_sync();
+          uint32_t og[D];
 #pragma unroll
-        for (int piece = 0; piece < D / 64; ++piece) {
-          uint32_t og[32];
-          tmem_ld32(o_col + piece * 32, og);
+          for (int c = 0; c < D; c += 32) tmem_ld32(lane_base + O_COL + c, og + c);
           tmem_ld_wait();
+          fence_before_sync();                       // the next item's first PV overwrites O
+          __syncwarp();
+          if (lane == 0) mbar_arrive(o_free);
           if (row < I.ntok) {
+            const float inv = l_row > 0.f ? 1.0f / l_row : 0.f;
+            __nv_bfloat16* dst = out + ((int64_t)(I.tok0 + row) * nq + I.h) * D;
 #pragma unroll
-            for (int c = 0; c < 32; c += 8) {
+            for (int c = 0; c < D; c += 8) {
               uint4 v;
               v.x = pack_bf16(__uint_as_float(og[c]) * inv, __uint_as_float(og[c + 1]) * inv);
               v.y = pack_bf16(__uint_as_float(og[c + 2]) * inv, __uint_as_float(og[c + 3]) * inv);
               v.z = pack_bf16(__uint_as_float(og[c + 4]) * inv, __uint_as_float(og[c + 5]) * inv);
               v.w = pack_bf16(__uint_as_float(og[c + 6]) * inv, __uint_as_float(og[c + 7]) * inv);
-              *reinterpret_cast<uint4*>(dst + piece * 32 + c) = v;
+              *reinterpret_cast<uint4*>(dst + c) = v;
             }
           }
         }
-        fence_before_sync();                         // the next item's first PV overwrites O after its P
       }
-      // the sums are read before any thread writes them for the next item
-      if (team == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
-      else asm volatile("bar.sync 2, 256;" ::: "memory");
+      shared_items += n_tiles > 1 ? 1 : 0;
       gt += n_tiles;
     }
+    // the announcement of the block's last tile is taken like any other
+    if (gt > 0 && ((gt - 1) & 1) != team) asm volatile("bar.sync %0, 64;" ::"r"(1 + quad * 2 + ((gt - 1) & 1)) : "memory");
     if (!ok) {
       *failed = 1;
-      if (lane == 0) ls_record_fault(err, LS_DEV_WAIT_TIMEOUT, 940 + quad);
+      if (lane == 0) ls_record_fault(err, LS_DEV_WAIT_TIMEOUT, 840 + quad);
+    }
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (producer) {
+      // ---- producers: K_WARP fetches Q and the key tiles, V_WARP the value tiles: a key stage
+      // is free earlier than the value stage of the same tile, and neither waits for the other's ----
+      const bool keys = warp == K_WARP;
+      uint64_t* free_bar = keys ? k_free : o_full;
+      uint64_t* full_bar = keys ? k_full : v_full;
+      const uint32_t dst_base = keys ? k_smem : v_smem;
+      int g = 0, j = 0;                 // tiles and items of this block so far
+      bool ok = true;
+      for (int round = 0; ok; ++round) {
+        Item I;
+        const int kind = get_item(round, I);
+        if (kind == 0) break;
+        if (kind == 2) continue;
+        int page = round == 0 ? first_page : lookup(I, 0);
+        if (keys) {
+          // a stage of Q is free once the last S product of the item before the one before has read it
+          const int qs = j & 1;
+          const uint32_t phase = (uint32_t)(j >> 1) & 1u;
+          ok = __all_sync(0xffffffffu, *failed == 0 && mbar_wait(&q_free[qs], phase ^ 1u));
+          if (!ok) {
+            *failed = 1;
+            if (lane == 0) ls_record_fault(err, LS_DEV_WAIT_TIMEOUT, 810);
+            break;
+          }
+          if (lane == 0) {
+            mbar_expect_tx(&q_full[qs], TILE_BYTES);
+#pragma unroll
+            for (int hh = 0; hh < HALVES; ++hh)
+              tma_load_2d(q_smem + qs * TILE_BYTES + hh * HALF_BYTES, &map_q, I.h * D + hh * 64, I.tok0, &q_full[qs]);
+          }
+          __syncwarp();
+        }
+        ++j;
+        for (int it = 0; it < I.n_tiles; ++it) {
+          const int s = g & 1;
+          const uint32_t phase = (uint32_t)(g >> 1) & 1u;
+          const int c0 = I.tile(it) * BLOCK_N;
+          ok = __all_sync(0xffffffffu, *failed == 0 && mbar_wait(&free_bar[s], phase ^ 1u));
+          if (!ok) {
+            *failed = 1;
+            if (lane == 0) ls_record_fault(err, LS_DEV_WAIT_TIMEOUT, 800 + s);
+            break;
+          }
+          if (lane == 0) mbar_expect_tx(&full_bar[s], TILE_BYTES);
+          __syncwarp();
+          if (lane < boxes) {
+            if (page < 0 || page >= num_pages) {
+              ls_record_fault(err, LS_DEV_PAGE_RANGE, c0 + lane * rows_per_box);
+              page = 0;
+            }
+            const int in_page = ((c0 + lane * rows_per_box) % page_size) / rows_per_box * rows_per_box;
+            const int y = ((page * 2 + (keys ? 0 : 1)) * nkv + I.kvh) * page_size + in_page;
+            tma_load_4d(dst_base + (uint32_t)(s * TILE_BYTES + lane * (rows_per_box >> 3) * GROUP_BYTES), &map_kv, 0, 0, 0,
+                        y >> 3, &full_bar[s]);
+          }
+          page = lookup(I, it + 1);     // after this tile's loads have gone out
+          ++g;
+        }
+      }
+      if (!ok && lane == 0) {
+        // wait (bounded) for the copies still in flight before the block winds down
+        for (int b = g > 2 ? g - 2 : 0; b < g; ++b) mbar_wait(&full_bar[b & 1], (uint32_t)(b >> 1) & 1u);
+        if (keys)
+          for (int b = j > 2 ? j - 2 : 0; b < j; ++b) mbar_wait(&q_full[b & 1], (uint32_t)(b >> 1) & 1u);
+      }
+    } else if (warp == MMA_WARP) {
+      // ---- MMA issue: the whole warp walks the loop and one elected lane issues, so that the
+      // instructions' operands are the same in every lane and stay in uniform registers (inside a
+      // branch of one lane every MMA paid for moving them there) ----
+      constexpr uint32_t idesc_s = instr_desc(BLOCK_M, BLOCK_N, false);
+      constexpr uint32_t idesc_o = instr_desc(BLOCK_M, D, true);
+      const bool issuer = elect_one();
+      // two walks over the block's tiles: S runs two tiles ahead of PV
+      struct Walk {
+        int round, n, it, j, g;    // round to look at next; tiles of the item (0: none is left); tile, item and tiles so far
+      };
+      // What steers the loop comes out of a reduction over the warp, whose result lies in a uniform register: the
+      // loop's state then stays there.  (Steered by values loaded from the work list, every MMA's descriptors and every
+      // barrier's address were moved there one by one, 2,100 cycles of this warp a tile, and nothing else set the pace.)
+      auto next_item = [&](Walk& w) {
+        int n;
+        do {
+          Item I;
+          const int kind = get_item(w.round, I);
+          n = __reduce_max_sync(0xffffffffu, kind == 0 ? -1 : kind == 2 ? 0 : I.n_tiles);
+          ++w.round;
+        } while (n == 0);
+        w.n = n > 0 ? n : 0;
+        w.it = 0;
+      };
+      auto advance = [&](Walk& w) {
+        ++w.g;
+        if (++w.it == w.n) {
+          ++w.j;
+          next_item(w);
+        }
+      };
+      const uint32_t tmem = __reduce_max_sync(0xffffffffu, tmem_base);
+      const uint64_t q_desc = desc_k_major(q_smem), k_desc = desc_k_major_groups<GROUP_BYTES>(k_smem);
+      const uint64_t v_desc = desc_mn_major<HALVES>(v_smem);
+      Walk ws = {0, 0, 0, 0, 0};
+      next_item(ws);
+      Walk wp = ws;
+      bool ok = true;
+      int s_tile = 0;                   // ws.g % 3
+      int p_tile = 0;                   // wp.g % 3 and the parity of wp.g / 3
+      uint32_t p_phase = 0;
+      // keys (and Q) of the tile at ws
+      auto wait_s = [&]() {
+        bool got = mbar_wait(&k_full[ws.g & 1], (uint32_t)(ws.g >> 1) & 1u);
+        if (ws.it == 0) got = got && mbar_wait(&q_full[ws.j & 1], (uint32_t)(ws.j >> 1) & 1u);
+        return got;
+      };
+      auto issue_s = [&]() {            // S of the tile at ws
+        // (the S tile is free: the PV product of the tile that lay in it has been issued before)
+        const int s = ws.g & 1, qs = ws.j & 1;
+        if (issuer) {
+#pragma unroll
+          for (int k = 0; k < D / UMMA_K; ++k) {
+            // (offsets in the descriptors' units of 16 bytes)
+            const uint32_t qoff = (uint32_t)((k >> 2) * HALF_BYTES + (k & 3) * UMMA_K * 2) >> 4;
+            const uint32_t koff = (uint32_t)((k >> 2) * 1024 + (k & 3) * UMMA_K * 2) >> 4;
+            umma(tmem + s_tile * BLOCK_N, q_desc + (uint32_t)(qs * (TILE_BYTES >> 4)) + qoff,
+                 k_desc + (uint32_t)(s * (TILE_BYTES >> 4)) + koff, idesc_s, k != 0 ? 1u : 0u);
+          }
+          umma_commit(&s_full[s_tile]);
+          umma_commit(&k_free[s]);
+          if (ws.it == ws.n - 1) umma_commit(&q_free[qs]);     // the item's last product with this Q
+        }
+        __syncwarp();
+        if (++s_tile == S_TILES) s_tile = 0;
+        advance(ws);
+      };
+      for (int ahead = 0; ahead < 2 && ok && ws.n != 0; ++ahead) {
+        ok = __all_sync(0xffffffffu, wait_s());
+        if (!ok) break;
+        fence_after_sync();
+        issue_s();
+      }
+      while (ok && wp.n != 0) {
+        // what is there long before it is needed is waited for together, while the product before runs
+        const int s = wp.g & 1;
+        bool got = mbar_wait(&v_full[s], (uint32_t)(wp.g >> 1) & 1u);
+        if (ws.n != 0) got = got && wait_s();
+        ok = __all_sync(0xffffffffu, got);
+        if (!ok) break;
+        fence_after_sync();
+        if (ws.n != 0) issue_s();
+        got = mbar_wait(&p_full[p_tile], p_phase);
+        // the first product of an item overwrites O
+        if (wp.it == 0 && wp.j > 0) got = got && mbar_wait(o_free, (uint32_t)(wp.j - 1) & 1u);
+        ok = __all_sync(0xffffffffu, got);
+        if (!ok) break;
+        fence_after_sync();
+        if (issuer) {
+#pragma unroll
+          for (int k = 0; k < BLOCK_N / UMMA_K; ++k) {
+            // P from tensor memory: 16 keys are 8 columns; V: 16 keys are two groups
+            umma_ts(tmem + O_COL, tmem + p_tile * BLOCK_N + k * (UMMA_K / 2),
+                    v_desc + (uint32_t)(s * (TILE_BYTES >> 4) + k * (2 * GROUP_BYTES >> 4)), idesc_o, (wp.it | k) != 0 ? 1u : 0u);
+          }
+          umma_commit(&o_full[s]);
+        }
+        __syncwarp();
+        if (++p_tile == S_TILES) {
+          p_tile = 0;
+          p_phase ^= 1u;
+        }
+        advance(wp);
+      }
+      if (!ok) {
+        *failed = 1;
+        if (issuer) ls_record_fault(err, LS_DEV_WAIT_TIMEOUT, 820);
+      }
     }
   }
   fence_before_sync();
   __syncthreads();
-  if (warp == 2) {
+  if (warp == TEAM_WARP) {
     fence_after_sync();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS)
                  : "memory");
@@ -1119,6 +781,22 @@ bool encode(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t rows, ui
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The cache pages [rows = page, k or v, head, position][d] as {64 elements, 8 rows, halves, groups of 8 rows}: a box takes
+// box_rows consecutive rows (a multiple of 8) and leaves them as groups of 8 rows, each as its halves, each 8 x 128 bytes.
+// (One box a page instead of one a page and half: a warp gets a TMA load out about every 100 cycles.)
+bool encode_pages(CUtensorMap* map, const void* ptr, uint64_t halves, uint64_t rows, uint32_t box_rows) {
+  EncodeTiled enc = encode_fn();
+  if (enc == nullptr) return false;
+  const cuuint64_t pitch = (cuuint64_t)halves * 128;
+  cuuint64_t dims[4] = {64, 8, (cuuint64_t)halves, (cuuint64_t)rows / 8};
+  cuuint64_t strides[3] = {pitch, 128, 8 * pitch};
+  cuuint32_t box[4] = {64, 8, (cuuint32_t)halves, box_rows / 8};
+  cuuint32_t elem[4] = {1, 1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, strides, box, elem,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int sm_count() {
   static int sms = 0;
   if (sms == 0) {
@@ -1129,67 +807,33 @@ int sm_count() {
   return sms;
 }
 
-// 0: a head a block always; 1: two heads of a key head a block where that pays; 2: wherever the group is even
-int pair_heads = 1;
-
-template <int HALVES>
+template <int HALVES, bool EXTRAS>
 int launch(const CUtensorMap& map_q, const CUtensorMap& map_kv, void* out, const int* work, int n_work,
            const int* block_table, int table_stride, int nq, int nkv, int page_size, int num_pages, int window,
            int keep_first, float scale, const float* slopes, const float* log_rates, const float* sinks, float softcap,
            int* err, cudaStream_t stream) {
-  constexpr int KV_BYTES = HALVES * HALF_BYTES;
-  const size_t smem = (size_t)KV_BYTES * (1 + 2 * STAGES) + 256 + 3 * 128 * GROUPS * 4 + 1024;
+  constexpr size_t smem = (size_t)HALVES * HALF_BYTES * 3 * STAGES + 256 + 6 * 128 * 4 + 1024;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<HALVES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess ||
-        cudaFuncSetAttribute(attention_prefill_tc_kernel<HALVES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<HALVES, EXTRAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess)
       return LS_E_SMEM;
     configured = true;
   }
-  if (slopes != nullptr || sinks != nullptr || softcap > 0.f || keep_first > 0) {
-    // a bias on the scores, a cap, a sink or kept first keys: the kernel with a head a block knows them
-    const long long items = (long long)n_work * nq;
-    const int blocks = items < sm_count() ? (int)items : sm_count();
-    LS_COUNT(LS_K_ATTENTION_PREFILL_TC), ls_launch(attention_prefill_tc_kernel<HALVES, true>, dim3(blocks), THREADS, smem, stream, map_q, map_kv,
-              (__nv_bfloat16*)out, work, n_work, block_table, table_stride, nq, nkv, page_size, num_pages, window,
-              keep_first, scale * 1.4426950408889634f, slopes, log_rates, sinks, softcap > 0.f ? softcap * 1.4426950408889634f : 0.f, err);
-    return ls_launch_status();
-  }
-  // two heads of a key head in a block where the group size is even and there are items enough
-  // to fill the device one and a half times over (with fewer, the longest item would set the
-  // time: a prompt of 2,048 tokens and 16 heads is 128 pairs, the longest of 16 double tiles)
-  if (pair_heads && (nq / nkv) % 2 == 0 &&
-      (pair_heads > 1 || 2LL * n_work * (nq / 2) >= 3LL * sm_count())) {
-    const size_t pair_smem = (size_t)KV_BYTES * (2 + 2 * STAGES) + 256 + 2 * 1024 * 4 + 1024;
-    static bool pair_configured = false;
-    if (!pair_configured) {
-      if (cudaFuncSetAttribute(attention_prefill_tc_pair_kernel<HALVES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)pair_smem) != cudaSuccess)
-        return LS_E_SMEM;
-      pair_configured = true;
-    }
-    const long long pair_items = (long long)n_work * (nq / 2);
-    const int pair_blocks = pair_items < sm_count() ? (int)pair_items : sm_count();
-    LS_COUNT(LS_K_ATTENTION_PREFILL_TC), ls_launch(attention_prefill_tc_pair_kernel<HALVES>, dim3(pair_blocks), PAIR_THREADS, pair_smem, stream, map_q, map_kv,
-              (__nv_bfloat16*)out, work, n_work, block_table, table_stride, nq, nkv, page_size, num_pages, window,
-              scale * 1.4426950408889634f, err);
-    return ls_launch_status();
-  }
   // a block per SM (its shared memory and its 512 columns of tensor memory fill one), or fewer items
   const long long items = (long long)n_work * nq;
   const int blocks = items < sm_count() ? (int)items : sm_count();
-  LS_COUNT(LS_K_ATTENTION_PREFILL_TC), ls_launch(attention_prefill_tc_kernel<HALVES, false>, dim3(blocks), THREADS, smem, stream, map_q, map_kv, (__nv_bfloat16*)out, work, n_work,
-            block_table, table_stride, nq, nkv, page_size, num_pages, window, 0, scale * 1.4426950408889634f,
-            (const float*)nullptr, (const float*)nullptr, (const float*)nullptr, 0.f, err);
+  LS_COUNT(LS_K_ATTENTION_PREFILL_TC), ls_launch(attention_prefill_tc_kernel<HALVES, EXTRAS>, dim3(blocks), THREADS, smem, stream, map_q, map_kv,
+            (__nv_bfloat16*)out, work, n_work, block_table, table_stride, nq, nkv, page_size, num_pages, window,
+            keep_first, scale * 1.4426950408889634f, slopes, log_rates, sinks, softcap > 0.f ? softcap * 1.4426950408889634f : 0.f, err);
   return ls_launch_status();
 }
 
 }  // namespace
 
 LS_API int ls_attention_prefill_tc_tile_tokens() { return BLOCK_M; }
-LS_API void ls_set_attention_prefill_pairs(int mode) { pair_heads = mode < 0 ? 0 : (mode > 2 ? 2 : mode); }
+// (a choice between kernels of one and of two heads a block, which there was: one kernel takes every launch)
+LS_API void ls_set_attention_prefill_pairs(int) {}
 
 // q, out: [tokens, nq * d] bfloat16; pages [num_pages, 2, nkv, page_size, d]; d 64 or 128; page
 // sizes 8, 16, 32, 64, 128.  Work items as for ls_attention_tile with up to 128 tokens each
@@ -1211,17 +855,17 @@ LS_API int ls_attention_prefill_tc(const void* q, const void* pages, void* out, 
   if (((uintptr_t)pages & 127) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15)) return LS_E_ALIGN;
   CUtensorMap map_q, map_kv;
   if (!encode(&map_q, q, (uint64_t)nq * d, (uint64_t)tokens, BLOCK_M)) return LS_E_SIZE;
-  if (!encode(&map_kv, pages, (uint64_t)d, (uint64_t)rows, page_size < BLOCK_N ? page_size : BLOCK_N)) return LS_E_SIZE;
-  if (d == 64)
-    return launch<1>(map_q, map_kv, out, work, n_work, block_table, table_stride, nq, nkv, page_size, num_pages,
-                     window, keep_first, scale, slopes, log_rates, sinks, softcap, err, stream);
-  return launch<2>(map_q, map_kv, out, work, n_work, block_table, table_stride, nq, nkv, page_size, num_pages,
-                   window, keep_first, scale, slopes, log_rates, sinks, softcap, err, stream);
+  if (!encode_pages(&map_kv, pages, (uint64_t)d / 64, (uint64_t)rows, page_size < BLOCK_N ? page_size : BLOCK_N)) return LS_E_SIZE;
+  // a bias on the scores, a cap, a sink, kept first keys or a scale that is not above 0: an instance of its own, so that the other keeps no branch for them
+  const bool extras = slopes != nullptr || sinks != nullptr || softcap > 0.f || keep_first > 0 || !(scale > 0.f);
+  auto go = d == 64 ? (extras ? launch<1, true> : launch<1, false>) : (extras ? launch<2, true> : launch<2, false>);
+  return go(map_q, map_kv, out, work, n_work, block_table, table_stride, nq, nkv, page_size, num_pages, window,
+            keep_first, scale, slopes, log_rates, sinks, softcap, err, stream);
 }
 
 LS_API const char* ls_constants_attention_prefill_tc() {
   static char buf[256];
   static const LsConstant c[] = {{"attention_prefill_tc.queries", BLOCK_M}, {"attention_prefill_tc.keys", BLOCK_N},
-                                 {"attention_prefill_tc.softmax_threads_per_row", GROUPS}};
+                                 {"attention_prefill_tc.softmax_threads_per_row", 1}};
   return ls_format_constants(buf, sizeof buf, c, (int)(sizeof c / sizeof c[0]));
 }

@@ -193,9 +193,8 @@ def set_gemm_tc_pairs(on: bool) -> None:
 
 
 def set_attention_prefill_pairs(mode: int) -> None:
-    """How the tensor-core attention of prompt portions takes the heads of a key head: 0 one
-    head a block; 1 (the default) two heads a block, sharing the key and value tiles, where the
-    group size is even and the items fill the device twice over; 2 wherever the group is even."""
+    """Chose between kernels with one and with two heads a block for the tensor-core attention of prompt
+    portions; one kernel takes every launch now, and the choice has no effect."""
     fn = library("tc").ls_set_attention_prefill_pairs
     fn.argtypes, fn.restype = [c_int], None
     fn(int(mode))
