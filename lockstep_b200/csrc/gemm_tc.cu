@@ -173,7 +173,8 @@ struct NormArgs {
 };
 constexpr int NORM_MAX_PARTS = 4;
 
-template <int BN, int EPI, typename TC>
+// SH: the most shares the instance folds (2, 4 or 8).
+template <int BN, int EPI, typename TC, int SH>
 __global__ void __launch_bounds__(192, 1)
 gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                        TC* __restrict__ C, int T, int N, int K, int64_t ldc,
@@ -333,23 +334,25 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
     const int n = n0 + row;
-    uint32_t peer[MAX_SHARES];
+    uint32_t peer[SH];
 #pragma unroll
-    for (int r = 0; r < MAX_SHARES; ++r)
+    for (int r = 0; r < SH; ++r)
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer[r]) : "r"(base), "r"(r < shares ? r : 0));
     // FOLD columns at a time: their shares' values (and the old values of a residual) are all
     // asked for before any is used, so that a block pays a few trips through the cluster's
-    // shared memory and not one per column
-    constexpr int FOLD = 4;
+    // shared memory and not one per column.  All columns of a block at 64 tokens where the shares are few (64 tokens, four
+    // shares: q/k/v of 1,024 to 4,096 features 7.4 -> 6.8 us, gate/up of 3,072 11.4 -> 8.6; 128 tokens 18.0 -> 12.4); with eight, four at
+    // a time are faster than eight (o and down 6.05 and 6.63 against 6.23 and 6.75).
+    constexpr int FOLD = SH == 8 ? 4 : 64 / SH;
     for (int c0 = (int)blockIdx.z; c0 < BN; c0 += FOLD * shares) {
-      float vg[FOLD][MAX_SHARES], vu[FOLD][MAX_SHARES], before[FOLD];
+      float vg[FOLD][SH], vu[FOLD][SH], before[FOLD];
 #pragma unroll
       for (int f = 0; f < FOLD; ++f) {
         const int c = c0 + f * shares;
         const bool live = c < BN && t0 + c < T;
         const uint32_t off_g = (uint32_t)((c * BM + row) * 4), off_u = (uint32_t)(((BN + c) * BM + row) * 4);
 #pragma unroll
-        for (int r = 0; r < MAX_SHARES; ++r) {
+        for (int r = 0; r < SH; ++r) {
           vg[f][r] = (live && r < shares) ? ld_cluster_f32(peer[r] + off_g) : 0.f;
           if (EPI == 2) vu[f][r] = (live && r < shares) ? ld_cluster_f32(peer[r] + off_u) : 0.f;
         }
@@ -363,7 +366,7 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         if (c >= BN || t0 + c >= T) break;
         float g = 0.f, u = 0.f;
 #pragma unroll
-        for (int r = 0; r < MAX_SHARES; ++r) {
+        for (int r = 0; r < SH; ++r) {
           if (r < shares) {
             g += vg[f][r];
             if (EPI == 2) u += vu[f][r];
@@ -1570,13 +1573,13 @@ int sm_count() {
   return sms;
 }
 
-template <int BN, int EPI, typename TC>
-int launch_cluster(const CUtensorMap& mw, const CUtensorMap& mx, void* C, int T, int N,
+template <int BN, int EPI, typename TC, int SH>
+int launch_cluster_of(const CUtensorMap& mw, const CUtensorMap& mx, void* C, int T, int N,
                    int K, int64_t ldc, const Plan& plan, int* err, cudaStream_t stream) {
   using S = ClusterShape<BN, EPI>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(gemm_tc_cluster_kernel<BN, EPI, TC>,
+    if (cudaFuncSetAttribute(gemm_tc_cluster_kernel<BN, EPI, TC, SH>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM) != cudaSuccess)
       return LS_E_SMEM;
     configured = true;
@@ -1596,10 +1599,18 @@ int launch_cluster(const CUtensorMap& mw, const CUtensorMap& mx, void* C, int T,
   cfg.attrs = attr;
   cfg.numAttrs = ls_dependent_launch ? 2 : 1;
   LS_COUNT(LS_K_GEMM_TC_CLUSTER);
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_cluster_kernel<BN, EPI, TC>, mw, mx, (TC*)C, T,
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_cluster_kernel<BN, EPI, TC, SH>, mw, mx, (TC*)C, T,
                                      N, K, ldc, plan.kb_per_share, plan.shares, err);
   if (e != cudaSuccess) return (int)e;
   return ls_launch_status();
+}
+
+template <int BN, int EPI, typename TC>
+int launch_cluster(const CUtensorMap& mw, const CUtensorMap& mx, void* C, int T, int N, int K, int64_t ldc, const Plan& plan,
+                   int* err, cudaStream_t stream) {
+  if (plan.shares <= 2) return launch_cluster_of<BN, EPI, TC, 2>(mw, mx, C, T, N, K, ldc, plan, err, stream);
+  if (plan.shares <= 4) return launch_cluster_of<BN, EPI, TC, 4>(mw, mx, C, T, N, K, ldc, plan, err, stream);
+  return launch_cluster_of<BN, EPI, TC, 8>(mw, mx, C, T, N, K, ldc, plan, err, stream);
 }
 
 constexpr int MAX_DYNAMIC_SMEM = 227 * 1024;
