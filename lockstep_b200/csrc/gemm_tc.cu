@@ -1776,6 +1776,7 @@ int run_rows(const void* X, const void* W, void* C, int c_dtype, int T, int N, i
   if ((ldx % 8) || ((uintptr_t)X & 15)) return LS_E_ALIGN;
   CUtensorMap mw, mx;
   const int ctas = rows_pairs ? 2 : 1;
+  // (up to 128 tokens in pairs too: single blocks with tiles of 128 took 3 to 20 % longer)
   // tiles of 256 features unless they would leave SMs without one (the tile's width changes no sum)
   const int tiles_t = (T + BM * ctas - 1) / (BM * ctas);
   const bool wide = epilogue != 2 && tiles_t * ((N + 255) / 256) * ctas >= sm_count();
@@ -1803,6 +1804,52 @@ int run_rows(const void* X, const void* W, void* C, int c_dtype, int T, int N, i
     return wide ? launch_rows_as<1, 256, float>(mw, mx, C, T, N, K, ldc, plan, err, stream)
                 : launch_rows_as<1, 128, float>(mw, mx, C, T, N, K, ldc, plan, err, stream);
   return LS_E_DTYPE;
+}
+
+// How many clusters of `shares` blocks with an SM's shared memory each the device runs at one time.
+int resident_clusters(int shares) {
+  static int known[MAX_SHARES + 1] = {};
+  if (known[shares] == 0) {
+    typedef __nv_bfloat16 bf16;
+    using S = ClusterShape<128, 0>;
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sm_count(), 1, shares);
+    cfg.blockDim = dim3(192);
+    cfg.dynamicSmemBytes = S::SMEM;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = shares;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    auto kernel = gemm_tc_cluster_kernel<128, 0, bf16, 8>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = sm_count() / shares;
+    }
+    known[shares] = n;
+  }
+  return known[shares];
+}
+
+// Whether 33 to 128 tokens of a product whose depth is shared out are better off with the tokens on the M side, one
+// tile of 256 on pairs of blocks that walk the whole depth, than in clusters (the bits are the same).  That walk takes 6 to
+// 7.5 us for a depth of 1,024, 10.5 for 2,048, 16 to 18 for 4,096, whatever the tokens; the clusters' time grows with the tokens, with fewer
+// shares (more columns to fold a block) and where they take a second round.  us, clusters / rows:
+//   depth 512, two shares: 64 tokens 10.4 / 5.8
+//   depth 1,024, 96 tokens: 4,096 features 8.6 / 7.4, 3,072 gated 11.3 / 10.7, 1,024 added 9.9 / 7.6; 64 tokens 6.8 / 7.3, 8.6 / 10.7, 7.1 / 7.4
+//   a second round of clusters of three: 6,144 features of 2,560 33 / 64 / 128 tokens 18.9 / 12.4, 20.2 / 12.4, 26.1 / 12.8; of 4,096 23.9 / 17.5 at
+//   33; 6,144 gated of 2,048 24.7 / 18.5 at 33
+//   a second round of clusters of seven and eight: 2,560 features of 4,096 16.6 / 17.1 at 64, 21.0 / 17.4 at 96; 2,048 of 2,048 11.5 / 11.3, 15.2 / 11.5;
+//   2,560 of 9,728 28.0 / 33.1 at 96
+//   one round of a deeper product: 1,024 of 2,048 8.0 / 10.8 at 96, 4,096 of 4,096 15.6 / 17.6
+bool rows_better(int T, int N, int K, const Plan& plan) {
+  if (T <= 32 || plan.shares < 2) return false;
+  if (K <= 512 || (T > 64 && K <= 1024)) return true;
+  return K <= 4096 && (T > 64 || plan.shares <= 3) && (N + BM - 1) / BM > resident_clusters(plan.shares);
 }
 
 // norm == nullptr: the token operand is read through `mx`; heads: the q/k/v epilogue's targets
@@ -1868,7 +1915,7 @@ int run(const void* X, const NormArgs* norm, const LsQkvStore* heads, const void
   const Plan plan = make_plan(T, N, K, epilogue);
   const int bn = plan.bn;
   if (epilogue == 3 && (!plan.in_cluster || bn > 32)) return LS_E_SIZE;    // before any work is done
-  if (T > 128) {
+  if (T > 128 || (norm == nullptr && epilogue != 3 && rows_better(T, N, K, plan))) {
     if (norm != nullptr || epilogue == 3) return LS_E_SIZE;
     return run_rows(X, W, C, c_dtype, T, N, K, ldx, ldw, ldc, epilogue, plan, err, stream);
   }

@@ -251,3 +251,27 @@ def test_qkv_heads_in_the_product_decline_what_they_do_not_cover():
     shallow = torch.zeros((nq + 2 * nkv) * d, 128, dtype=torch.bfloat16, device=dev())
     assert K.library("tc").ls_gemm_tc_k_shares(shallow.shape[0], 128) == 1
     assert not call(8, w_=shallow)
+
+
+@pytest.mark.parametrize("n,k", [(6144, 2560), (1024, 512), (4096, 1024), (2048, 2048), (1000, 1024), (2560, 4096)])
+def test_rows_of_33_to_128_tokens_have_the_same_bits_on_either_side_of_the_rules(n, k):
+    """Products that go to the kernel with the tokens as rows below 129 tokens, some from 33 and some from 65 on, and to clusters
+    before that: a row's bits are those of the same row among 300."""
+    from lockstep_b200 import kernels as K
+
+    g = torch.Generator(device=dev()).manual_seed(n + k)
+    x = torch.randn(300, k, generator=g, device=dev()).to(torch.bfloat16)
+    w = (torch.randn(2 * n, k, generator=g, device=dev()) * 0.1).to(torch.bfloat16)
+    old = torch.randn(300, n, generator=g, device=dev())
+    err, ran = K.new_error_word(dev()), set()
+    for code, weight, kind in ((K.EPILOGUE_STORE, w[:n].contiguous(), torch.bfloat16), (K.EPILOGUE_RESIDUAL, w[:n].contiguous(), torch.float32),
+                               (K.EPILOGUE_SILU_MUL, w, torch.bfloat16), (K.EPILOGUE_GELU, w[:n].contiguous(), torch.bfloat16)):
+        full = old.to(kind)
+        assert K.gemm_nt_tc(x, weight, full, code, err)
+        for t in (32, 33, 64, 65, 100, 128):
+            part, before = old[:t].to(kind), K.kernel_counts()
+            assert K.gemm_nt_tc(x[:t].contiguous(), weight, part, code, err)
+            ran |= {(t, name) for name, count in K.kernel_counts().items() if count > before.get(name, 0)}
+            assert torch.equal(part, full[:t]), (code, t)
+    K.raise_on_fault(err)
+    assert (128, "gemm_tc_rows_pair") in ran and (32, "gemm_tc_rows_pair") not in ran
