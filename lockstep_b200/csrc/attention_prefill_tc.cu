@@ -173,7 +173,8 @@ struct Item {
 //
 // What bounds it: MMAs (1,024 cycles a tile of 128 x 128 with d = 128), exponentials (1,024 on the special-function
 // units), shared memory (160 KB a tile at 128 bytes a cycle) and L2 (64 KB a tile an SM) have to run side by side; a tile
-// takes about 1,800 cycles, paced by the arrival of keys and values.  Measured, 16 query and 8 key heads of 128, pages of 16, with a
+// takes about 1,850 cycles, paced by S and PV one after the other and the issuing warp's waits between them (tensor pipe and
+// special-function units half busy, L2 a quarter; a third stage of values changes nothing).  Measured, 16 query and 8 key heads of 128, pages of 16, with a
 // head a block and four threads a row / two heads a block / now: 2,048 tokens 30.0 / - / 25.1 us, 2,048 after
 // 6,144 148.8 / 148.4 / 113.6 us, 8,192 - / 276 / 244 us (1,126 TFLOP/s).
 // Two teams on different tiles, with no chain between a tile's softmax and the next tile's S.  A row's sums need one
