@@ -8,7 +8,7 @@
 //   S = Q K^T     tcgen05.mma, Q [128 x d] and the key tile [128 x d] K-major in
 //                 shared memory (TMA, 128-byte swizzle), S in tensor memory
 //   softmax       a thread reads its row's 128 scores from S with tcgen05.ld: maximum,
-//                 p = exp2(s * scale * log2 e - m_ref), the running sum l in registers; P
+//                 p = exp2(s * scale * log2 e - m_ref), the sums of p over the tile's quarters; P
 //                 rounded to bfloat16 goes back to tensor memory (tcgen05.st), two keys a column,
 //                 over the scores it came from
 //   PV            tcgen05.mma with P [128 x 128] as the A operand in tensor memory and the
@@ -175,12 +175,16 @@ struct Item {
 // units), shared memory (160 KB a tile at 128 bytes a cycle) and L2 (64 KB a tile an SM) have to run side by side; a tile
 // takes about 1,850 cycles, paced by S and PV one after the other and the issuing warp's waits between them (tensor pipe and
 // special-function units half busy, L2 a quarter; a third stage of values changes nothing).  Measured, 16 query and 8 key heads of 128, pages of 16, with a
-// head a block and four threads a row / two heads a block / now: 2,048 tokens 30.0 / - / 25.1 us, 2,048 after
-// 6,144 148.8 / 148.4 / 113.6 us, 8,192 - / 276 / 244 us (1,126 TFLOP/s).
+// head a block and four threads a row (two heads a block for the last two) / now: 2,048 tokens 30.5 / 25.9 us, 2,048 after
+// 6,144 149.7 / 116.1 us, 8,192 277 / 248 us (1,110 TFLOP/s).
 // Two teams on different tiles, with no chain between a tile's softmax and the next tile's S.  A row's sums need one
 // order: m_ref of a row goes from team to team with the tiles (through shared memory and a named barrier of the two
-// warps that share the row's quarter of tensor memory, before the exponentials are taken), O is one accumulator and each
-// team keeps the sum l of its own tiles, which the team that has the item's last tile adds up.
+// warps that share the row's quarter of tensor memory, before the exponentials are taken), and O is one accumulator.  The sum
+// l of a row is four chains over the tiles, one of each quarter of a tile's keys (32), added in order at the end: a wholly
+// masked tile changes none of them, so l does not depend on where the row's item begins.  The chains go from team to team with m_ref: at
+// tile t a team gets them through tile t - 3, adds its own tile t - 2 and passes them on, so that none waits for exponentials; the team
+// with the item's last tile adds the last two.  (With a sum of its own tiles a team, 2,048 tokens took 25.6 us and 8,192 245.8, now
+// 25.9 and 247.7, but a row's bits depended on the parity of its tiles in the item.)
 //
 // EXTRAS: the scores may get a bias that grows with the logarithm of the distance of key and query taken
 // off (slopes[head] x ln(1 + log_rates[head] x distance): in the units of the exponentials,
@@ -219,11 +223,13 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   uint64_t* p_full = bars + 13;        // [3] P of a tile is in tensor memory
   uint64_t* o_full = bars + 16;        // [2] PV of a tile has been added to O (and has read its values)
   uint64_t* o_free = bars + 18;        // the item's O has been read
-  uint64_t* l_full = bars + 19;        // [4] the sums of the team without the item's last tile
+  uint64_t* l_full = bars + 19;        // [4] the sums of the item's last tile but one lie in shared memory
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 23);
   volatile uint32_t* failed = tmem_slot + 1;
   float* hand_m = reinterpret_cast<float*>(bars + 32);   // [2 teams][128 rows] m_ref after a team's tile
-  float* hand_l = hand_m + 2 * 128;                      // [4][128 rows] sums handed over at an item's end
+  float4* hand_l = reinterpret_cast<float4*>(hand_m + 2 * 128);   // [2 teams][128 rows] the sums of weights through the tile two before
+  float4* end_s = hand_l + 2 * 128;                      // [4][128 rows] the sums of an item's last tile but one
+  float* end_f = reinterpret_cast<float*>(end_s + 4 * 128);       // [4][128 rows] and its rescaling
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int total_items = n_work * nq;
@@ -335,9 +341,13 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       const int pos = pos0 + row;
       const int lo = ls_first_key(pos, window);
       const int lo_last = ls_first_key(pos_last, window);
-      // m_ref: the row's, as this team knows it; l_run: the sum over this team's tiles, in its units;
-      // m_before: m_ref before the item's last tile, in whose units the other team hands its sum over
-      float m_ref = -CUDART_INF_F, l_run = 0.f, m_before = -CUDART_INF_F;
+      // m_ref: the row's, as this team knows it; quarter, factor: the sums of weights of this team's last tile, a sum a quarter
+      // of its keys, and the tile's rescaling
+      float m_ref = -CUDART_INF_F, factor = 1.f;
+      float4 quarter = make_float4(0.f, 0.f, 0.f, 0.f);
+      auto chained = [](float4 l, float f, float4 s) {
+        return make_float4(fmaf(l.x, f, s.x), fmaf(l.y, f, s.y), fmaf(l.z, f, s.z), fmaf(l.w, f, s.w));
+      };
       float bias_a = 0.f, bias_b = 0.f;
       bool biased = false, linear = false;
       if constexpr (EXTRAS) {
@@ -419,16 +429,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         // m_ref after the tile before, from the other team (an item's first tile meets it too, for the
         // barrier's sake: a team may not announce two tiles before the other has taken the first)
         if (g > 0) asm volatile("bar.sync %0, 64;" ::"r"(1 + quad * 2 + ((g - 1) & 1)) : "memory");
-        if (it > 0) {
-          const float m_prev = hand_m[((g - 1) & 1) * 128 + row];
-          // (m_ref is -inf before the first key a row sees; l_run is 0 then)
-          if (m_prev != m_ref) l_run *= m_ref == -CUDART_INF_F ? 0.f : ex2(m_ref - m_prev);
-          m_ref = m_prev;
-        }
-        m_before = m_ref;
+        if (it > 0) m_ref = hand_m[((g - 1) & 1) * 128 + row];
         const float m_new = tile_max * scale_eff;
         const bool move = m_new > m_ref + LAZY;                      // true too for the first key a row sees
-        const float factor = move ? ((m_ref == -CUDART_INF_F) ? 0.f : ex2(m_ref - m_new)) : 1.f;
+        // the chains through the other team's tile before the last come with m_ref, this team's last tile is added
+        if (it > 1)
+          hand_l[(g & 1) * 128 + row] =
+              chained(it > 2 ? hand_l[((g - 1) & 1) * 128 + row] : make_float4(0.f, 0.f, 0.f, 0.f), factor, quarter);
+        factor = move ? ((m_ref == -CUDART_INF_F) ? 0.f : ex2(m_ref - m_new)) : 1.f;
         if (move) m_ref = m_new;
         hand_m[(g & 1) * 128 + row] = m_ref;
         asm volatile("bar.arrive %0, 64;" ::"r"(1 + quad * 2 + (g & 1)) : "memory");
@@ -450,14 +458,15 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           }
         }
         // p = exp2(s * scale - m_ref), rounded to bfloat16, two keys a column, written over scores this
-        // thread has taken, from where the PV product takes it as its A operand; the sum in four
-        // running sums, folded in a fixed order
-        float ps[4] = {0.f, 0.f, 0.f, 0.f};
+        // thread has taken, from where the PV product takes it as its A operand; the sum of a quarter of the tile's keys
+        // in four running sums, folded in a fixed order
+        float sum[4];
         const bool dead = m_ref == -CUDART_INF_F;          // nothing seen yet by this row
         const float add = dead ? 0.f : -m_ref;
 #pragma unroll
         for (int n0 = 0; n0 < BLOCK_N; n0 += 32) {
           uint32_t pk[16];
+          float ps[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
           for (int jj = 0; jj < 32; jj += 4) {
             float p[4];
@@ -473,9 +482,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             pk[(jj >> 1) + 1] = pack_bf16(p[2], p[3]);
           }
           tmem_st16(s_addr + (n0 >> 1), pk);
+          sum[n0 / 32] = (ps[0] + ps[1]) + (ps[2] + ps[3]);
         }
-        float psum = (ps[0] + ps[1]) + (ps[2] + ps[3]);
-        if (__any_sync(0xffffffffu, dead && psum != 0.f)) {
+        if (__any_sync(0xffffffffu, dead && (sum[0] + sum[1]) + (sum[2] + sum[3]) != 0.f)) {
           // (a row that has seen scores that are no numbers and nothing else weighs nothing)
           tmem_st_wait();
 #pragma unroll
@@ -487,7 +496,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             for (int e = 0; e < 32; ++e) pk[e] = dead ? 0u : pk[e];
             tmem_st32(s_addr + c, pk);
           }
-          if (dead) psum = 0.f;
+          if (dead) sum[0] = sum[1] = sum[2] = sum[3] = 0.f;
         }
         // value rows of keys past the last position were never written: they must not be NaN,
         // since P is zero there and the MMA multiplies all the same
@@ -506,27 +515,28 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         fence_before_sync();
         __syncwarp();
         if (lane == 0 && ok) mbar_arrive(p_bar);
-        l_run = fmaf(l_run, factor, psum);
+        quarter = make_float4(sum[0], sum[1], sum[2], sum[3]);
       }
-      // ---- the item's end: the team that had the last tile takes the other's sum and writes the
-      // rows out, while the other goes on to the next item ----
+      // ---- the item's end: the team that had the last tile takes what the other had of the tile before and writes
+      // the rows out, while the other goes on to the next item ----
       const int g_last = gt + n_tiles - 1;
       const int lb = shared_items & 3;
       const uint32_t l_par = (uint32_t)(shared_items >> 2) & 1u;
       if ((g_last & 1) != team) {
         if (n_tiles > 1) {
-          hand_l[lb * 128 + row] = l_run;
+          end_s[lb * 128 + row] = quarter;
+          end_f[lb * 128 + row] = factor;
           __syncwarp();
           if (lane == 0) mbar_arrive(&l_full[lb]);
         }
       } else {
-        float l_row = l_run;
+        float4 l = n_tiles > 2 ? hand_l[(g_last & 1) * 128 + row] : make_float4(0.f, 0.f, 0.f, 0.f);
         if (n_tiles > 1) {
           if (ok && !mbar_wait(&l_full[lb], l_par)) ok = false;
-          // (rounded one by one: the same sum whichever team has the last tile)
-          if (m_before != -CUDART_INF_F)
-            l_row = __fadd_rn(__fmul_rn(hand_l[lb * 128 + row], ex2(m_before - m_ref)), l_row);
+          l = chained(l, end_f[lb * 128 + row], end_s[lb * 128 + row]);
         }
+        l = chained(l, factor, quarter);
+        float l_row = ((l.x + l.y) + l.z) + l.w;
         if constexpr (EXTRAS) {
           // the sink, in the units of this row's sums (2^m_ref)
           if (sinks != nullptr && m_ref != -CUDART_INF_F) l_row += ex2(fmaf(sinks[I.h], 1.4426950408889634f, -m_ref));
@@ -813,7 +823,7 @@ int launch(const CUtensorMap& map_q, const CUtensorMap& map_kv, void* out, const
            const int* block_table, int table_stride, int nq, int nkv, int page_size, int num_pages, int window,
            int keep_first, float scale, const float* slopes, const float* log_rates, const float* sinks, float softcap,
            int* err, cudaStream_t stream) {
-  constexpr size_t smem = (size_t)HALVES * HALF_BYTES * 3 * STAGES + 256 + 6 * 128 * 4 + 1024;
+  constexpr size_t smem = (size_t)HALVES * HALF_BYTES * 3 * STAGES + 256 + (2 + 2 * 4 + 4 * 5) * 128 * 4 + 1024;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(attention_prefill_tc_kernel<HALVES, EXTRAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -392,6 +392,117 @@ def test_wide_rows_normed_inside_a_product_of_few_blocks_have_the_bits_of_the_ke
     k.raise_on_fault(err)
 
 
+# ---------------------------------------------------------------------------
+# bfloat16 attention of prompt portions on the tensor cores
+# ---------------------------------------------------------------------------
+
+class Prompt:
+    """Requests of bfloat16 queries, keys and values in a shuffled cache, and the kernel over portions of them."""
+
+    def __init__(self, nq, nkv, d, page, lengths, mask=0, extra=None, seed=0):
+        from lockstep_b200.engine.batch import mask_parts
+
+        g = torch.Generator().manual_seed(seed + nq + d)
+        self.nq, self.nkv, self.d, self.mask, self.lengths = nq, nkv, d, mask, lengths
+        self.window, self.keep = mask_parts(mask)
+        self.scale = d ** -0.5
+        self.q = [torch.randn(n, nq, d, generator=g).bfloat16() for n in lengths]
+        self.k, self.v = ([torch.randn(n, nkv, d, generator=g).bfloat16() for n in lengths] for _ in range(2))
+        count = [-(-n // page) for n in lengths]
+        ids, at = torch.randperm(sum(count), generator=g).to(torch.int32), 0
+        self.table = torch.zeros(len(lengths), max(count), dtype=torch.int32)
+        pages = torch.full((sum(count), 2, nkv, page, d), math.nan).bfloat16()        # behind a request's end: never written
+        for r, n in enumerate(lengths):
+            self.table[r, :count[r]] = ids[at:at + count[r]]
+            at += count[r]
+            for which, rows in ((0, self.k[r]), (1, self.v[r])):
+                key = torch.arange(n)
+                pages[self.table[r, key // page].long(), which, :, key % page] = rows
+        self.pages, self.table = pages.to(dev()), self.table.to(dev())
+        self.slopes = self.rates = self.sinks = None
+        self.cap = 4.0 if extra == "cap" else 0.0
+        if extra in ("linear", "log"):
+            self.slopes = torch.rand(nq, generator=g) * 0.2
+        if extra == "log":
+            self.rates = torch.rand(nq, generator=g)
+        if extra == "sinks":
+            self.sinks = torch.randn(nq, generator=g)
+
+    def run(self, portions):
+        """portions (request, start, tokens), two tokens at least; the rows of each, [tokens, nq, d]."""
+        from lockstep_b200.engine.batch import plan_attention
+
+        k = K()
+        rows, off = [], 0
+        for r, start, n in portions:
+            rows.append((r, off, start, n))
+            off += n
+        q = torch.cat([self.q[r][start:start + n] for r, start, n in portions]).view(off, -1).to(dev())
+        tile = plan_attention(rows, self.mask, k.attention_split_size(), k.attention_prefill_tc_tile_tokens())[0]
+        out, err = torch.full_like(q, math.nan), k.new_error_word(dev())
+        on = lambda t: None if t is None else t.to(dev())
+        assert k.attention_prefill_tc(q, self.pages, out, torch.from_numpy(tile).to(dev()), len(tile), self.table, self.nq,
+                                      self.nkv, self.d, self.window, self.scale, err, on(self.slopes), on(self.rates),
+                                      on(self.sinks), softcap=self.cap, keep_first=self.keep)
+        k.raise_on_fault(err)
+        return [x.view(-1, self.nq, self.d) for x in out.cpu().split([n for _, _, n in portions])]
+
+    def plain(self, r):
+        from lockstep_b200.engine.batch import first_key
+
+        n = self.lengths[r]
+        pos = np.arange(n)
+        seen = (pos[None, :] <= pos[:, None]) & ((pos[None, :] >= first_key(pos, self.window)[:, None]) | (pos[None, :] < self.keep))
+        away = torch.from_numpy(np.maximum(pos[:, None] - pos[None, :], 0)).double()
+        want = torch.empty(n, self.nq, self.d, dtype=torch.float64)
+        for h in range(self.nq):
+            kv = h // (self.nq // self.nkv)
+            s = self.q[r][:, h].double() @ self.k[r][:, kv].double().T * self.scale
+            if self.cap:
+                s = self.cap * torch.tanh(s / self.cap)
+            if self.rates is not None:
+                s = s - self.slopes[h].double() * torch.log1p(self.rates[h].double() * away)
+            elif self.slopes is not None:
+                s = s - self.slopes[h].double() * away
+            s = s.masked_fill(~torch.from_numpy(seen), -math.inf)
+            if self.sinks is not None:
+                s = torch.cat([s, self.sinks[h].double().expand(n, 1)], 1)
+            want[:, h] = torch.softmax(s, 1)[:, :n] @ self.v[r][:, kv].double()
+        return want
+
+
+@pytest.mark.parametrize("extra", [None, "sinks", "log", "linear", "cap"])
+@pytest.mark.parametrize("nq,nkv,d,page,mask", [(4, 2, 128, 16, 0), (2, 1, 64, 8, 300), (2, 2, 128, 128, (500, 4)), (4, 1, 64, 32, (300, 200)),
+                                                (2, 1, 128, 64, (130, 129)), (2, 1, 128, 16, -200)])
+def test_a_bfloat16_row_of_a_prompt_has_the_same_bits_however_it_is_cut(nq, nkv, d, page, mask, extra):
+    """A prompt of 1,500 tokens whole, and from 0, 1, 37 and 127 tokens past the edges of two neighbouring tiles on, with
+    windows, chunks and kept first keys: the tile that a row's item begins with is another one each time, and a row has the same bits.
+    Values against float64: P and the result are rounded to 2^-9 of themselves, of values up to 4.5."""
+    prompt = Prompt(nq, nkv, d, page, [1500], mask, extra)
+    whole = prompt.run([(0, 0, 1500)])[0]
+    assert (whole.double() - prompt.plain(0)).abs().max() <= 2e-2
+    for edge in (1024, 1152):
+        for past in (0, 1, 37, 127):
+            start = edge + past
+            assert torch.equal(prompt.run([(0, start, 1500 - start)])[0], whole[start:]), start
+    assert torch.equal(prompt.run([(0, 700, 2)])[0], whole[700:702])
+
+
+@pytest.mark.parametrize("nq,nkv,d,mask,extra", [(16, 8, 128, 0, None), (8, 2, 64, (100, 4), None), (16, 4, 128, 90, "log"), (8, 8, 64, 0, "cap")])
+def test_many_short_portions_have_the_rows_of_each_alone(nq, nkv, d, mask, extra):
+    """Sixty requests with portions of one, two and three tiles of keys: several items a block, so that a block's items end in
+    either team's tile and hand over their places in shared and tensor memory one after the other."""
+    lengths = [(37, 128, 129, 200, 257, 300, 384, 2, 90, 250)[i % 10] for i in range(60)]
+    starts = [(0, 1, 100, 0)[i % 4] for i in range(60)]
+    portions = [(i, s, n - s) for i, (s, n) in enumerate(zip(starts, lengths)) if n - s > 1]
+    prompt = Prompt(nq, nkv, d, 16, lengths, mask, extra, seed=3)
+    together = prompt.run(portions)
+    for (r, start, n), rows in zip(portions, together):
+        if r < 10 or r % 7 == 0:
+            assert (rows.double() - prompt.plain(r)[start:]).abs().max() <= 2e-2, r
+            assert torch.equal(rows, prompt.run([(r, start, n)])[0]), r
+
+
 @pytest.mark.parametrize("nq,nkv,d,page,mask", [(4, 2, 128, 16, 0), (3, 3, 16, 8, 0), (8, 2, 64, 64, 100), (8, 1, 128, 32, (300, 40)),
                                                 (2, 1, 112, 16, -96), (4, 4, 128, 128, 0)])
 def test_float32_splits_of_single_tokens_have_the_bits_of_the_tile_kernel(nq, nkv, d, page, mask):
