@@ -40,6 +40,14 @@ constexpr int HALF_BYTES = 128 * 128;     // 128 rows of 64 elements
 constexpr uint32_t TMEM_COLS = 512;
 constexpr int MMA_WARP = 0, K_WARP = 1, V_WARP = 2, TEAM_WARP = 4;
 constexpr int THREADS = 12 * 32;
+// Instances, so that none keeps registers for another's terms: plain scores; first keys that stay visible or sinks; a logarithmic bias; a
+// linear bias, a cap or a scale that is not above 0 (times which -inf is not what a masked score is to be).  The last two take kept
+// keys and sinks as well.
+enum { PLAIN, KEPT_OR_SINK, LOG_BIAS, LINEAR_OR_CAP };
+template <int V>
+struct Kind {
+  static constexpr int value = V;
+};
 
 // A key or value tile lies in groups of 8 keys, a group as its halves of 64 elements, a half as 8
 // rows of 128 bytes (128-byte swizzle): what one TMA box of a page leaves (see encode_pages).
@@ -186,14 +194,14 @@ struct Item {
 // with the item's last tile adds the last two.  (With a sum of its own tiles a team, 2,048 tokens took 25.6 us and 8,192 245.8, now
 // 25.9 and 247.7, but a row's bits depended on the parity of its tiles in the item.)
 //
-// EXTRAS: the scores may get a bias that grows with the logarithm of the distance of key and query taken
+// KIND beyond PLAIN: the scores may get a bias that grows with the logarithm of the distance of key and query taken
 // off (slopes[head] x ln(1 + log_rates[head] x distance): in the units of the exponentials,
 // slopes[head] x lg2(1 + log_rates[head] x distance), one more special-function instruction a score),
 // and the softmax's denominator one more term exp(sinks[head]) at the end of a row.  With slopes and no log_rates the
 // bias is slopes[head] x distance, and with cap_log2 > 0 (a cap times lg2 e) the scaled score first becomes
 // cap tanh(score / cap), again in the units of the exponentials.  keep_first > 0: the first
 // keep_first keys of the sequence stay visible behind the window; their tiles come first.
-template <int HALVES, bool EXTRAS>
+template <int HALVES, int KIND>
 __global__ void __launch_bounds__(THREADS, 1)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                             __nv_bfloat16* __restrict__ out, const int* __restrict__ work, int n_work,
@@ -201,6 +209,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             int num_pages, int window, int keep_first, float scale_log2, const float* __restrict__ slopes,
                             const float* __restrict__ log_rates, const float* __restrict__ sinks, float cap_log2, int* err) {
   ls_dependency_trigger();
+  constexpr bool EXTRAS = KIND != PLAIN, BIASED = KIND == LOG_BIAS || KIND == LINEAR_OR_CAP;
   constexpr int D = HALVES * 64;
   constexpr int TILE_BYTES = HALVES * HALF_BYTES;        // K or V of one tile; also Q of one item
   constexpr int GROUP_BYTES = HALVES * 1024;             // 8 keys of a tile
@@ -349,21 +358,15 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         return make_float4(fmaf(l.x, f, s.x), fmaf(l.y, f, s.y), fmaf(l.z, f, s.z), fmaf(l.w, f, s.w));
       };
       float bias_a = 0.f, bias_b = 0.f;
-      bool biased = false, linear = false;
-      if constexpr (EXTRAS) {
-        if (log_rates != nullptr) {
-          bias_a = slopes[I.h];
-          bias_b = log_rates[I.h];
-          biased = true;
-        } else if (slopes != nullptr || cap_log2 > 0.f || !(scale_log2 > 0.f)) {
-          bias_a = slopes != nullptr ? slopes[I.h] * 1.4426950408889634f : 0.f;      // the slope in the exponentials' units
-          bias_b = cap_log2 > 0.f ? scale_log2 / cap_log2 : 0.f;                     // score -> score x scale / cap
-          biased = linear = true;
-        }
+      if constexpr (KIND == LOG_BIAS) {
+        bias_a = slopes[I.h];
+        bias_b = log_rates[I.h];
+      } else if constexpr (KIND == LINEAR_OR_CAP) {
+        bias_a = slopes != nullptr ? slopes[I.h] * 1.4426950408889634f : 0.f;      // the slope in the exponentials' units
+        bias_b = cap_log2 > 0.f ? scale_log2 / cap_log2 : 0.f;                     // score -> score x scale / cap
       }
-      // (a scale that is not above 0 too, since -inf times it is not what a masked score is to be;)
       // with a bias the scores are put into the exponentials' units as they are read, and no scale is left
-      const float scale_eff = biased ? 1.0f : scale_log2;
+      const float scale_eff = BIASED ? 1.0f : scale_log2;
       for (int it = 0; it < n_tiles; ++it) {
         const int g = gt + it;
         const uint32_t s_addr = lane_base + (uint32_t)(s_tile * BLOCK_N);
@@ -378,47 +381,71 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         const int c0 = I.tile(it) * BLOCK_N;                         // first key of the tile
         if (ok && !mbar_wait(s_bar, s_par)) ok = false;
         fence_after_sync();
+        // every key of the tile is seen by every row: no masks (uniform over the block); elsewhere a masked score
+        // becomes -inf (selects and not branches), whose exponential is 0
+        const bool full_tile = c0 + BLOCK_N - 1 <= pos0 && (c0 >= lo_last || c0 + BLOCK_N <= kept);
+        if constexpr (BIASED) {
+          // Bias and masks go over the scores in tensor memory, 32 at a time in a loop.  Unrolled over a row's 128 registers they are four
+          // times the code, which a launch of a tile or two mostly fetches, and registers spilled (one instance for every bias).
+          // 16 query and 8 key heads, us, that / this / four threads a row as it was before there were teams: logarithmic 2,048 tokens
+          // 41.8 / 36.6 / 41.3, 2,048 after 6,144 in a window of 512 39.7 / 30.3 / 35.5; a cap 53.1 / 45.9 / 52.6; linear 46.0 / 38.2 / 39.4.
+          // (A prompt of 25 tokens and two more in the 2,048 wide Malazen design: 1.31 / 1.26 / 1.27 ms.)
+#pragma unroll 1
+          for (int q0 = 0; q0 < BLOCK_N; q0 += 32) {
+            uint32_t x[32];
+            tmem_ld32(s_addr + q0, x);
+            tmem_ld_wait();
+            const int c = c0 + q0;
+            const float d0 = (float)(pos - c);           // distance of the piece's first key (masked keys: clamped)
+            if constexpr (KIND == LOG_BIAS) {
+#pragma unroll
+              for (int jj = 0; jj < 32; ++jj)
+                x[jj] = __float_as_uint(fmaf(__uint_as_float(x[jj]), scale_log2, -bias_a * lg2(fmaf(bias_b, fmaxf(d0 - (float)jj, 0.f), 1.0f))));
+            } else if (cap_log2 > 0.f) {
+#pragma unroll
+              for (int jj = 0; jj < 32; ++jj)
+                x[jj] = __float_as_uint(fmaf(-bias_a, fmaxf(d0 - (float)jj, 0.f), cap_log2 * tanh_of(__uint_as_float(x[jj]) * bias_b)));
+            } else {
+#pragma unroll
+              for (int jj = 0; jj < 32; ++jj)
+                x[jj] = __float_as_uint(fmaf(-bias_a, fmaxf(d0 - (float)jj, 0.f), __uint_as_float(x[jj]) * scale_log2));
+            }
+            if (!full_tile) {
+              const int after = pos - c;                             // the last place of the piece that the row sees
+              const int from = kept > c ? kept - c : 0;              // between the kept keys and the window
+              const uint32_t gap = lo - c > from ? (uint32_t)(lo - c - from) : 0u;
+#pragma unroll
+              for (int jj = 0; jj < 32; ++jj) x[jj] = (uint32_t)(jj - from) < gap ? __float_as_uint(-CUDART_INF_F) : x[jj];
+#pragma unroll
+              for (int jj = 0; jj < 32; ++jj) x[jj] = jj <= after ? x[jj] : __float_as_uint(-CUDART_INF_F);
+            }
+            tmem_st32(s_addr + q0, x);
+          }
+          tmem_st_wait();
+        }
         uint32_t sc[BLOCK_N];
 #pragma unroll
         for (int q0 = 0; q0 < BLOCK_N; q0 += 32) tmem_ld32(s_addr + q0, sc + q0);
         tmem_ld_wait();
-        if constexpr (EXTRAS) {
-          if (biased && linear) {
-            const float d0 = (float)(pos - c0);
-            const bool capped = cap_log2 > 0.f;
-#pragma unroll
-            for (int jj = 0; jj < BLOCK_N; ++jj) {
-              const float dist = fmaxf(d0 - (float)jj, 0.f);
-              const float raw = __uint_as_float(sc[jj]);
-              const float v = capped ? cap_log2 * tanh_of(raw * bias_b) : raw * scale_log2;
-              sc[jj] = __float_as_uint(fmaf(-bias_a, dist, v));
-            }
-          } else if (biased) {
-            const float d0 = (float)(pos - c0);        // distance of the tile's first key (masked keys: clamped)
-#pragma unroll
-            for (int jj = 0; jj < BLOCK_N; ++jj) {
-              const float dist = fmaxf(d0 - (float)jj, 0.f);
-              sc[jj] = __float_as_uint(fmaf(__uint_as_float(sc[jj]), scale_log2, -bias_a * lg2(fmaf(bias_b, dist, 1.0f))));
-            }
-          }
-        }
-        // every key of the tile is seen by every row: no masks (uniform over the block); elsewhere a masked score
-        // becomes -inf (selects and not branches), whose exponential is 0
-        const bool full_tile = c0 + BLOCK_N - 1 <= pos0 && (c0 >= lo_last || c0 + BLOCK_N <= kept);
-        if (!full_tile) {
-          // (a key's place is kept where place - first < count, as unsigned numbers)
-          const int first = lo - c0 > 0 ? lo - c0 : 0;
-          const uint32_t count = pos - c0 - first + 1 > 0 ? (uint32_t)(pos - c0 - first + 1) : 0u;
+        if (!BIASED && !full_tile) {
+          const int after = pos - c0;                                // the last place of the tile that the row sees
+          const int first = lo - c0;                                 // the first within its window
           if (c0 >= lo_last) {                                       // no window within the tile: the diagonal alone
 #pragma unroll
-            for (int jj = 0; jj < BLOCK_N; ++jj) sc[jj] = jj <= pos - c0 ? sc[jj] : __float_as_uint(-CUDART_INF_F);
-          } else {
-            const int lead = EXTRAS ? min(kept - c0, pos - c0 + 1) : 0;
+            for (int jj = 0; jj < BLOCK_N; ++jj) sc[jj] = jj <= after ? sc[jj] : __float_as_uint(-CUDART_INF_F);
+          } else if (EXTRAS && c0 < kept) {
+            // between the kept keys and the window, then the diagonal (one condition for both took registers for 128 predicates)
+            const int from = kept - c0;
+            const uint32_t gap = first > from ? (uint32_t)(first - from) : 0u;
 #pragma unroll
-            for (int jj = 0; jj < BLOCK_N; ++jj) {
-              const bool seen = (uint32_t)(jj - first) < count || (EXTRAS && jj < lead);
-              sc[jj] = seen ? sc[jj] : __float_as_uint(-CUDART_INF_F);
-            }
+            for (int jj = 0; jj < BLOCK_N; ++jj) sc[jj] = (uint32_t)(jj - from) < gap ? __float_as_uint(-CUDART_INF_F) : sc[jj];
+#pragma unroll
+            for (int jj = 0; jj < BLOCK_N; ++jj) sc[jj] = jj <= after ? sc[jj] : __float_as_uint(-CUDART_INF_F);
+          } else {
+#pragma unroll
+            for (int jj = 0; jj < BLOCK_N; ++jj) sc[jj] = jj >= first ? sc[jj] : __float_as_uint(-CUDART_INF_F);
+#pragma unroll
+            for (int jj = 0; jj < BLOCK_N; ++jj) sc[jj] = jj <= after ? sc[jj] : __float_as_uint(-CUDART_INF_F);
           }
         }
         float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
@@ -818,7 +845,7 @@ int sm_count() {
   return sms;
 }
 
-template <int HALVES, bool EXTRAS>
+template <int HALVES, int KIND>
 int launch(const CUtensorMap& map_q, const CUtensorMap& map_kv, void* out, const int* work, int n_work,
            const int* block_table, int table_stride, int nq, int nkv, int page_size, int num_pages, int window,
            int keep_first, float scale, const float* slopes, const float* log_rates, const float* sinks, float softcap,
@@ -826,7 +853,7 @@ int launch(const CUtensorMap& map_q, const CUtensorMap& map_kv, void* out, const
   constexpr size_t smem = (size_t)HALVES * HALF_BYTES * 3 * STAGES + 256 + (2 + 2 * 4 + 4 * 5) * 128 * 4 + 1024;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<HALVES, EXTRAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<HALVES, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess)
       return LS_E_SMEM;
     configured = true;
@@ -834,7 +861,7 @@ int launch(const CUtensorMap& map_q, const CUtensorMap& map_kv, void* out, const
   // a block per SM (its shared memory and its 512 columns of tensor memory fill one), or fewer items
   const long long items = (long long)n_work * nq;
   const int blocks = items < sm_count() ? (int)items : sm_count();
-  LS_COUNT(LS_K_ATTENTION_PREFILL_TC), ls_launch(attention_prefill_tc_kernel<HALVES, EXTRAS>, dim3(blocks), THREADS, smem, stream, map_q, map_kv,
+  LS_COUNT(LS_K_ATTENTION_PREFILL_TC), ls_launch(attention_prefill_tc_kernel<HALVES, KIND>, dim3(blocks), THREADS, smem, stream, map_q, map_kv,
             (__nv_bfloat16*)out, work, n_work, block_table, table_stride, nq, nkv, page_size, num_pages, window,
             keep_first, scale * 1.4426950408889634f, slopes, log_rates, sinks, softcap > 0.f ? softcap * 1.4426950408889634f : 0.f, err);
   return ls_launch_status();
@@ -867,9 +894,10 @@ LS_API int ls_attention_prefill_tc(const void* q, const void* pages, void* out, 
   CUtensorMap map_q, map_kv;
   if (!encode(&map_q, q, (uint64_t)nq * d, (uint64_t)tokens, BLOCK_M)) return LS_E_SIZE;
   if (!encode_pages(&map_kv, pages, (uint64_t)d / 64, (uint64_t)rows, page_size < BLOCK_N ? page_size : BLOCK_N)) return LS_E_SIZE;
-  // a bias on the scores, a cap, a sink, kept first keys or a scale that is not above 0: an instance of its own, so that the other keeps no branch for them
-  const bool extras = slopes != nullptr || sinks != nullptr || softcap > 0.f || keep_first > 0 || !(scale > 0.f);
-  auto go = d == 64 ? (extras ? launch<1, true> : launch<1, false>) : (extras ? launch<2, true> : launch<2, false>);
+  auto of = [&](auto kind) { return d == 64 ? launch<1, decltype(kind)::value> : launch<2, decltype(kind)::value>; };
+  auto go = log_rates != nullptr ? of(Kind<LOG_BIAS>())
+            : slopes != nullptr || softcap > 0.f || !(scale > 0.f) ? of(Kind<LINEAR_OR_CAP>())
+            : sinks != nullptr || keep_first > 0 ? of(Kind<KEPT_OR_SINK>()) : of(Kind<PLAIN>());
   return go(map_q, map_kv, out, work, n_work, block_table, table_stride, nq, nkv, page_size, num_pages, window,
             keep_first, scale, slopes, log_rates, sinks, softcap, err, stream);
 }
