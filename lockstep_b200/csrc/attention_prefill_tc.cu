@@ -870,8 +870,6 @@ int launch(const CUtensorMap& map_q, const CUtensorMap& map_kv, void* out, const
 }  // namespace
 
 LS_API int ls_attention_prefill_tc_tile_tokens() { return BLOCK_M; }
-// (a choice between kernels of one and of two heads a block, which there was: one kernel takes every launch)
-LS_API void ls_set_attention_prefill_pairs(int) {}
 
 // q, out: [tokens, nq * d] bfloat16; pages [num_pages, 2, nkv, page_size, d]; d 64 or 128; page
 // sizes 8, 16, 32, 64, 128.  Work items as for ls_attention_tile with up to 128 tokens each

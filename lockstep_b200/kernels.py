@@ -192,14 +192,6 @@ def set_gemm_tc_pairs(on: bool) -> None:
     fn(1 if on else 0)
 
 
-def set_attention_prefill_pairs(mode: int) -> None:
-    """Chose between kernels with one and with two heads a block for the tensor-core attention of prompt
-    portions; one kernel takes every launch now, and the choice has no effect."""
-    fn = library("tc").ls_set_attention_prefill_pairs
-    fn.argtypes, fn.restype = [c_int], None
-    fn(int(mode))
-
-
 def set_dependent_launch(on: bool) -> None:
     """Programmatic dependent launch of all kernels (on by default): a kernel is
     scheduled while its predecessor drains and waits for it before it touches memory."""

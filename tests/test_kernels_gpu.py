@@ -307,20 +307,14 @@ def test_attention_prefix_portion_and_decode(dtype, nq, nkv, d, page, window):
     got = run_attention(k, q[550:], pages, ids, 550, window, scale, False)
     assert (got - want[550:]).abs().max() <= bound
     if dtype == torch.bfloat16 and d in (64, 128):
-        # the tensor-core kernel: a whole prompt, a ragged tail, two tokens at a tile's edge
-        # (tcgen05, 128-token tiles)
-        for kernel in ("prefill_tc",):
-            for lo, hi in [(0, 700), (550, 700), (0, 1), (63, 65), (640, 642), (100, 229), (127, 130), (0, 129)]:
-                got = run_attention(k, q[lo:hi], pages, ids, lo, window, scale, kernel)
-                assert (got - want[lo:hi]).abs().max() <= bound, (kernel, lo, hi)
-                if (nq // nkv) % 2 == 0:
-                    # two heads of a key head in a block: another kernel, the same sums, the same bits
-                    k.set_attention_prefill_pairs(2)
-                    try:
-                        paired = run_attention(k, q[lo:hi], pages, ids, lo, window, scale, kernel)
-                    finally:
-                        k.set_attention_prefill_pairs(1)
-                    assert torch.equal(paired, got), (kernel, lo, hi)
+        # the tensor-core kernel (tcgen05, 128-token tiles): a whole prompt, a ragged tail, two tokens at a tile's edge;
+        # a row has the same bits in each
+        whole = run_attention(k, q, pages, ids, 0, window, scale, "prefill_tc")
+        for lo, hi in [(0, 700), (550, 700), (0, 1), (63, 65), (640, 642), (100, 229), (127, 130), (0, 129)]:
+            got = run_attention(k, q[lo:hi], pages, ids, lo, window, scale, "prefill_tc")
+            assert (got - want[lo:hi]).abs().max() <= bound, (lo, hi)
+            if hi - lo > 1:                          # (one token alone is a decoded token: splits and a fold)
+                assert torch.equal(got, whole[lo:hi]), (lo, hi)
     # single tokens at telling places: first, page edges, split edges, last
     for pos in [0, 1, page - 1, page, 255, 256, 257, 511, 512, 699]:
         sub_pages, sub_ids = pages, ids
@@ -340,11 +334,10 @@ def test_attention_prefix_portion_and_decode(dtype, nq, nkv, d, page, window):
 
 @pytest.mark.parametrize("nq,nkv,d,page,n,window", [(16, 8, 128, 16, 8192, 0), (8, 2, 64, 8, 5000, 0),
                                                      (32, 8, 128, 32, 4096, 1000), (4, 1, 128, 16, 12000, 0)])
-def test_the_two_prompt_attention_kernels_agree_bit_for_bit_on_long_prompts(nq, nkv, d, page, n, window):
-    """One head a block against the two heads of a key head a block, on prompts long enough that a
-    launch would take the second by itself, five runs each: the same bits every time (the second
-    kernel writes P over the scores it came from and relies on the order of the MMAs; a race
-    would show as a run that differs)."""
+def test_prompt_attention_of_long_prompts_gives_the_same_bits_every_time(nq, nkv, d, page, n, window):
+    """Prompts long enough that every block walks several items, six runs: the same bits every time (P is written over
+    the scores it came from, the teams hand a row's maximum and sums to each other, and a tile's places in shared and tensor
+    memory are used again in the order of the MMAs; a race would show as a run that differs)."""
     from lockstep_b200.engine.batch import plan_attention
 
     k = K()
@@ -356,21 +349,15 @@ def test_the_two_prompt_attention_kernels_agree_bit_for_bit_on_long_prompts(nq, 
     tile, _, _, _ = plan_attention([(0, 0, 0, n)], window, k.attention_split_size(), 128)
     work = torch.from_numpy(tile).to(dev())
     err = k.new_error_word(dev())
-    outs = {0: [], 2: []}
-    try:
-        for mode in (0, 2):
-            k.set_attention_prefill_pairs(mode)
-            for _ in range(1 if mode == 0 else 5):
-                out = torch.full_like(q, float("nan"))
-                assert k.attention_prefill_tc(q, pages, out, work, len(tile), table, nq, nkv, d, window,
-                                              1 / math.sqrt(d), err)
-                outs[mode].append(out)
-    finally:
-        k.set_attention_prefill_pairs(1)
+    outs = []
+    for _ in range(6):
+        out = torch.full_like(q, float("nan"))
+        assert k.attention_prefill_tc(q, pages, out, work, len(tile), table, nq, nkv, d, window, 1 / math.sqrt(d), err)
+        outs.append(out)
     k.raise_on_fault(err)
-    assert bool(torch.isfinite(outs[0][0].float()).all())
-    for out in outs[2]:
-        assert torch.equal(out, outs[0][0])
+    assert bool(torch.isfinite(outs[0].float()).all())
+    for out in outs[1:]:
+        assert torch.equal(out, outs[0])
     # spot rows against plain attention
     qf = q.double().cpu().view(n, nq, d)
     for r in (0, 127, 128, n // 2 + 3, n - 1):
@@ -382,7 +369,7 @@ def test_the_two_prompt_attention_kernels_agree_bit_for_bit_on_long_prompts(nq, 
             kk = pages[pg, 0, kv, off].double().cpu()
             vv = pages[pg, 1, kv, off].double().cpu()
             want[h] = torch.softmax(kk @ qf[r, h] / math.sqrt(d), 0) @ vv
-        assert (outs[0][0][r].double().cpu().view(nq, d) - want).abs().max() <= 2e-2, r
+        assert (outs[0][r].double().cpu().view(nq, d) - want).abs().max() <= 2e-2, r
 
 
 @pytest.mark.parametrize("dtype", DTYPES)

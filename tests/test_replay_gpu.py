@@ -177,25 +177,27 @@ def test_long_decoding_and_first_tokens(zoo):
 
 
 @pytest.mark.parametrize("name", ["D", "E"])
-def test_prompt_attention_with_two_heads_a_block_gives_the_same_bits(zoo, name):
-    """The tensor-core attention of prompts has a kernel with one query head a block and one with
-    the two heads of a key head a block (taken where a launch has items enough); which one runs
-    depends on the batch, so both must give every row the same bits."""
-    from lockstep_b200 import kernels as K
-
+def test_bfloat16_prompt_rows_do_not_depend_on_the_cutting(zoo, name):
+    """A prompt in one portion and in portions of two tokens and more, whose edges lie anywhere in the attention's tiles: the
+    same bits in every row.  (A single token is a decoded one, whose attention has other sums in bfloat16.)"""
     folder, requests, plain = zoo(name, "bfloat16")
+    sizes = (7, 131, 2, 60, 3, 128, 33, 200, 29, 300)
+    cut = []
+    for uid, toks in requests.items():
+        at, i = 0, 0
+        while at < len(toks):
+            n = sizes[i % len(sizes)]
+            if len(toks) - at - n < 2:
+                n = len(toks) - at
+            cut.append({"entries": [(uid, toks[at:at + n], list(range(n)))], "end": [uid] if at + n == len(toks) else []})
+            at, i = at + n, i + 1
     rows = {}
-    try:
-        for mode in (0, 2):
-            K.set_attention_prefill_pairs(mode)
-            steps = make_plan("portions", name, requests)
-            rows[mode] = H.run_plan(make_runner(folder, name, "bfloat16", steps), steps)
-    finally:
-        K.set_attention_prefill_pairs(1)
-    H.assert_rows_close(rows[2], plain, "bfloat16", f"{name}/two heads a block", config=name)
-    assert rows[0].keys() == rows[2].keys()
-    for key in rows[0]:
-        assert torch.equal(rows[0][key], rows[2][key]), key
+    for mode, steps in (("whole", make_plan("whole", name, requests)), ("cut", cut)):
+        rows[mode] = H.run_plan(make_runner(folder, name, "bfloat16", steps), steps)
+    H.assert_rows_close(rows["cut"], plain, "bfloat16", f"{name}/cut", config=name)
+    assert rows["whole"].keys() == rows["cut"].keys()
+    for key in rows["whole"]:
+        assert torch.equal(rows["whole"][key], rows["cut"][key]), key
 
 
 @pytest.mark.parametrize("name", ["D", "E"])
