@@ -503,6 +503,31 @@ def test_many_short_portions_have_the_rows_of_each_alone(nq, nkv, d, mask, extra
             assert torch.equal(rows, prompt.run([(r, start, n)])[0]), r
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.125, -3.0])
+def test_prompt_attention_takes_a_scale_that_is_not_above_0(scale):
+    prompt = Prompt(4, 2, 64, 16, [300], (100, 4))
+    prompt.scale = scale
+    assert (prompt.run([(0, 0, 300)])[0].double() - prompt.plain(0)).abs().max() <= 2e-2
+
+
+@pytest.mark.parametrize("d,extra", [(128, None), (64, "log")])
+def test_a_row_whose_scores_are_no_numbers_weighs_nothing(d, extra):
+    """A query that is NaN gives a row of zeros and leaves the others their bits; a key that is NaN is NaN in every row that sees
+    it beside others, and zeros in the row that sees it alone."""
+    prompt = Prompt(2, 1, d, 16, [300], 0, extra)
+    clean = prompt.run([(0, 0, 300)])[0]
+    for row in (0, 130, 299):
+        prompt.q[0][row, 1] = math.nan
+    got = prompt.run([(0, 0, 300)])[0]
+    hit = torch.zeros(300, 2, dtype=torch.bool)
+    hit[[0, 130, 299], 1] = True
+    assert bool((got[hit] == 0).all()) and torch.equal(got[~hit], clean[~hit])
+    prompt = Prompt(2, 1, d, 16, [300], 0, extra)
+    prompt.pages[int(prompt.table[0, 0]), 0, 0, 0, 3] = math.nan
+    got = prompt.run([(0, 0, 300)])[0]
+    assert bool((got[0] == 0).all()) and bool(got[1:].isnan().all())
+
+
 @pytest.mark.parametrize("nq,nkv,d,page,mask", [(4, 2, 128, 16, 0), (3, 3, 16, 8, 0), (8, 2, 64, 64, 100), (8, 1, 128, 32, (300, 40)),
                                                 (2, 1, 112, 16, -96), (4, 4, 128, 128, 0)])
 def test_float32_splits_of_single_tokens_have_the_bits_of_the_tile_kernel(nq, nkv, d, page, mask):
