@@ -3,8 +3,8 @@
 //
 // Orientation: up to 128 tokens, the weight tile is the MMA's M side (128 rows of
 // W) and the tokens are its N side (16..128 per tile), so a batch of one decoded
-// token wastes no rows of the MMA; more tokens are the M side themselves
-// (gemm_tc_rows_kernel: 256 a tile on a pair of blocks, tcgen05 cta_group::2, each
+// token wastes no rows of the MMA; more tokens, and 33 to 128 of some products
+// (rows_better), are the M side themselves (gemm_tc_rows_kernel: 256 a tile on a pair of blocks, tcgen05 cta_group::2, each
 // block with its 128 tokens and half of the weight rows), whose outputs then lie
 // side by side in a thread.
 // Either way an output element is the same dot product, accumulated in the same
@@ -340,9 +340,10 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer[r]) : "r"(base), "r"(r < shares ? r : 0));
     // FOLD columns at a time: their shares' values (and the old values of a residual) are all
     // asked for before any is used, so that a block pays a few trips through the cluster's
-    // shared memory and not one per column.  All columns of a block at 64 tokens where the shares are few (64 tokens, four
-    // shares: q/k/v of 1,024 to 4,096 features 7.4 -> 6.8 us, gate/up of 3,072 11.4 -> 8.6; 128 tokens 18.0 -> 12.4); with eight, four at
-    // a time are faster than eight (o and down 6.05 and 6.63 against 6.23 and 6.75).
+    // shared memory and not one per column.  Where the shares are few, all columns of a block at 64 tokens (two and four shares;
+    // 48 of 64 with three, which take the instance of four) or half of them at 128: 64 tokens, four
+    // shares: q/k/v of 1,024 to 4,096 features 7.4 -> 6.8 us, gate/up of 3,072 11.4 -> 8.6; 128 tokens 18.0 -> 12.4.  With five to eight,
+    // four at a time are faster than eight (o and down 6.05 and 6.63 against 6.23 and 6.75).
     constexpr int FOLD = SH == 8 ? 4 : 64 / SH;
     for (int c0 = (int)blockIdx.z; c0 < BN; c0 += FOLD * shares) {
       float vg[FOLD][SH], vu[FOLD][SH], before[FOLD];
@@ -1559,7 +1560,7 @@ Plan make_plan(int T, int N, int K, int epilogue) {
   p.shares = (total_kb + p.kb_per_share - 1) / p.kb_per_share;    // every share has work
   p.in_cluster = p.shares > 1 && T <= 128;
   p.bn = 16;                                        // token tile of the kernels with the weights on the M side
-  while (p.bn < T && p.bn < 128) p.bn *= 2;         // (more than 128 tokens go to the kernel with tokens as rows)
+  while (p.bn < T && p.bn < 128) p.bn *= 2;         // (more go to the kernel with the tokens as rows; so do some of fewer, see rows_better)
   return p;
 }
 
@@ -1769,7 +1770,7 @@ int launch_rows_as(const CUtensorMap& mw, const CUtensorMap& mx, void* C, int T,
   return launch_rows<EPI, FN, 1, TC>(mw, mx, C, T, N, K, ldc, plan, err, stream);
 }
 
-// more than 128 tokens: the kernel with the tokens on the M side
+// more than 128 tokens, and 33 to 128 where rows_better says so: the kernel with the tokens on the M side
 int run_rows(const void* X, const void* W, void* C, int c_dtype, int T, int N, int K, int64_t ldx, int64_t ldw,
              int64_t ldc, int epilogue, const Plan& plan, int* err, cudaStream_t stream) {
   typedef __nv_bfloat16 bf16;
@@ -1964,7 +1965,7 @@ LS_API int ls_kernel_launches_tc(unsigned long long* out, int n) {
   return LS_K_COUNT;
 }
 
-// Whether products of more than 128 tokens run on pairs of blocks (the default) or on single
+// Whether products in the kernel with the tokens as rows run on pairs of blocks (the default) or on single
 // blocks; the sums are the same either way.
 LS_API void ls_set_gemm_tc_pairs(int on) { rows_pairs = on ? 1 : 0; }
 

@@ -253,25 +253,30 @@ def test_qkv_heads_in_the_product_decline_what_they_do_not_cover():
     assert not call(8, w_=shallow)
 
 
-@pytest.mark.parametrize("n,k", [(6144, 2560), (1024, 512), (4096, 1024), (2048, 2048), (1000, 1024), (2560, 4096)])
-def test_rows_of_33_to_128_tokens_have_the_same_bits_on_either_side_of_the_rules(n, k):
-    """Products that go to the kernel with the tokens as rows below 129 tokens, some from 33 and some from 65 on, and to clusters
-    before that: a row's bits are those of the same row among 300."""
+@pytest.mark.parametrize("n,k,shares,first", [
+    (6272, 2560, 3, 33), (1024, 512, 2, 33),                                   # a second round of clusters of three; a depth of 512
+    (4096, 1024, 4, 65), (1000, 1024, 4, 65), (2304, 2048, 8, 65), (2688, 4096, 7, 65),     # a depth of 1,024; second rounds
+    (6600, 2560, 2, 129), (4801, 2560, 3, 129), (4000, 4096, 4, 129), (1000, 2048, 8, 129)])  # one round of a deeper product
+def test_rows_of_33_to_128_tokens_have_the_same_bits_on_either_side_of_the_rules(n, k, shares, first):
+    """A product of 33 to 128 tokens whose depth is shared out runs in clusters below ``first`` tokens and in the kernel with the
+    tokens as rows from there on; a row's bits are those of the same row among 32 (clusters too) and among 300 (rows)."""
     from lockstep_b200 import kernels as K
 
+    assert K.library("tc").ls_gemm_tc_k_shares(n, k) == shares
     g = torch.Generator(device=dev()).manual_seed(n + k)
     x = torch.randn(300, k, generator=g, device=dev()).to(torch.bfloat16)
     w = (torch.randn(2 * n, k, generator=g, device=dev()) * 0.1).to(torch.bfloat16)
     old = torch.randn(300, n, generator=g, device=dev())
-    err, ran = K.new_error_word(dev()), set()
+    err, names = K.new_error_word(dev()), ("gemm_tc_few", "gemm_tc_cluster", "gemm_tc_rows_pair")
     for code, weight, kind in ((K.EPILOGUE_STORE, w[:n].contiguous(), torch.bfloat16), (K.EPILOGUE_RESIDUAL, w[:n].contiguous(), torch.float32),
                                (K.EPILOGUE_SILU_MUL, w, torch.bfloat16), (K.EPILOGUE_GELU, w[:n].contiguous(), torch.bfloat16)):
         full = old.to(kind)
         assert K.gemm_nt_tc(x, weight, full, code, err)
-        for t in (32, 33, 64, 65, 100, 128):
+        for t in (32, 33, 64, 65, 101, 128):
             part, before = old[:t].to(kind), K.kernel_counts()
             assert K.gemm_nt_tc(x[:t].contiguous(), weight, part, code, err)
-            ran |= {(t, name) for name, count in K.kernel_counts().items() if count > before.get(name, 0)}
+            after = K.kernel_counts()
+            ran = [name for name in names if after[name] > before.get(name, 0)]
+            assert ran == ["gemm_tc_few" if t <= 32 else "gemm_tc_cluster" if t < first else "gemm_tc_rows_pair"], (code, t)
             assert torch.equal(part, full[:t]), (code, t)
     K.raise_on_fault(err)
-    assert (128, "gemm_tc_rows_pair") in ran and (32, "gemm_tc_rows_pair") not in ran
