@@ -181,7 +181,7 @@ struct Item {
 //
 // What bounds it: MMAs (1,024 cycles a tile of 128 x 128 with d = 128), exponentials (1,024 on the special-function
 // units), shared memory (160 KB a tile at 128 bytes a cycle) and L2 (64 KB a tile an SM) have to run side by side; a tile
-// takes about 1,850 cycles, paced by S and PV one after the other and the issuing warp's waits between them (tensor pipe and
+// takes about 1,880 cycles, paced by S and PV one after the other and the issuing warp's waits between them (tensor pipe and
 // special-function units half busy, L2 a quarter; a third stage of values changes nothing).  Measured, 16 query and 8 key heads of 128, pages of 16, with a
 // head a block and four threads a row (two heads a block for the last two) / now: 2,048 tokens 30.5 / 25.9 us, 2,048 after
 // 6,144 149.7 / 116.1 us, 8,192 277 / 248 us (1,110 TFLOP/s).

@@ -103,8 +103,9 @@ def attend(rt: Runtime, q, ctx, cache, nq: int, nkv: int, d: int, mask, scale: f
            extras: ScoreExtras, close: MapDifference | None = None) -> torch.Tensor:
     """Causal attention of the step's queries ``q`` [tokens, nq d] over a layer's pages (heads of one
     size ``d``): prompt portions by tiles, single tokens by splits and a fold.  Returns [tokens, nq d]
-    in the engine's type.  ``exact``: every row takes the tile kernel, so that a row's bits do not
-    depend on whether it was decoded or part of a prompt.  ``mask``: a window (0: none, < 0: chunks of -window
+    in the engine's type.  ``exact``: every row takes one of the kernels with the sums of ``attention_tile``, element by
+    element (that one, ``attention_rows`` and ``attention_split``), so that a row's bits do not depend on whether it was decoded or
+    part of a prompt.  ``mask``: a window (0: none, < 0: chunks of -window
     positions), or a pair of a window and the number of first positions that stay visible.  ``close``: what turns the
     attention's rows into the ones to return."""
     t = q.shape[0]
@@ -221,7 +222,7 @@ class GQAttention(Mixer):
         self.position, self.rt = position, runtime
         self.w_qkv = self.w_o = self.q_gain = self.k_gain = self.qkv_bias = self.o_bias = self.v_mix = None
         self.extras = ScoreExtras()
-        # in float32 every row takes the tile kernel, so that a row's bits do not
+        # in float32 every attention kernel has the same sums, so that a row's bits do not
         # depend on whether it was decoded or part of a prompt
         self.exact = runtime.dtype == torch.float32
 
