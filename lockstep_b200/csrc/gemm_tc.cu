@@ -1648,8 +1648,15 @@ int launch_few(const CUtensorMap& mw, const CUtensorMap& mx, const NormArgs& nor
   // before it ends.  (Steps of one request / 8 at a context of 1,500 / 16 at 300 / 32 at 60, ms with 24 / 40 / 40 / 40 decoded tokens
   // and the prompts: what is used 21.59 / 62.7 / 51.5 / 51.4, 113 KB 21.83 / 62.6 / 51.1 / 51.5, 114 to 140 KB 20.60 / 63.3 / 51.2 / 50.7,
   // the whole SM 20.59 / 64.6 / 52.2 / 51.4.)
+  // A product on at most a third of the SMs asks for a whole one all the same: the next kernels' blocks find SMs enough without
+  // sharing.  (Decode steps of 1,024 wide layers of 8 query and 4 key heads at a context of 2,048, whose products other than q/k/v have 32
+  // blocks, ms a step, the whole SM for all products / 140 KB for all / this rule: 8 requests 0.320 / 0.330 / 0.323, 16 0.383 / 0.387 / 0.380,
+  // 32 0.545 / 0.565 / 0.540.  A line at half of the SMs would take in o and down of the 0.6B sizes, 64 blocks: the one request above
+  // 20.75, 8 at 4,000 211.1 against 209.2 ms.)
   const int used = (int)lay.bars_off + bars_bytes + 1024;
-  lay.smem = (uint32_t)(used > FEW_SMEM ? used : FEW_SMEM);
+  const long long blocks = (long long)((N + BM - 1) / BM) * ((T + BN - 1) / BN) * plan.shares;
+  const int asked = 3 * blocks <= sm_count() ? MAX_DYNAMIC_SMEM : FEW_SMEM;
+  lay.smem = (uint32_t)(used > asked ? used : asked);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((N + BM - 1) / BM, (T + BN - 1) / BN, plan.shares);
   cfg.blockDim = dim3(192);
